@@ -83,7 +83,7 @@ def parse():
                          "(exchange over NCCL), else this many slabs on one GPU (exchange by device copies)")
     ap.add_argument("--kernels", action="store_true",
                     help="only launch the hot kernels on the workload's data (for an ncu capture); prints their times")
-    ap.add_argument("--stream-kernel", choices=("xp", "zp"), default="xp",
+    ap.add_argument("--stream-kernel", choices=("march", "xp", "zp"), default="march",
                     help="streaming operator kernel for FP64 / FP32 iterates (vx_set_stream_kernel)")
     ap.add_argument("--tc", action="store_true",
                     help="with --kernels: the tensor-core element-block operator (4 launches) instead")

@@ -324,6 +324,7 @@ struct OpArgs2 {
 }  // namespace vx
 
 #include "vx_zp.cuh"
+#include "vx_march.cuh"
 
 namespace vx {
 
@@ -749,10 +750,17 @@ inline ZpGrid zp_grid_for(const Grid& g) {
     return zp_grid(g, ZpCfg<TC>::NW, sm_count());
 }
 
+template <typename TC>
+dim3 march_grid(const Grid& g, int* cx) {
+    const int tz = (g.nz + 1 + TZ - 1) / TZ, own = march_rows<TC>() - 2, ty = (g.ny + 1 + own - 1) / own;
+    *cx = march_cx(g, tz * ty, March<TC>::MINB * sm_count());
+    return dim3(tz, ty, (g.nx + 1 + *cx - 1) / *cx);
+}
+
 // Streaming kernel for FP64 / FP32 iterates (process-wide; the other storage forms always run
-// parity_stream_xp): VX_KERNEL_XP (element-plane pairs, the default) or VX_KERNEL_ZP (node-column
-// pairs).
-static std::atomic<int> g_stream_kernel{VX_KERNEL_XP};
+// parity_march): VX_KERNEL_MARCH (the default), VX_KERNEL_XP (element-plane pairs) or VX_KERNEL_ZP
+// (node-column pairs).
+static std::atomic<int> g_stream_kernel{VX_KERNEL_MARCH};
 
 // CTAs (= partial sums) of a fused reducing launch of precision `prec` on grid g
 int64_t stream_ctas(const Grid& g, int prec) {
@@ -762,9 +770,14 @@ int64_t stream_ctas(const Grid& g, int prec) {
             const ZpGrid z = prec == VX_F32 ? zp_grid_for<float>(g) : zp_grid_for<double>(g);
             return int64_t(z.tz) * z.ty * z.chunks;
         }
+        if (kind == VX_KERNEL_XP) {
+            const Tiling t = tiling(prec, true);
+            dim3 d = stream_grid(g, t, stream_cx(g, t));
+            return int64_t(d.x) * d.y * d.z;
+        }
     }
-    const Tiling t = tiling(prec, true);
-    dim3 d = stream_grid(g, t, stream_cx(g, t));
+    int cx;
+    dim3 d = prec == VX_F64 ? march_grid<double>(g, &cx) : march_grid<float>(g, &cx);
     return int64_t(d.x) * d.y * d.z;
 }
 
@@ -784,57 +797,52 @@ template <typename TC, typename TU, typename TE, typename TY, int EPI, int MASK,
 int launch_stream(const OpArgs<TC, TU, TE, TY, TR>& a_in, cudaStream_t s, const char* what) {
     constexpr bool v2 = !REV && !SIMP && MASK != MASK_DOF;
     static_assert(v2 || std::is_same<TR, TY>::value, "parity_stream takes r and invd of the output type");
-    // iterates in FP64 / FP32: either streaming kernel (parity_zp stages 4- or 8-byte words)
-    constexpr bool zp_ok = v2 && (std::is_same<TU, double>::value || std::is_same<TU, float>::value);
+    // iterates in FP64 / FP32: any streaming kernel (parity_zp stages 4- or 8-byte words)
+    constexpr bool selectable = v2 && (std::is_same<TU, double>::value || std::is_same<TU, float>::value);
     OpArgs<TC, TU, TE, TY, TR> a = a_in;
-    const bool cubic = a.cubic;
     static std::atomic<uint64_t> configured[2];            // per kernel of this instantiation: devices opted in
-    const int kind = zp_ok ? g_stream_kernel.load(std::memory_order_relaxed) : VX_KERNEL_XP;
-    if constexpr (zp_ok) {
-        if (kind == VX_KERNEL_ZP) {
-            const ZpGrid z = zp_grid_for<TC>(a.g);
-            a.cx = z.cx;
-            const OpArgs2<TC, TU, TE, TY, TR> a2 = packed_args<TC, TU, TE, TY, TR, EPI, MASK>(a);
-            using Lz = ZpLayout<TC, TU, TE>;
-            static std::atomic<uint64_t> cfg_zp[2];
-            auto kz = cubic ? parity_zp<TC, TU, TE, TY, TR, EPI, MASK, true> : parity_zp<TC, TU, TE, TY, TR, EPI, MASK, false>;
-            int st = smem_opt_in(cfg_zp[cubic ? 1 : 0], (const void*)kz, Lz::BYTES, what);
+    if constexpr (v2) {
+        const bool cubic = a.cubic;
+        const int kind = selectable ? g_stream_kernel.load(std::memory_order_relaxed) : VX_KERNEL_MARCH;
+        using Args = OpArgs2<TC, TU, TE, TY, TR>;
+        auto go = [&](void (*k)(const Args), std::atomic<uint64_t>& done, dim3 grid, unsigned threads, size_t smem) -> int {
+            const Args a2 = packed_args<TC, TU, TE, TY, TR, EPI, MASK>(a);
+            int st = smem_opt_in(done, (const void*)k, smem, what);
             if (st) return st;
-            vx::launch(kz, dim3(z.tz, z.ty, z.chunks), unsigned(Lz::NW * 32), Lz::BYTES, s, a2);
+            vx::launch(k, grid, threads, smem, s, a2);
             VX_CHECK_LAUNCH(what);
             return VX_OK;
-        }
-    }
-    {
-        const Tiling t = tiling(std::is_same<TC, double>::value ? VX_F64 : VX_F32, v2);
-        a.cx = stream_cx(a.g, t);
-        size_t smem, threads;
-        if constexpr (v2) {
-            threads = XpCfg<TC>::NW * 32;
-            smem = size_t(2) * XpCfg<TC>::NW * 6 * 32 * sizeof(V2<TC>);
-        } else {
-            threads = NW * 32;
-            smem = size_t(2) * NW * 6 * 32 * sizeof(TC);
-        }
-        if constexpr (v2) {
-            const OpArgs2<TC, TU, TE, TY, TR> a2 = packed_args<TC, TU, TE, TY, TR, EPI, MASK>(a);
-            if (cubic) {
-                auto k = parity_stream_xp<TC, TU, TE, TY, TR, EPI, MASK, true>;
-                int st = smem_opt_in(configured[1], (const void*)k, smem, what);
-                if (st) return st;
-                vx::launch(k, stream_grid(a.g, t, a.cx), unsigned(threads), smem, s, a2);
-            } else {
-                auto k = parity_stream_xp<TC, TU, TE, TY, TR, EPI, MASK, false>;
-                int st = smem_opt_in(configured[0], (const void*)k, smem, what);
-                if (st) return st;
-                vx::launch(k, stream_grid(a.g, t, a.cx), unsigned(threads), smem, s, a2);
+        };
+        if constexpr (selectable) {
+            if (kind == VX_KERNEL_ZP) {
+                const ZpGrid z = zp_grid_for<TC>(a.g);
+                a.cx = z.cx;
+                using Lz = ZpLayout<TC, TU, TE>;
+                static std::atomic<uint64_t> cfg_zp[2];
+                return go(cubic ? parity_zp<TC, TU, TE, TY, TR, EPI, MASK, true> : parity_zp<TC, TU, TE, TY, TR, EPI, MASK, false>,
+                          cfg_zp[cubic ? 1 : 0], dim3(z.tz, z.ty, z.chunks), unsigned(Lz::NW * 32), Lz::BYTES);
             }
-        } else {
-            auto k = parity_stream<TC, TU, TE, TY, EPI, MASK, REV, SIMP>;
-            int st = smem_opt_in(configured[0], (const void*)k, smem, what);
-            if (st) return st;
-            vx::launch(k, stream_grid(a.g, t, a.cx), unsigned(threads), smem, s, a);
+            if (kind == VX_KERNEL_XP) {
+                const Tiling t = tiling(std::is_same<TC, double>::value ? VX_F64 : VX_F32, v2);
+                a.cx = stream_cx(a.g, t);
+                static std::atomic<uint64_t> cfg_xp[2];
+                return go(cubic ? parity_stream_xp<TC, TU, TE, TY, TR, EPI, MASK, true>
+                                : parity_stream_xp<TC, TU, TE, TY, TR, EPI, MASK, false>,
+                          cfg_xp[cubic ? 1 : 0], stream_grid(a.g, t, a.cx), XpCfg<TC>::NW * 32,
+                          size_t(2) * XpCfg<TC>::NW * 6 * 32 * sizeof(V2<TC>));
+            }
         }
+        const dim3 grid = march_grid<TC>(a.g, &a.cx);
+        return go(cubic ? parity_march<TC, TU, TE, TY, TR, EPI, MASK, true> : parity_march<TC, TU, TE, TY, TR, EPI, MASK, false>,
+                  configured[cubic ? 1 : 0], grid, March<TC>::NW * 32, march_smem<TC>());
+    } else {
+        const Tiling t = tiling(VX_F64, false);
+        a.cx = stream_cx(a.g, t);
+        const size_t smem = size_t(2) * NW * 6 * 32 * sizeof(TC);
+        auto k = parity_stream<TC, TU, TE, TY, EPI, MASK, REV, SIMP>;
+        int st = smem_opt_in(configured[0], (const void*)k, smem, what);
+        if (st) return st;
+        vx::launch(k, stream_grid(a.g, t, a.cx), NW * 32, smem, s, a);
         VX_CHECK_LAUNCH(what);
         return VX_OK;
     }
@@ -1282,7 +1290,7 @@ extern "C" int vx_true_residual_noalloc(int prec, int nx, int ny, int nz, const 
 }
 
 extern "C" int vx_set_stream_kernel(int kind) {
-    if (kind != VX_KERNEL_ZP && kind != VX_KERNEL_XP) {
+    if (kind != VX_KERNEL_MARCH && kind != VX_KERNEL_ZP && kind != VX_KERNEL_XP) {
         set_error("vx_set_stream_kernel: unknown kernel %d", kind);
         return -1;
     }
