@@ -272,6 +272,9 @@ int vx_device_status(int* status, int clear);
  * after it.  Returns the previous selection, or -1 for an unknown kind.  No counterpart in the
  * reference. */
 enum { VX_KERNEL_XP = 0, VX_KERNEL_ZP = 1, VX_KERNEL_MARCH = 2 };
+/* Or'ed into the `prec` of vx_matvec, vx_jacobi_sweep, vx_residual, vx_apply_dot, vx_true_residual and
+ * vx_operator_partials: this call runs VX_KERNEL_XP where it would run VX_KERNEL_MARCH. */
+enum { VX_STREAM_XP = 0x100 };
 int vx_set_stream_kernel(int kind);
 
 /* Tensor-core element-block operator, an experiment measured against the streaming kernels and not

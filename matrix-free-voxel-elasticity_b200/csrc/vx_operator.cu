@@ -53,6 +53,7 @@ struct OpArgs {
     double emin, de, penal;   // SIMP modulus E = emin + de * rho^penal
     int cx;                   // owned node planes per CTA (x chunk)
     bool cubic;               // host side: the blocks have the cube pattern (CubeK)
+    bool xp;                  // host side: parity_stream_xp instead of parity_march (VX_STREAM_XP)
     BlocksT<TC> C;
 };
 
@@ -757,14 +758,20 @@ dim3 march_grid(const Grid& g, int* cx) {
     return dim3(tz, ty, (g.nx + 1 + *cx - 1) / *cx);
 }
 
-// Streaming kernel for FP64 / FP32 iterates (process-wide; the other storage forms always run
-// parity_march): VX_KERNEL_MARCH (the default), VX_KERNEL_XP (element-plane pairs) or VX_KERNEL_ZP
-// (node-column pairs).
+// Streaming kernel for FP64 / FP32 iterates (process-wide; the other storage forms run parity_march):
+// VX_KERNEL_MARCH (the default), VX_KERNEL_XP (element-plane pairs) or VX_KERNEL_ZP (node-column pairs).
+// A call whose selector carries VX_STREAM_XP runs parity_stream_xp instead of parity_march.
 static std::atomic<int> g_stream_kernel{VX_KERNEL_MARCH};
 
+inline int stream_kind(bool selectable, bool xp) {
+    const int kind = selectable ? g_stream_kernel.load(std::memory_order_relaxed) : VX_KERNEL_MARCH;
+    return xp && kind == VX_KERNEL_MARCH ? VX_KERNEL_XP : kind;
+}
+
 // CTAs (= partial sums) of a fused reducing launch of precision `prec` on grid g
-int64_t stream_ctas(const Grid& g, int prec) {
-    const int kind = g_stream_kernel.load(std::memory_order_relaxed);
+int64_t stream_ctas(const Grid& g, int sel) {
+    const int prec = sel & ~VX_STREAM_XP;
+    const int kind = stream_kind(true, sel & VX_STREAM_XP);
     if (prec == VX_F32 || prec == VX_F64) {
         if (kind == VX_KERNEL_ZP) {
             const ZpGrid z = prec == VX_F32 ? zp_grid_for<float>(g) : zp_grid_for<double>(g);
@@ -803,7 +810,7 @@ int launch_stream(const OpArgs<TC, TU, TE, TY, TR>& a_in, cudaStream_t s, const 
     static std::atomic<uint64_t> configured[2];            // per kernel of this instantiation: devices opted in
     if constexpr (v2) {
         const bool cubic = a.cubic;
-        const int kind = selectable ? g_stream_kernel.load(std::memory_order_relaxed) : VX_KERNEL_MARCH;
+        const int kind = stream_kind(selectable, a.xp);
         using Args = OpArgs2<TC, TU, TE, TY, TR>;
         auto go = [&](void (*k)(const Args), std::atomic<uint64_t>& done, dim3 grid, unsigned threads, size_t smem) -> int {
             const Args a2 = packed_args<TC, TU, TE, TY, TR, EPI, MASK>(a);
@@ -822,15 +829,15 @@ int launch_stream(const OpArgs<TC, TU, TE, TY, TR>& a_in, cudaStream_t s, const 
                 return go(cubic ? parity_zp<TC, TU, TE, TY, TR, EPI, MASK, true> : parity_zp<TC, TU, TE, TY, TR, EPI, MASK, false>,
                           cfg_zp[cubic ? 1 : 0], dim3(z.tz, z.ty, z.chunks), unsigned(Lz::NW * 32), Lz::BYTES);
             }
-            if (kind == VX_KERNEL_XP) {
-                const Tiling t = tiling(std::is_same<TC, double>::value ? VX_F64 : VX_F32, v2);
-                a.cx = stream_cx(a.g, t);
-                static std::atomic<uint64_t> cfg_xp[2];
-                return go(cubic ? parity_stream_xp<TC, TU, TE, TY, TR, EPI, MASK, true>
-                                : parity_stream_xp<TC, TU, TE, TY, TR, EPI, MASK, false>,
-                          cfg_xp[cubic ? 1 : 0], stream_grid(a.g, t, a.cx), XpCfg<TC>::NW * 32,
-                          size_t(2) * XpCfg<TC>::NW * 6 * 32 * sizeof(V2<TC>));
-            }
+        }
+        if (kind == VX_KERNEL_XP) {
+            const Tiling t = tiling(std::is_same<TC, double>::value ? VX_F64 : VX_F32, v2);
+            a.cx = stream_cx(a.g, t);
+            static std::atomic<uint64_t> cfg_xp[2];
+            return go(cubic ? parity_stream_xp<TC, TU, TE, TY, TR, EPI, MASK, true>
+                            : parity_stream_xp<TC, TU, TE, TY, TR, EPI, MASK, false>,
+                      cfg_xp[cubic ? 1 : 0], stream_grid(a.g, t, a.cx), XpCfg<TC>::NW * 32,
+                      size_t(2) * XpCfg<TC>::NW * 6 * 32 * sizeof(V2<TC>));
         }
         const dim3 grid = march_grid<TC>(a.g, &a.cx);
         return go(cubic ? parity_march<TC, TU, TE, TY, TR, EPI, MASK, true> : parity_march<TC, TU, TE, TY, TR, EPI, MASK, false>,
@@ -973,8 +980,9 @@ __global__ void energy_kernel(Grid g, const __grid_constant__ Ke ke, const doubl
 using namespace vx;
 
 // =========================================================================== C ABI
-extern "C" int vx_matvec(int prec, int nx, int ny, int nz, const double* blocks, const void* E,
+extern "C" int vx_matvec(int sel, int nx, int ny, int nz, const double* blocks, const void* E,
                          const void* u, void* y, const uint8_t* node_mask, cudaStream_t stream) {
+    const int prec = sel & ~VX_STREAM_XP;
     int st = check_grid(nx, ny, nz);
     if (st) return st;
     VX_CHECK_ARG(blocks && E && u && y, VX_ERR_NULL_POINTER, "vx_matvec: NULL pointer");
@@ -987,6 +995,7 @@ extern "C" int vx_matvec(int prec, int nx, int ny, int nz, const double* blocks,
         a.g = Grid{nx, ny, nz}; a.u = (const X*)u; a.E = (const M*)E; a.y = (TC*)y; a.node_mask = node_mask;
         a.C = convert_blocks<TC>(blocks);
         a.cubic = cube_pattern(blocks);
+        a.xp = sel & VX_STREAM_XP;
         rc = node_mask ? launch_stream<TC, X, M, TC, EPI_RAW, MASK_NODE, false, false>(a, stream, "vx_matvec")
                        : launch_stream<TC, X, M, TC, EPI_RAW, MASK_NONE, false, false>(a, stream, "vx_matvec");
     });
@@ -1124,9 +1133,10 @@ namespace {
 // the right-hand side, the inverse diagonal and the residual output are auxiliary vectors; the
 // reducing forms (apply_dot, true_residual) exist for VX_F64 and VX_F32.
 template <int EPI>
-int fused_dispatch(const char* what, int prec, int nx, int ny, int nz, const double* blocks, const void* E,
+int fused_dispatch(const char* what, int sel, int nx, int ny, int nz, const double* blocks, const void* E,
                    const uint8_t* node_mask, const void* x, const void* r, const void* invd, double omega,
                    void* out, double* partials, cudaStream_t stream, int dot_x0 = 0, int dot_x1 = INT_MAX) {
+    const int prec = sel & ~VX_STREAM_XP;
     int st = check_grid(nx, ny, nz);
     if (st) return st;
     VX_CHECK_ARG(blocks && E && x && out, VX_ERR_NULL_POINTER, "%s: NULL pointer", what);
@@ -1153,6 +1163,7 @@ int fused_dispatch(const char* what, int prec, int nx, int ny, int nz, const dou
             a.dot_x0 = dot_x0; a.dot_x1 = dot_x1;
             a.C = convert_blocks<TC>(blocks);
             a.cubic = cube_pattern(blocks);
+            a.xp = sel & VX_STREAM_XP;
             rc = node_mask ? launch_stream<TC, X, M, TY, EPI, MASK_NODE, false, false, R>(a, stream, what)
                            : launch_stream<TC, X, M, TY, EPI, MASK_NONE, false, false, R>(a, stream, what);
         }
@@ -1178,9 +1189,10 @@ extern "C" int vx_residual(int prec, int nx, int ny, int nz, const double* block
                                         nullptr, 0.0, res, nullptr, stream);
 }
 
-extern "C" int64_t vx_operator_partials(int prec, int nx, int ny, int nz) {
+extern "C" int64_t vx_operator_partials(int sel, int nx, int ny, int nz) {
+    const int prec = sel & ~VX_STREAM_XP;
     if (check_grid(nx, ny, nz) || (prec != VX_F64 && prec != VX_F32)) return -1;
-    return stream_ctas(Grid{nx, ny, nz}, prec);
+    return stream_ctas(Grid{nx, ny, nz}, sel);
 }
 
 extern "C" int vx_apply_dot(int prec, int nx, int ny, int nz, const double* blocks, const void* E,

@@ -74,9 +74,10 @@ class VoxelOperator:
     """K(E) on a (nx, ny, nz) voxel grid in `dtype` storage (float64, float32, or bfloat16 with
     FP32 arithmetic).  `aux_dtype` (default `dtype`) is the storage of the modulus and of the
     auxiliary vectors (right-hand side, inverse diagonal, residual output); float32 iterates with
-    bfloat16 auxiliaries is the VX_F32_BF16AUX mode."""
+    bfloat16 auxiliaries is the VX_F32_BF16AUX mode.  `stream="xp"` has the matvec, sweep, residual and
+    reducing forms run the element-plane-pair kernel where the default would run (VX_STREAM_XP)."""
 
-    def __init__(self, shape, ke, dtype=torch.float64, aux_dtype=None):
+    def __init__(self, shape, ke, dtype=torch.float64, aux_dtype=None, stream=None):
         self.shape = tuple(int(s) for s in shape)
         if len(self.shape) != 3 or min(self.shape) < 1:
             raise ValueError(f"invalid grid {shape}")
@@ -87,6 +88,9 @@ class VoxelOperator:
             raise ValueError(f"unsupported storage: iterate {dtype}, auxiliary {aux_dtype}")
         self.dtype, self.aux_dtype = dtype, aux_dtype
         self.prec = STORAGE[(dtype, aux_dtype)]
+        if stream not in (None, "xp"):
+            raise ValueError(f"unknown stream kernel {stream!r}")
+        self._sel = self.prec | (_lib.VX_STREAM_XP if stream == "xp" else 0)
         self.nodes = n_nodes(self.shape)
         self.ndof = 3 * self.nodes
         self.n_elem = n_elems(self.shape)
@@ -97,7 +101,7 @@ class VoxelOperator:
     @property
     def partials_size(self) -> int:
         """doubles of scratch the fused reducing forms (apply_dot / true_residual) need"""
-        return int(_lib.load().vx_operator_partials(self.prec, *self.shape))
+        return int(_lib.load().vx_operator_partials(self._sel, *self.shape))
 
     def _vec(self, t, what, dtype=None):
         return _ptr(t, what, dtype or self.dtype, self.ndof)
@@ -118,7 +122,7 @@ class VoxelOperator:
     def matvec(self, u, E, node_mask=None, out=None):
         """y = K u (node_mask None) or y = M K (M u) + (I - M) u."""
         y = self._out(out)
-        _lib.call("vx_matvec", self.prec, *self.shape, self._bp, self._E(E), self._vec(u, "u"),
+        _lib.call("vx_matvec", self._sel, *self.shape, self._bp, self._E(E), self._vec(u, "u"),
                   _ptr(y, "y", torch.float32 if self.dtype == torch.bfloat16 else self.dtype, self.ndof),
                   self._mask(node_mask), stream_ptr())
         return y
@@ -144,7 +148,7 @@ class VoxelOperator:
         """out = x + omega * inv_diag * (r - A x), A the Dirichlet operator (bfloat16: every
         vector in bf16, FP32 arithmetic)."""
         o = self._out(out, self.dtype)
-        _lib.call("vx_jacobi_sweep", self.prec, *self.shape, self._bp, self._E(E), self._mask(node_mask),
+        _lib.call("vx_jacobi_sweep", self._sel, *self.shape, self._bp, self._E(E), self._mask(node_mask),
                   self._vec(x, "x"), self._vec(r, "r", self.aux_dtype), self._vec(inv_diag, "inv_diag", self.aux_dtype),
                   float(omega), self._vec(o, "out"), stream_ptr())
         return o
@@ -152,19 +156,19 @@ class VoxelOperator:
     def residual(self, x, r, E, node_mask, out=None):
         """out = (r - A x) * M."""
         o = self._out(out, self.aux_dtype)
-        _lib.call("vx_residual", self.prec, *self.shape, self._bp, self._E(E), self._mask(node_mask),
+        _lib.call("vx_residual", self._sel, *self.shape, self._bp, self._E(E), self._mask(node_mask),
                   self._vec(x, "x"), self._vec(r, "r", self.aux_dtype), self._vec(o, "out", self.aux_dtype),
                   stream_ptr())
         return o
 
     def apply_dot(self, p, E, node_mask, q, partials):
         """q = A p; partials[cta] = sum p.q over the CTA's nodes (reduce with reduce_partials)."""
-        _lib.call("vx_apply_dot", self.prec, *self.shape, self._bp, self._E(E), self._mask(node_mask),
+        _lib.call("vx_apply_dot", self._sel, *self.shape, self._bp, self._E(E), self._mask(node_mask),
                   self._vec(p, "p"), self._vec(q, "q"), _ptr(partials, "partials", torch.float64), stream_ptr())
 
     def true_residual(self, x, b, E, node_mask, res, partials):
         """res = b - A x; partials[cta] = sum res^2 over the CTA's nodes."""
-        _lib.call("vx_true_residual", self.prec, *self.shape, self._bp, self._E(E), self._mask(node_mask),
+        _lib.call("vx_true_residual", self._sel, *self.shape, self._bp, self._E(E), self._mask(node_mask),
                   self._vec(x, "x"), self._vec(b, "b"), self._vec(res, "res"),
                   _ptr(partials, "partials", torch.float64), stream_ptr())
 

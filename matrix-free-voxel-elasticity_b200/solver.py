@@ -36,6 +36,18 @@ def hierarchy_shapes(shape, max_coarse_x=16):
     return shapes
 
 
+# Grids whose multigrid solves keep the element-plane-pair kernel on every level.  Below about 20,000
+# elements such a solve is bound by its launches, and on rough moduli its two- or three-level cycle often
+# does not converge: the iterate at maxiter then depends on every rounding, so these solves keep the
+# operations in the order they always had.
+SMALL_GRID = 20000
+
+
+def small_grid_stream(shape):
+    """`stream` of the VoxelOperators of a multigrid solve on the finest grid `shape`."""
+    return "xp" if shape[0] * shape[1] * shape[2] < SMALL_GRID else None
+
+
 def _s():
     return stream_ptr()
 
@@ -104,8 +116,9 @@ class MGHierarchy:
                 E64, mask = Ec, mc
             L = _Level()
             L.shape = s
-            L.op = VoxelOperator(s, self.ke * 2 ** i, dtype, aux_dtype)
-            L.op64 = L.op if dtype == torch.float64 else VoxelOperator(s, self.ke * 2 ** i, torch.float64)
+            st = small_grid_stream(self.shapes[0])
+            L.op = VoxelOperator(s, self.ke * 2 ** i, dtype, aux_dtype, stream=st)
+            L.op64 = L.op if dtype == torch.float64 else VoxelOperator(s, self.ke * 2 ** i, torch.float64, stream=st)
             L.E64, L.mask = E64, mask
             L.E = E64 if aux_dtype == torch.float64 else E64.to(aux_dtype)
             inv64 = L.op64.diagonal(E64, mask, inverse=True)
