@@ -151,6 +151,11 @@ int vx_residual(int prec, int nx, int ny, int nz, const double* blocks, const vo
 int vx_restrict(int prec, int nx, int ny, int nz, const void* fine, const uint8_t* coarse_mask,
                 void* coarse, cudaStream_t stream);
 
+/* The same with the coarse level's first sweep from zero: x = omega inv_diag coarse (an iterate), what
+ * vx_scaled_product would form from the stored restriction.  Replaces src/voxel_mg.py:163 for x = 0. */
+int vx_restrict_sweep(int prec, int nx, int ny, int nz, const void* fine, const uint8_t* coarse_mask,
+                      void* coarse, const void* inv_diag, double omega, void* x, cudaStream_t stream);
+
 /* x += (P ec) * M on the fine grid (nx,ny,nz) from coarse (nx/2,ny/2,nz/2).
  * Replaces: src/voxel_mg.py:74-80,92-97 prolong (+ the add and mask of :171). */
 int vx_prolong_add(int prec, int nx, int ny, int nz, const void* coarse, const uint8_t* fine_mask,

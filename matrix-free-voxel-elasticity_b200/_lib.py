@@ -40,6 +40,7 @@ SIGNATURES = {
     "vx_operator_partials": (c_int64, [c_int, c_int, c_int, c_int]),
     "vx_apply_dot": (c_int, [c_int, c_int, c_int, c_int, _D, _P, _P, _P, _P, _P, _P]),
     "vx_true_residual": (c_int, [c_int, c_int, c_int, c_int, _D, _P, _P, _P, _P, _P, _P, _P]),
+    "vx_restrict_sweep": (c_int, [c_int, c_int, c_int, c_int, _P, _P, _P, _P, c_double, _P, _P]),
     "vx_restrict": (c_int, [c_int, c_int, c_int, c_int, _P, _P, _P, _P]),
     "vx_prolong_add": (c_int, [c_int, c_int, c_int, c_int, _P, _P, _P, _P]),
     "vx_coarsen_modulus": (c_int, [c_int, c_int, c_int, c_int, _P, _P, _P]),

@@ -13,81 +13,148 @@ __device__ __forceinline__ void node_coords(const Grid& g, int64_t n, int& ix, i
     ix = int(n / (int64_t(g.nz + 1) * (g.ny + 1)));
 }
 
-// Launch shape of the restriction: threads along z (TZ_T x TY_T per CTA), grid (z chunks, y rows /
-// TY_T, x planes), so no thread divides to find its node; offsets in 32 bits (fewer than 2^31 DOFs).
-constexpr int TZ_T = 64, TY_T = 2;
-inline dim3 transfer_grid(const Grid& g) {
-    return dim3(unsigned((g.nz + 1 + TZ_T - 1) / TZ_T), unsigned((g.ny + 1 + TY_T - 1) / TY_T), unsigned(g.nx + 1));
-}
 __device__ __forceinline__ int node32(const Grid& g, int ix, int iy, int iz) { return (ix * (g.ny + 1) + iy) * (g.nz + 1) + iz; }
 
-// coarse node (I,J,K) of fine grid f: rc = sum w(a) w(b) w(d) f(2I+a, 2J+b, 2K+d), w(0)=1, w(+-1)=1/2.
-// Arithmetic in arith_t<T> (bf16 storage: FP32).
-template <typename T>
-__global__ void __launch_bounds__(TZ_T * TY_T) restrict_kernel(Grid f, Grid c, const T* __restrict__ fine,
-                                                              const uint8_t* __restrict__ cmask, T* __restrict__ coarse) {
+// Restriction: coarse node (I,J,K) of fine grid f: rc = sum w(a) w(b) w(d) f(2I+a, 2J+b, 2K+d), w(0)=1,
+// w(+-1)=1/2; arithmetic in arith_t<T> (bf16 storage: FP32).
+// A thread owns one word of a fine row span and forms the x and y passes from the nine rows around its
+// coarse row (independent, fully coalesced loads; the row shared with the next coarse row is carried over,
+// the next rows' loads are in flight over the barrier), the CTA does the z pass through shared memory.  A
+// CTA takes rj coarse rows of one coarse plane.  With x != NULL the first sweep of the coarse level from
+// zero, x = omega invd r, rides on the store.  The gather of one coarse node per thread that this replaces
+// read 27 words with a stride of two nodes and was bound by its load latency.
+// Measured (us, L2 flushed, FP32 / bf16 / FP64, before -> now): 576x288x288 276 / 207 / 549 -> 209 / 195 /
+// 280 (3.1 TB/s in FP32), 256x128x128 37 / 31 / 63 -> 31 / 27 / 40.
+constexpr int RT_MAX = 256, RK_MAX = (RT_MAX / 3 - 1) / 2;       // 42 coarse nodes of a span
+template <typename T, typename X>
+__global__ void __launch_bounds__(RT_MAX) restrict_kernel(Grid f, Grid c, int rk, int rj, const T* __restrict__ fine,
+                                                          const uint8_t* __restrict__ cmask, T* __restrict__ coarse,
+                                                          const T* __restrict__ invd, double omega, X* __restrict__ x) {
     vx::pdl_begin();
     using A = arith_t<T>;
-    const int K = blockIdx.x * TZ_T + threadIdx.x, J = blockIdx.y * TY_T + threadIdx.y, I = blockIdx.z;
-    if (K > c.nz || J > c.ny) return;
-    const int n = node32(c, I, J, K);
-    const unsigned bits = cmask ? unsigned(cmask[n]) : 7u;
-    auto ld = [&](int i) { return Storage<T>::load(fine + i); };
-    for (int comp = 0; comp < 3; ++comp) {
-        A ty[3][3];   // after the x pass, at fine (y = 2J + b - 1, z = 2K + d - 1)
-        for (int b = 0; b < 3; ++b)
-            for (int d = 0; d < 3; ++d) {
-                const int fy = 2 * J + b - 1, fz = 2 * K + d - 1;
-                A v = A(0);
-                if (fy >= 0 && fy <= f.ny && fz >= 0 && fz <= f.nz) {
-                    v = ld(3 * node32(f, 2 * I, fy, fz) + comp);
-                    if (2 * I + 1 <= f.nx) v = v + A(0.5) * ld(3 * node32(f, 2 * I + 1, fy, fz) + comp);
-                    if (I >= 1) v = v + A(0.5) * ld(3 * node32(f, 2 * I - 1, fy, fz) + comp);
-                }
-                ty[b][d] = v;
-            }
-        A tz[3];
-        for (int d = 0; d < 3; ++d) {
-            A v = ty[1][d];
-            if (2 * J + 1 <= f.ny) v = v + A(0.5) * ty[2][d];
-            if (J >= 1) v = v + A(0.5) * ty[0][d];
-            tz[d] = v;
+    using Raw = typename Storage<T>::raw_t;
+    __shared__ A tz[2][RT_MAX];
+    const int t = threadIdx.x, I = blockIdx.z, K0 = blockIdx.x * rk;
+    const int nk = min(rk, c.nz + 1 - K0);                       // coarse nodes of this CTA's span
+    const bool right = 2 * I + 1 <= f.nx, left = I >= 1;
+    const int row = 3 * (f.nz + 1), plane = row * (f.ny + 1);
+    const int fw = 3 * (2 * K0 - 1) + t;                         // this thread's word of the fine row
+    const bool in = t < 3 * (2 * nk + 1) && fw >= 0 && fw < row;
+    const T* const base = fine + 2 * I * plane + (in ? fw : 0);
+    struct Row { Raw v, r, l; };                                 // unconverted: a conversion would wait for the load
+    auto load = [&](int fy) -> Row {                             // the three planes' words of fine row fy
+        Row o{Raw(0.0f), Raw(0.0f), Raw(0.0f)};
+        if (in && fy >= 0 && fy <= f.ny) {
+            const T* p = base + fy * row;
+            o.v = Storage<T>::raw(p);
+            if (right) o.r = Storage<T>::raw(p + plane);
+            if (left) o.l = Storage<T>::raw(p - plane);
         }
-        A v = tz[1];
-        if (2 * K + 1 <= f.nz) v = v + A(0.5) * tz[2];
-        if (K >= 1) v = v + A(0.5) * tz[0];
-        Storage<T>::store(coarse + 3 * n + comp, ((bits >> comp) & 1u) ? v : A(0));
+        return o;
+    };
+    auto xpass = [&](const Row& o) -> A {
+        A v = Storage<T>::cvt(o.v);
+        if (right) v = v + A(0.5) * A(Storage<T>::cvt(o.r));
+        if (left) v = v + A(0.5) * A(Storage<T>::cvt(o.l));
+        return v;
+    };
+    const int J0 = blockIdx.y * rj, J1 = min(J0 + rj, c.ny + 1);
+    const Row lo = load(2 * J0 - 1);
+    Row mi = load(2 * J0), up = load(2 * J0 + 1);
+    A below = xpass(lo);
+    const bool out = t < 3 * nk;
+    const int kk = t / 3, comp = t - 3 * kk, K = K0 + kk, w = t + 3 * kk + 3;      // coarse word t, fine word 2K
+    for (int J = J0; J < J1; ++J) {
+        A* const buf = tz[J & 1];
+        A v = xpass(mi);
+        const A above = xpass(up);
+        if (2 * J + 1 <= f.ny) v = v + A(0.5) * above;
+        if (J >= 1) v = v + A(0.5) * below;
+        below = above;
+        buf[t] = v;
+        if (J + 1 < J1) {
+            mi = load(2 * J + 2);
+            up = load(2 * J + 3);
+        }
+        __syncthreads();
+        if (out) {
+            A s = buf[w];
+            if (2 * K + 1 <= f.nz) s = s + A(0.5) * buf[w + 3];
+            if (K >= 1) s = s + A(0.5) * buf[w - 3];
+            const int n = node32(c, I, J, K);
+            const unsigned bits = cmask ? unsigned(cmask[n]) : 7u;
+            s = ((bits >> comp) & 1u) ? s : A(0);
+            Storage<T>::store(coarse + 3 * n + comp, s);
+            if (x) {
+                using B = arith_t<X>;
+                Storage<X>::store(x + 3 * n + comp, B(omega) * B(Storage<T>::load(invd + 3 * n + comp)) * B(Storage<T>::round(s)));
+            }
+        }
     }
 }
+struct RestrictShape { dim3 grid; unsigned threads; int rk, rj; };
+// Rows per CTA: the more, the fewer loads are repeated (9 a word at one row, 6.4 at eight) but the longer a
+// CTA's chain of dependent rows; eight while about 1000 CTAs are left, fewer on small grids (FP32, 1 / 2 / 4 / 8 rows: 576x288x288
+// 373 / 279 / 232 / 209 us, 128x64x64 12.3 / 10.3 / 10.2 / 12.4, 64x32x32 8.2 / 8.2 / 10.2 / 12.3).
+inline RestrictShape restrict_shape(const Grid& c) {
+    RestrictShape r;
+    const int chunks = (c.nz + 1 + RK_MAX - 1) / RK_MAX;
+    r.rk = (c.nz + 1 + chunks - 1) / chunks;
+    r.rj = 8;
+    while (r.rj > 1 && int64_t(chunks) * ((c.ny + r.rj) / r.rj) * (c.nx + 1) < 1000) r.rj /= 2;
+    r.grid = dim3(unsigned(chunks), unsigned((c.ny + r.rj) / r.rj), unsigned(c.nx + 1));
+    r.threads = unsigned((3 * (2 * r.rk + 1) + 31) / 32 * 32);
+    return r;
+}
 
-// x(i,j,k) += (P ec)(i,j,k) * mask; P is the separable trilinear interpolation.  One thread per fine
-// node in a 1-D launch: consecutive threads read and write consecutive nodes of x (measured faster
-// than the 3-D launch of the restriction, whose threads gather from three fine planes).
+// Prolongation: x(i,j,k) += (P ec)(i,j,k) * mask; P is the separable trilinear interpolation.
+// A thread owns one fine word (z, component) of the four fine rows (2I, 2I+1) x (2J, 2J+1), which
+// interpolate from the same four coarse rows: at most eight coarse loads feed four updates, and every
+// access is a run of consecutive words.  3-D launch, so no thread divides by a grid extent.
+// Bound by HBM (4.1 TB/s in FP32); measured (us, L2 flushed, FP32 / bf16 / FP64, one fine node per thread
+// -> now): 576x288x288 463 / 557 / 580 -> 309 / 330 / 549, 256x128x128 49 / 59 / 57 -> 41 / 41 / 52.
+constexpr int PT = 128;
 template <typename T>
-__global__ void prolong_add_kernel(Grid f, Grid c, const T* __restrict__ coarse, const uint8_t* __restrict__ fmask,
-                                   T* __restrict__ x) {
+__global__ void __launch_bounds__(PT) prolong_add_kernel(Grid f, Grid c, const T* __restrict__ coarse,
+                                                         const uint8_t* __restrict__ fmask, T* __restrict__ x) {
     vx::pdl_begin();
     using A = arith_t<T>;
-    const int64_t n = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (n >= f.nodes()) return;
-    int i, j, k;
-    node_coords(f, n, i, j, k);
-    const unsigned bits = fmask ? unsigned(fmask[n]) : 7u;
-    const int I0 = i >> 1, J0 = j >> 1, K0 = k >> 1;
-    const bool ox = i & 1, oy = j & 1, oz = k & 1;
-    for (int comp = 0; comp < 3; ++comp) {
-        A py[2];
-        for (int d = 0; d <= int(oz); ++d) {
-            A px[2];
-            for (int b = 0; b <= int(oy); ++b) {
-                const int64_t a0 = 3 * c.node(I0, J0 + b, K0 + d) + comp;
-                const A c0 = Storage<T>::load(coarse + a0);
-                px[b] = ox ? A(0.5) * (c0 + Storage<T>::load(coarse + a0 + 3 * int64_t(c.ny + 1) * (c.nz + 1))) : c0;
-            }
-            py[d] = oy ? A(0.5) * (px[0] + px[1]) : px[0];
-        }
-        const A v = oz ? A(0.5) * (py[0] + py[1]) : py[0];
-        if ((bits >> comp) & 1u) Storage<T>::store(x + 3 * n + comp, Storage<T>::load(x + 3 * n + comp) + v);
+    const int w = blockIdx.x * PT + threadIdx.x, J = blockIdx.y, I = blockIdx.z;
+    if (w >= 3 * (f.nz + 1)) return;
+    const int k = w / 3, comp = w - 3 * k;
+    const bool oz = k & 1, ox = 2 * I + 1 <= f.nx, oy = 2 * J + 1 <= f.ny;
+    const int crow = 3 * (c.nz + 1), cplane = crow * (c.ny + 1);
+    const T* p = coarse + I * cplane + J * crow + 3 * (k >> 1) + comp;
+    const int frow = 3 * (f.nz + 1), fplane = frow * (f.ny + 1);
+    T* px = x + 2 * I * fplane + 2 * J * frow + w;
+    const uint8_t* pm = fmask ? fmask + (2 * I * (f.ny + 1) + 2 * J) * (f.nz + 1) + k : nullptr;
+    A xo[4];
+    unsigned bits[4] = {7u, 7u, 7u, 7u};
+    #pragma unroll
+    for (int q = 0; q < 4; ++q) {                                // (x parity, y parity) = (q & 1, q >> 1)
+        if ((q & 1 && !ox) || (q >> 1 && !oy)) continue;
+        xo[q] = Storage<T>::load(px + (q & 1) * fplane + (q >> 1) * frow);
+        if (fmask) bits[q] = pm[((q & 1) * (f.ny + 1) + (q >> 1)) * (f.nz + 1)];
+    }
+    A r[2][4];                                                   // the four rows at K and K + 1
+    #pragma unroll
+    for (int d = 0; d < 2; ++d) {
+        if (d && !oz) break;
+        const A a = Storage<T>::load(p + 3 * d);
+        const A b = ox ? A(Storage<T>::load(p + 3 * d + cplane)) : a;
+        const A e = oy ? A(Storage<T>::load(p + 3 * d + crow)) : a;
+        const A g = ox && oy ? A(Storage<T>::load(p + 3 * d + cplane + crow)) : a;
+        const A ab = A(0.5) * (a + b), eg = A(0.5) * (e + g);
+        r[d][0] = a;
+        r[d][1] = ab;
+        r[d][2] = A(0.5) * (a + e);
+        r[d][3] = A(0.5) * (ab + eg);
+    }
+    #pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        if ((q & 1 && !ox) || (q >> 1 && !oy)) continue;
+        const A v = oz ? A(0.5) * (r[0][q] + r[1][q]) : r[0][q];
+        if ((bits[q] >> comp) & 1u) Storage<T>::store(px + (q & 1) * fplane + (q >> 1) * frow, xo[q] + v);
     }
 }
 
@@ -259,7 +326,7 @@ inline unsigned blocks_for(int64_t n, int t) { return unsigned((n + t - 1) / t);
 int check_even(int nx, int ny, int nz, const char* what) {
     int st = check_grid(nx, ny, nz);
     if (st) return st;
-    if (nx + 1 > 65535 || (ny + 1 + TY_T - 1) / TY_T > 65535) {      // grid dimensions of the transfer launches
+    if (nx + 1 > 65535 || (ny + 2) / 2 > 65535) {                    // grid dimensions of the transfer launches
         set_error("%s: fine grid (%d, %d, %d) is too long in x or y for one launch", what, nx, ny, nz);
         return VX_ERR_INVALID_ARGUMENT;
     }
@@ -274,19 +341,35 @@ int check_even(int nx, int ny, int nz, const char* what) {
 
 using namespace vx;
 
-extern "C" int vx_restrict(int prec, int nx, int ny, int nz, const void* fine, const uint8_t* coarse_mask,
-                           void* coarse, cudaStream_t stream) {
-    int st = check_even(nx, ny, nz, "vx_restrict");
+namespace {
+int launch_restrict(const char* what, int prec, int nx, int ny, int nz, const void* fine, const uint8_t* coarse_mask,
+                    void* coarse, const void* invd, double omega, void* x, cudaStream_t stream) {
+    int st = check_even(nx, ny, nz, what);
     if (st) return st;
-    VX_CHECK_ARG(fine && coarse, VX_ERR_NULL_POINTER, "vx_restrict: NULL pointer");
+    VX_CHECK_ARG(fine && coarse, VX_ERR_NULL_POINTER, "%s: NULL pointer", what);
     Grid f{nx, ny, nz}, c{nx / 2, ny / 2, nz / 2};
+    const RestrictShape r = restrict_shape(c);
     const bool ok = dispatch_prec(prec, [&](auto t) {             // auxiliary vectors on both sides
         using R = typename decltype(t)::R;
-        vx::launch(restrict_kernel<R>, transfer_grid(c), dim3(TZ_T, TY_T), 0, stream, f, c, (const R*)fine, coarse_mask, (R*)coarse);
+        using X = typename decltype(t)::X;
+        vx::launch(restrict_kernel<R, X>, r.grid, r.threads, 0, stream, f, c, r.rk, r.rj, (const R*)fine, coarse_mask, (R*)coarse,
+                   (const R*)invd, omega, (X*)x);
     });
-    VX_CHECK_ARG(ok, VX_ERR_INVALID_ARGUMENT, "vx_restrict: unsupported precision %d", prec);
-    VX_CHECK_LAUNCH("vx_restrict");
+    VX_CHECK_ARG(ok, VX_ERR_INVALID_ARGUMENT, "%s: unsupported precision %d", what, prec);
+    VX_CHECK_LAUNCH(what);
     return VX_OK;
+}
+}  // namespace
+
+extern "C" int vx_restrict(int prec, int nx, int ny, int nz, const void* fine, const uint8_t* coarse_mask,
+                           void* coarse, cudaStream_t stream) {
+    return launch_restrict("vx_restrict", prec, nx, ny, nz, fine, coarse_mask, coarse, nullptr, 0.0, nullptr, stream);
+}
+
+extern "C" int vx_restrict_sweep(int prec, int nx, int ny, int nz, const void* fine, const uint8_t* coarse_mask,
+                                 void* coarse, const void* inv_diag, double omega, void* x, cudaStream_t stream) {
+    VX_CHECK_ARG(inv_diag && x, VX_ERR_NULL_POINTER, "vx_restrict_sweep: NULL pointer");
+    return launch_restrict("vx_restrict_sweep", prec, nx, ny, nz, fine, coarse_mask, coarse, inv_diag, omega, x, stream);
 }
 
 extern "C" int vx_prolong_add(int prec, int nx, int ny, int nz, const void* coarse, const uint8_t* fine_mask,
@@ -297,7 +380,8 @@ extern "C" int vx_prolong_add(int prec, int nx, int ny, int nz, const void* coar
     Grid f{nx, ny, nz}, c{nx / 2, ny / 2, nz / 2};
     const bool ok = dispatch_prec(prec, [&](auto t) {             // iterates on both sides
         using X = typename decltype(t)::X;
-        vx::launch(prolong_add_kernel<X>, blocks_for(f.nodes(), 256), 256, 0, stream, f, c, (const X*)coarse, fine_mask, (X*)x);
+        const dim3 grid(blocks_for(3 * (int64_t(nz) + 1), PT), unsigned(c.ny + 1), unsigned(c.nx + 1));
+        vx::launch(prolong_add_kernel<X>, grid, PT, 0, stream, f, c, (const X*)coarse, fine_mask, (X*)x);
     });
     VX_CHECK_ARG(ok, VX_ERR_INVALID_ARGUMENT, "vx_prolong_add: unsupported precision %d", prec);
     VX_CHECK_LAUNCH("vx_prolong_add");

@@ -354,10 +354,11 @@ class MGHierarchy:
         res = bufs[1 - ci] if L.res is None else L.res
         L.op.residual(bufs[ci], r, L.E, L.mask, out=res)
         nxt = self.levels[l + 1]
-        _lib.call("vx_restrict", self.prec, *L.shape, res.data_ptr(), nxt.mask.data_ptr(), nxt.r.data_ptr(), _s())
-        if l + 1 < len(self.levels) - 1:
-            _lib.call("vx_scaled_product", self.prec, nxt.n, nxt.omega, nxt.invd.data_ptr(), nxt.r.data_ptr(),
-                      nxt.x.data_ptr(), _s())
+        if l + 1 < len(self.levels) - 1:                    # the coarse level's first sweep rides on the restriction
+            _lib.call("vx_restrict_sweep", self.prec, *L.shape, res.data_ptr(), nxt.mask.data_ptr(), nxt.r.data_ptr(),
+                      nxt.invd.data_ptr(), nxt.omega, nxt.x.data_ptr(), _s())
+        else:
+            _lib.call("vx_restrict", self.prec, *L.shape, res.data_ptr(), nxt.mask.data_ptr(), nxt.r.data_ptr(), _s())
         xc = self._level(l + 1, nxt.r)
         _lib.call("vx_prolong_add", self.prec, *L.shape, xc.data_ptr(), L.mask.data_ptr(), bufs[ci].data_ptr(), _s())
         for _ in range(self.post):

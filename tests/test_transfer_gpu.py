@@ -93,3 +93,25 @@ def test_restriction_is_the_transpose_of_prolongation():
     _lib.call("vx_prolong_add", _lib.VX_F64, *shape, u.data_ptr(), None, Pu.data_ptr(), _s())
     a, b = float(Rr @ u), float(r @ Pu)
     assert abs(a - b) <= 1e-13 * max(abs(a), abs(b))
+
+
+@pytest.mark.parametrize("shape", [(36, 18, 64), (8, 130, 130), (4, 66, 172), (32, 2, 84)])
+@pytest.mark.parametrize("dtype,aux", [(torch.float64, torch.float64), (torch.float32, torch.float32),
+                                       (torch.float32, torch.bfloat16), (torch.bfloat16, torch.bfloat16)])
+def test_restriction_with_the_first_coarse_sweep(shape, dtype, aux):
+    """vx_restrict_sweep leaves vx_restrict's coarse vector and vx_scaled_product's x, bit for bit, at
+    spans of the coarse row of one CTA (42 nodes) and of several."""
+    rng = np.random.default_rng(sum(shape))
+    coarse = tuple(s // 2 for s in shape)
+    nf, nc = 3 * vo.n_nodes(shape), 3 * vo.n_nodes(coarse)
+    prec = vx.operators.STORAGE[(dtype, aux)]
+    rf = torch.as_tensor(rng.standard_normal(nf), device="cuda").to(aux)
+    d = torch.as_tensor(rng.random(nc), device="cuda").to(aux)
+    cm = torch.as_tensor(_masks(coarse, rng), device="cuda")
+    rc, rs = (torch.empty(nc, dtype=aux, device="cuda") for _ in range(2))
+    xc, xs = (torch.empty(nc, dtype=dtype, device="cuda") for _ in range(2))
+    _lib.call("vx_restrict", prec, *shape, rf.data_ptr(), cm.data_ptr(), rc.data_ptr(), _s())
+    _lib.call("vx_scaled_product", prec, nc, 0.6, d.data_ptr(), rc.data_ptr(), xc.data_ptr(), _s())
+    _lib.call("vx_restrict_sweep", prec, *shape, rf.data_ptr(), cm.data_ptr(), rs.data_ptr(), d.data_ptr(), 0.6,
+              xs.data_ptr(), _s())
+    assert torch.equal(rs, rc) and torch.equal(xs, xc)
