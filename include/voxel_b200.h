@@ -380,6 +380,36 @@ int vx_cg_direction(int prec, int zprec, int64_t n, const double* S, const void*
                     cudaStream_t stream);
 int vx_dots_pr(int prec, int zprec, int64_t n, const void* r, const void* zn, const void* zo,
                double* partials, cudaStream_t stream);
+
+/* Reductions finished in the kernel that forms the partials: the CTA that arrives last sums them in
+ * vx_solver_finalize's order and applies its recurrence `op` to S.  *counter (device, 4 bytes) is 0
+ * before the call and again when the kernel has completed; calls that share it must be ordered.
+ * prec of the operator forms may carry VX_STREAM_XP (a finalize launch then follows). */
+int vx_dots_pr_fin(int op, int prec, int zprec, int64_t n, const void* r, const void* zn, const void* zo,
+                   double* partials, double* S, unsigned* counter, cudaStream_t stream);
+int vx_apply_dot_fin(int op, int prec, int nx, int ny, int nz, const double* blocks, const void* E,
+                     const uint8_t* node_mask, const void* p, void* q, double* partials, double* S,
+                     unsigned* counter, cudaStream_t stream);
+int vx_true_residual_fin(int op, int prec, int nx, int ny, int nz, const double* blocks, const void* E,
+                         const uint8_t* node_mask, const void* x, const void* b, void* res, double* partials,
+                         double* S, unsigned* counter, cudaStream_t stream);
+/* One FP64 Jacobi-preconditioned CG step: with update, x += alpha p and r -= alpha q (not once the loop
+ * has converged or broken down); z <- inv_diag r; then beta from r . z and r . (z - z_old), z_old being z
+ * as it was.  partials: vx_jacobi_step_partials(n) doubles. */
+int64_t vx_jacobi_step_partials(int64_t n);
+int vx_jacobi_step(int64_t n, double* S, double* x, const double* p, double* r, const double* q,
+                   const double* inv_diag, double* z, int update, double* partials, unsigned* counter,
+                   cudaStream_t stream);
+/* The same iteration on small systems (n <= vx_small_cg_limit()) with every CTA summing the partials it needs:
+ * vx_small_step takes alpha from the G partials pq of vx_apply_dot (fin; recurrence of FIN_PQ) and updates x,
+ * and with step also r, z and the partials (vx_jacobi_step_partials(n) doubles) from which vx_small_direction
+ * takes beta for p = z + beta p.  rz travels in S[7] (after the direction) and S[0] (after the step). */
+int64_t vx_small_cg_limit(void);
+int vx_small_step(int64_t n, int64_t G, const double* pq, double* S, double* x, const double* p, double* r,
+                  const double* q, const double* inv_diag, double* z, int fin, int step, double* partials,
+                  cudaStream_t stream);
+int vx_small_direction(int64_t n, const double* partials, double* S, const double* z, double* p,
+                       cudaStream_t stream);
 /* FP64 x += S[alpha] p (skipped once S says done or breakdown) followed by vx_cg_direction, with p
  * read once: the x update of src/voxel_mg.py:199 deferred into the direction update of :209 on the
  * iterations that do not test the true residual.  z, z_old iterates of `zprec`. */

@@ -40,6 +40,14 @@ SIGNATURES = {
     "vx_operator_partials": (c_int64, [c_int, c_int, c_int, c_int]),
     "vx_apply_dot": (c_int, [c_int, c_int, c_int, c_int, _D, _P, _P, _P, _P, _P, _P]),
     "vx_true_residual": (c_int, [c_int, c_int, c_int, c_int, _D, _P, _P, _P, _P, _P, _P, _P]),
+    "vx_dots_pr_fin": (c_int, [c_int, c_int, c_int, c_int64, _P, _P, _P, _P, _P, _P, _P]),
+    "vx_apply_dot_fin": (c_int, [c_int, c_int, c_int, c_int, c_int, _D, _P, _P, _P, _P, _P, _P, _P, _P]),
+    "vx_true_residual_fin": (c_int, [c_int, c_int, c_int, c_int, c_int, _D, _P, _P, _P, _P, _P, _P, _P, _P, _P]),
+    "vx_small_cg_limit": (c_int64, []),
+    "vx_small_step": (c_int, [c_int64, c_int64, _P, _P, _P, _P, _P, _P, _P, _P, c_int, c_int, _P, _P]),
+    "vx_small_direction": (c_int, [c_int64, _P, _P, _P, _P, _P]),
+    "vx_jacobi_step_partials": (c_int64, [c_int64]),
+    "vx_jacobi_step": (c_int, [c_int64, _P, _P, _P, _P, _P, _P, _P, c_int, _P, _P, _P]),
     "vx_restrict_sweep": (c_int, [c_int, c_int, c_int, c_int, _P, _P, _P, _P, c_double, _P, _P]),
     "vx_restrict": (c_int, [c_int, c_int, c_int, c_int, _P, _P, _P, _P]),
     "vx_prolong_add": (c_int, [c_int, c_int, c_int, c_int, _P, _P, _P, _P]),
@@ -149,7 +157,7 @@ CAPTURE_STREAM = None
 KERNELS_PER_CALL = {"vx_tc_element_product": 1, "vx_coarse_pack_factor": 3, "vx_dots": 2, "vx_assemble_dense": 1, "vx_true_residual_noalloc": 2, "vx_coarse_apply_factor": 2,
                     "vx_batch_coarse_apply_factor": 2}
 HOST_ONLY = {"vx_last_error", "vx_version", "vx_element_matrix", "vx_element", "vx_parity_blocks",
-             "vx_operator_partials", "vx_partials_size", "vx_solver_slots", "vx_solver_partials",
+             "vx_operator_partials", "vx_partials_size", "vx_jacobi_step_partials", "vx_small_cg_limit", "vx_solver_slots", "vx_solver_partials",
              "vx_graph_while_begin", "vx_graph_destroy", "vx_capture_status", "vx_graph_launch",
              "vx_oc_partials", "vx_graph_body_nodes", "vx_plane_fix_partials", "vx_device_status",
              "vx_coarse_factor_workspace", "vx_set_stream_kernel",

@@ -403,6 +403,10 @@ parity_march(const __grid_constant__ OpArgs2<TC, TU, TE, TY, TR> args) {
     if constexpr (EPI == EPI_TRUE_RES || EPI == EPI_APPLY_DOT) {
         const int64_t bid = (int64_t(blockIdx.z) * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;
         block_sum_store<NWS * 32>(acc, a.partials + bid);
+        if (a.counter) {
+            static_assert(NWS * 32 == FT, "the last CTA finishes the reduction with FT threads");
+            finalize_last(a.fin, int64_t(gridDim.x) * gridDim.y * gridDim.z, a.partials, a.S, a.counter);
+        }
     }
 }
 

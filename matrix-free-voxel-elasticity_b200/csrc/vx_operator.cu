@@ -16,7 +16,7 @@
 //   on the grid boundary.
 // dense_gather: the reference's node-owned dense 24x24 mapping (independent control path).
 // diag / energy / coarse-grid helpers.
-#include "vx_common.cuh"
+#include "vx_finalize.cuh"
 #include <climits>
 #include "vx_pair.cuh"
 
@@ -50,6 +50,9 @@ struct OpArgs {
     TC omega;
     double* partials;         // TRUE_RES (|res|^2) / APPLY_DOT (p.q): one double per CTA
     int dot_x0, dot_x1;       // node planes [dot_x0, dot_x1) enter the partial sums
+    int fin;                  // with counter: the reduction the last CTA finishes (FinOp) into S
+    double* S;
+    unsigned* counter;
     double emin, de, penal;   // SIMP modulus E = emin + de * rho^penal
     int cx;                   // owned node planes per CTA (x chunk)
     bool cubic;               // host side: the blocks have the cube pattern (CubeK)
@@ -1135,7 +1138,8 @@ namespace {
 template <int EPI>
 int fused_dispatch(const char* what, int sel, int nx, int ny, int nz, const double* blocks, const void* E,
                    const uint8_t* node_mask, const void* x, const void* r, const void* invd, double omega,
-                   void* out, double* partials, cudaStream_t stream, int dot_x0 = 0, int dot_x1 = INT_MAX) {
+                   void* out, double* partials, cudaStream_t stream, int dot_x0 = 0, int dot_x1 = INT_MAX, int fin = 0,
+                   double* S = nullptr, unsigned* counter = nullptr) {
     const int prec = sel & ~VX_STREAM_XP;
     int st = check_grid(nx, ny, nz);
     if (st) return st;
@@ -1161,6 +1165,7 @@ int fused_dispatch(const char* what, int sel, int nx, int ny, int nz, const doub
             a.u = (const X*)x; a.E = (const M*)E; a.y = (TY*)out; a.node_mask = node_mask;
             a.r = (const R*)r; a.invd = (const R*)invd; a.omega = TC(omega); a.partials = partials;
             a.dot_x0 = dot_x0; a.dot_x1 = dot_x1;
+            a.fin = fin; a.S = S; a.counter = counter;
             a.C = convert_blocks<TC>(blocks);
             a.cubic = cube_pattern(blocks);
             a.xp = sel & VX_STREAM_XP;
@@ -1209,6 +1214,38 @@ extern "C" int vx_true_residual(int prec, int nx, int ny, int nz, const double* 
     VX_CHECK_ARG(b && partials, VX_ERR_NULL_POINTER, "vx_true_residual: NULL b / partials");
     return fused_dispatch<EPI_TRUE_RES>("vx_true_residual", prec, nx, ny, nz, blocks, E, node_mask, x, b,
                                         nullptr, 0.0, res, partials, stream);
+}
+
+// The reducing forms followed by their finalisation (vx_solver_finalize): parity_march finishes the
+// reduction in its last CTA, the other kernels launch the finalize kernel.
+namespace {
+template <int EPI>
+int fused_fin(const char* what, int op, int sel, int nx, int ny, int nz, const double* blocks, const void* E,
+              const uint8_t* node_mask, const void* x, const void* r, void* out, double* partials, double* S,
+              unsigned* counter, cudaStream_t stream) {
+    VX_CHECK_ARG(partials && S && counter, VX_ERR_NULL_POINTER, "%s: NULL pointer", what);
+    VX_CHECK_ARG(op >= 0 && op <= FIN_RR_ONLY && op != FIN_BETA_PR, VX_ERR_INVALID_ARGUMENT, "%s: bad op %d", what, op);
+    const bool march = stream_kind(true, sel & VX_STREAM_XP) == VX_KERNEL_MARCH;
+    int st = fused_dispatch<EPI>(what, sel, nx, ny, nz, blocks, E, node_mask, x, r, nullptr, 0.0, out, partials, stream, 0,
+                                 INT_MAX, op, S, march ? counter : nullptr);
+    if (st || march) return st;
+    return vx_solver_finalize(op, stream_ctas(Grid{nx, ny, nz}, sel), partials, S, stream);
+}
+}  // namespace
+
+extern "C" int vx_apply_dot_fin(int op, int prec, int nx, int ny, int nz, const double* blocks, const void* E,
+                                const uint8_t* node_mask, const void* p, void* q, double* partials, double* S,
+                                unsigned* counter, cudaStream_t stream) {
+    return fused_fin<EPI_APPLY_DOT>("vx_apply_dot_fin", op, prec, nx, ny, nz, blocks, E, node_mask, p, nullptr, q, partials,
+                                    S, counter, stream);
+}
+
+extern "C" int vx_true_residual_fin(int op, int prec, int nx, int ny, int nz, const double* blocks, const void* E,
+                                    const uint8_t* node_mask, const void* x, const void* b, void* res, double* partials,
+                                    double* S, unsigned* counter, cudaStream_t stream) {
+    VX_CHECK_ARG(b, VX_ERR_NULL_POINTER, "vx_true_residual_fin: NULL b");
+    return fused_fin<EPI_TRUE_RES>("vx_true_residual_fin", op, prec, nx, ny, nz, blocks, E, node_mask, x, b, res, partials,
+                                   S, counter, stream);
 }
 
 // The reducing forms with the sums restricted to node planes x_lo <= ix < x_hi (the output is

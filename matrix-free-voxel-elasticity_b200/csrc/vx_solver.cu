@@ -7,93 +7,17 @@
 // body captured as the body of a conditional WHILE graph node, a complete solve is a single graph
 // launch with no host round trip per iteration; the condition kernel stops the loop on
 // convergence, on breakdown or at maxiter.
-#include "vx_common.cuh"
+#include "vx_finalize.cuh"
+#include <algorithm>
 
 namespace vx {
-
-constexpr int FT = 256;
-
-enum Slot {
-    S_RZ = 0, S_PQ = 1, S_ALPHA = 2, S_RR = 3, S_REL = 4, S_NB = 5, S_BETA = 6, S_RZN = 7, S_RZD = 8,
-    S_TOL = 9, S_DONE = 10, S_IT = 11, S_MAXIT = 12, S_MV = 13, S_BREAK = 14, S_CHECK = 15, S_COUNT = 16
-};
-
-enum FinOp {
-    FIN_PQ = 0,        // S[PQ] = sum; alpha = rz / pq (breakdown if pq == 0); it += 1; mv += 1
-    FIN_TRUE = 1,      // S[RR] = sum; rel = sqrt(rr) / nb; mv += 1; done if rel <= tol
-    FIN_BETA_PR = 2,   // rzn = sum0, rzd = sum1; beta = rzd / rz; rz = rzn      (flexible / Polak-Ribiere)
-    FIN_BETA_FR = 3,   // rzn = sum0; beta = rzn / rz; rz = rzn                  (Fletcher-Reeves)
-    FIN_NB = 4,        // nb = sqrt(sum)
-    FIN_RZ = 5,        // rz = sum0
-    FIN_RR_ONLY = 6    // rr = sum; rel = sqrt(rr) / nb (no counters, no flag)
-};
-
-__device__ __forceinline__ double warp_sum(double v) {
-    #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-    return v;
-}
-
-__device__ double block_sum_ft(double v) {
-    __shared__ double red[FT / 32];
-    v = warp_sum(v);
-    __syncthreads();
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
-    __syncthreads();
-    double s = 0.0;
-    if (threadIdx.x < 32) s = warp_sum(threadIdx.x < FT / 32 ? red[threadIdx.x] : 0.0);
-    return s;
-}
 
 // Slot blockIdx.y (a batch of independent systems solved in lockstep) uses S + 16 slot and
 // partials + slot * pstride; unbatched launches have one slot.
 __global__ void __launch_bounds__(FT) finalize_kernel(int op, int64_t G, const double* __restrict__ partials,
                                                       double* __restrict__ S, int64_t pstride) {
     vx::pdl_begin();
-    S += S_COUNT * int64_t(blockIdx.y);
-    partials += pstride * int64_t(blockIdx.y);
-    double s0 = 0.0, s1 = 0.0;
-    for (int64_t j = threadIdx.x; j < G; j += FT) s0 += partials[j];
-    s0 = block_sum_ft(s0);
-    if (op == FIN_BETA_PR) {
-        for (int64_t j = threadIdx.x; j < G; j += FT) s1 += partials[G + j];
-        s1 = block_sum_ft(s1);
-    }
-    if (threadIdx.x != 0) return;
-    switch (op) {
-        case FIN_PQ:
-            if (S[S_DONE] != 0.0) break;            // a converged warm start: the body is a no-op
-            S[S_PQ] = s0;
-            S[S_MV] += 1.0;
-            if (s0 == 0.0 || !isfinite(s0)) { S[S_BREAK] = 1.0; S[S_ALPHA] = 0.0; }   // no step is taken
-            else { S[S_ALPHA] = S[S_RZ] / s0; S[S_IT] += 1.0; }
-            break;
-        case FIN_TRUE:
-            if (S[S_DONE] != 0.0) break;
-            S[S_RR] = s0;
-            S[S_REL] = sqrt(s0) / S[S_NB];
-            S[S_MV] += 1.0;
-            if (S[S_REL] <= S[S_TOL]) S[S_DONE] = 1.0;
-            if (!isfinite(S[S_REL])) S[S_BREAK] = 1.0;
-            break;
-        case FIN_BETA_PR:
-            S[S_RZN] = s0;
-            S[S_RZD] = s1;
-            S[S_BETA] = s1 / S[S_RZ];
-            S[S_RZ] = s0;
-            break;
-        case FIN_BETA_FR:
-            S[S_RZN] = s0;
-            S[S_BETA] = s0 / S[S_RZ];
-            S[S_RZ] = s0;
-            break;
-        case FIN_NB: S[S_NB] = sqrt(s0); break;
-        case FIN_RZ: S[S_RZ] = s0; break;
-        case FIN_RR_ONLY:
-            S[S_RR] = s0;
-            S[S_REL] = sqrt(s0) / S[S_NB];
-            break;
-    }
+    fin_reduce(op, G, partials + pstride * int64_t(blockIdx.y), S + S_COUNT * int64_t(blockIdx.y));
 }
 
 // x += alpha p; r -= alpha q (r update skipped when it is about to be replaced by b - A x).
@@ -153,7 +77,8 @@ __global__ void cg_direction_update_kernel(int64_t n, const double* __restrict__
 // (slot blockIdx.y: vectors at slot * vs, partials at slot * 2G)
 template <typename T, typename TZ>
 __global__ void __launch_bounds__(FT) dots_pr_kernel(int64_t n, const T* __restrict__ r, const TZ* __restrict__ zn,
-                                                     const TZ* __restrict__ zo, double* __restrict__ partials, int64_t vs) {
+                                                     const TZ* __restrict__ zo, double* partials, int64_t vs,
+                                                     int fin, double* S, unsigned* counter) {
     vx::pdl_begin();
     const int64_t G = gridDim.x;
     {
@@ -164,6 +89,7 @@ __global__ void __launch_bounds__(FT) dots_pr_kernel(int64_t n, const T* __restr
         partials += 2 * G * int64_t(blockIdx.y);
     }
     double a = 0.0, b = 0.0;
+    #pragma unroll 4
     for (int64_t i = int64_t(blockIdx.x) * FT + threadIdx.x; i < n; i += G * FT) {
         const double ri = double(r[i]), zi = double(Storage<TZ>::load(zn + i));
         a = fma(ri, zi, a);
@@ -175,6 +101,138 @@ __global__ void __launch_bounds__(FT) dots_pr_kernel(int64_t n, const T* __restr
         b = block_sum_ft(b);
         if (threadIdx.x == 0) partials[G + blockIdx.x] = b;
     }
+    if (counter) finalize_last(fin, G, partials, S, counter);
+}
+
+// One Jacobi-preconditioned CG step between two operator applications: x += alpha p, r -= alpha q (skipped
+// when update is 0 or once the loop has converged or broken down), z = d r over the previous z, the partials
+// of r . z and r . (z - z_old) and, in the last CTA, beta.  One pass over each vector where the separate
+// update, product, dots and finalize kernels read r three times and z twice; on small grids, where every
+// launch costs 2 to 3 us, three launches less an iteration.
+__global__ void __launch_bounds__(FT) jacobi_step_kernel(int64_t n, double* S, double* __restrict__ x,
+                                                         const double* __restrict__ p, double* __restrict__ r,
+                                                         const double* __restrict__ q, const double* __restrict__ d,
+                                                         double* __restrict__ z, int update, double* partials,
+                                                         unsigned* counter) {
+    vx::pdl_begin();
+    const int64_t G = gridDim.x;
+    const bool move = update && S[S_DONE] == 0.0 && S[S_BREAK] == 0.0;
+    const double alpha = S[S_ALPHA];
+    double a = 0.0, b = 0.0;
+    for (int64_t i = int64_t(blockIdx.x) * FT + threadIdx.x; i < n; i += G * FT) {
+        double ri = r[i];
+        if (move) {
+            x[i] = x[i] + alpha * p[i];
+            ri = ri - alpha * q[i];
+            r[i] = ri;
+        }
+        const double zo = z[i], zi = d[i] * ri;
+        z[i] = zi;
+        a = fma(ri, zi, a);
+        b = fma(ri, zi - zo, b);
+    }
+    a = block_sum_ft(a);
+    b = block_sum_ft(b);
+    if (threadIdx.x == 0) {
+        partials[blockIdx.x] = a;
+        partials[G + blockIdx.x] = b;
+    }
+    finalize_last(FIN_BETA_PR, G, partials, S, counter);
+}
+
+// The same iteration for small grids (at most SMALL_CTAS CTAs of one entry per thread), where the hand-over of
+// a sum through the last CTA (a fence, an atomic, the partials' and scalars' round trips: 2 to 3 us) costs
+// more than the work: every CTA of the kernel that needs a sum adds up the partials itself, in the same
+// order, and CTA 0 alone writes the scalars.  No kernel reads a slot that it writes: the step takes rz from
+// S_RZN and leaves it in S_RZ, the direction takes S_RZ and leaves the new one in S_RZN.
+// 32x16x16, 700 iterations: 12.8 -> 9.0 us an iteration (separate update, product, dots and
+// finalize kernels: 15.2).
+constexpr int64_t SMALL_CTAS = 1184;
+__device__ __forceinline__ double sum_partials(int64_t G, const double* __restrict__ partials) {
+    __shared__ double total;
+    double s = 0.0;
+    #pragma unroll 4
+    for (int64_t j = threadIdx.x; j < G; j += FT) s += partials[j];
+    s = block_sum_ft(s);
+    if (threadIdx.x == 0) total = s;
+    __syncthreads();
+    s = total;
+    __syncthreads();
+    return s;
+}
+
+// alpha = rz / (p . q) from the G partials pq (FIN_PQ), then x += alpha p and, with step, r -= alpha q, z = d r
+// and the partials of r . z and r . (z - z_old); fin 0 (after a true residual) skips alpha and the updates.
+__global__ void __launch_bounds__(FT) small_step_kernel(int64_t n, int64_t G, const double* __restrict__ pq, double* S,
+                                                        double* __restrict__ x, const double* __restrict__ p,
+                                                        double* __restrict__ r, const double* __restrict__ q,
+                                                        const double* __restrict__ d, double* __restrict__ z,
+                                                        int fin, int step, double* __restrict__ partials) {
+    vx::pdl_begin();
+    const int64_t i = int64_t(blockIdx.x) * FT + threadIdx.x;
+    const bool in = i < n;
+    double xi = 0.0, pi = 0.0, ri = 0.0, qi = 0.0, di = 0.0, zo = 0.0;
+    if (in) {
+        if (fin) { xi = x[i]; pi = p[i]; }
+        if (step) { ri = r[i]; di = d[i]; zo = z[i]; if (fin) qi = q[i]; }
+    }
+    if (fin) {
+        const double rz = S[S_RZN];
+        const bool done = S[S_DONE] != 0.0, broken = S[S_BREAK] != 0.0;
+        const double s = sum_partials(G, pq);
+        const bool stop = s == 0.0 || !isfinite(s);
+        const double alpha = stop ? 0.0 : rz / s;
+        if (blockIdx.x == 0 && threadIdx.x == 0) {
+            S[S_RZ] = rz;
+            if (!done) {
+                S[S_PQ] = s;
+                S[S_MV] += 1.0;
+                S[S_ALPHA] = alpha;
+                if (stop) S[S_BREAK] = 1.0;
+                else S[S_IT] += 1.0;
+            }
+        }
+        if (in && !done && !broken && !stop) {
+            x[i] = xi + alpha * pi;
+            if (step) {
+                ri = ri - alpha * qi;
+                r[i] = ri;
+            }
+        }
+    }
+    if (!step) return;
+    const double zi = di * ri;
+    if (in) z[i] = zi;
+    const double a = block_sum_ft(ri * zi), b = block_sum_ft(ri * (zi - zo));
+    if (threadIdx.x == 0) {
+        partials[blockIdx.x] = a;
+        partials[gridDim.x + blockIdx.x] = b;
+    }
+}
+
+// beta from the step's partials (FIN_BETA_PR), p = z + beta p
+__global__ void __launch_bounds__(FT) small_direction_kernel(int64_t n, const double* __restrict__ partials, double* S,
+                                                             const double* __restrict__ z, double* __restrict__ p) {
+    vx::pdl_begin();
+    const int64_t i = int64_t(blockIdx.x) * FT + threadIdx.x, G = gridDim.x;
+    const bool in = i < n;
+    const double zi = in ? z[i] : 0.0, pi = in ? p[i] : 0.0, rz = S[S_RZ];
+    double s0 = 0.0, s1 = 0.0;
+    #pragma unroll 4
+    for (int64_t j = threadIdx.x; j < G; j += FT) { s0 += partials[j]; s1 += partials[G + j]; }
+    __shared__ double beta_s;
+    s0 = block_sum_ft(s0);
+    s1 = block_sum_ft(s1);
+    if (threadIdx.x == 0) {
+        beta_s = s1 / rz;
+        if (blockIdx.x == 0) {
+            S[S_RZN] = s0;
+            S[S_RZD] = s1;
+            S[S_BETA] = beta_s;
+        }
+    }
+    __syncthreads();
+    if (in) p[i] = zi + beta_s * pi;
 }
 
 // z = d * r (Jacobi) with partial r . z
@@ -258,6 +316,9 @@ __global__ void condition_kernel(cudaGraphConditionalHandle h, const double* __r
     }
 }
 
+// one entry per thread while the partials stay few: on small grids the step is one memory round trip
+int64_t step_ctas(int64_t n) { return std::min<int64_t>((n + FT - 1) / FT, 1184); }
+
 int64_t fixed_ctas(int64_t n) {
     int64_t g = (n + FT * 8 - 1) / (FT * 8);
     return g < 1 ? 1 : (g > 1184 ? 1184 : g);
@@ -334,22 +395,75 @@ extern "C" int vx_cg_direction_update(int zprec, int64_t n, const double* S, con
     return VX_OK;
 }
 
+namespace {
+int launch_dots_pr(const char* what, int prec, int zprec, int64_t n, const void* r, const void* zn, const void* zo,
+                   double* partials, int fin, double* S, unsigned* counter, cudaStream_t stream) {
+    VX_CHECK_ARG(n > 0, VX_ERR_INVALID_ARGUMENT, "%s: n must be positive", what);
+    VX_CHECK_ARG(r && zn && partials, VX_ERR_NULL_POINTER, "%s: NULL pointer", what);
+    const unsigned G = unsigned(fixed_ctas(n));
+    auto go = [&](auto rt, auto zt) {
+        using T = decltype(rt);
+        using TZ = decltype(zt);
+        vx::launch(dots_pr_kernel<T, TZ>, G, FT, 0, stream, n, (const T*)r, (const TZ*)zn, (const TZ*)zo, partials,
+                   int64_t(0), fin, S, counter);
+    };
+    if (prec == VX_F64 && zprec == VX_F64) go(double(), double());
+    else if (prec == VX_F64 && zprec == VX_F32) go(double(), float());
+    else if (prec == VX_F64 && zprec == VX_BF16_F32) go(double(), __nv_bfloat16());
+    else if (prec == VX_F32 && zprec == VX_F32) go(float(), float());
+    else { set_error("%s: unsupported precisions %d/%d", what, prec, zprec); return VX_ERR_INVALID_ARGUMENT; }
+    VX_CHECK_LAUNCH(what);
+    return VX_OK;
+}
+}  // namespace
+
 extern "C" int vx_dots_pr(int prec, int zprec, int64_t n, const void* r, const void* zn, const void* zo,
                           double* partials, cudaStream_t stream) {
-    VX_CHECK_ARG(n > 0, VX_ERR_INVALID_ARGUMENT, "vx_dots_pr: n must be positive");
-    VX_CHECK_ARG(r && zn && partials, VX_ERR_NULL_POINTER, "vx_dots_pr: NULL pointer");
-    const unsigned G = unsigned(fixed_ctas(n));
-    if (prec == VX_F64 && zprec == VX_F64)
-        vx::launch(dots_pr_kernel<double, double>, G, FT, 0, stream, n, (const double*)r, (const double*)zn, (const double*)zo, partials, int64_t(0));
-    else if (prec == VX_F64 && zprec == VX_F32)
-        vx::launch(dots_pr_kernel<double, float>, G, FT, 0, stream, n, (const double*)r, (const float*)zn, (const float*)zo, partials, int64_t(0));
-    else if (prec == VX_F64 && zprec == VX_BF16_F32)
-        vx::launch(dots_pr_kernel<double, __nv_bfloat16>, G, FT, 0, stream, n, (const double*)r, (const __nv_bfloat16*)zn,
-                                                                    (const __nv_bfloat16*)zo, partials, int64_t(0));
-    else if (prec == VX_F32 && zprec == VX_F32)
-        vx::launch(dots_pr_kernel<float, float>, G, FT, 0, stream, n, (const float*)r, (const float*)zn, (const float*)zo, partials, int64_t(0));
-    else { set_error("vx_dots_pr: unsupported precisions %d/%d", prec, zprec); return VX_ERR_INVALID_ARGUMENT; }
-    VX_CHECK_LAUNCH("vx_dots_pr");
+    return launch_dots_pr("vx_dots_pr", prec, zprec, n, r, zn, zo, partials, 0, nullptr, nullptr, stream);
+}
+
+extern "C" int vx_dots_pr_fin(int op, int prec, int zprec, int64_t n, const void* r, const void* zn, const void* zo,
+                              double* partials, double* S, unsigned* counter, cudaStream_t stream) {
+    VX_CHECK_ARG(op >= 0 && op <= FIN_RR_ONLY && (op != FIN_BETA_PR || zo), VX_ERR_INVALID_ARGUMENT, "vx_dots_pr_fin: bad op");
+    VX_CHECK_ARG(S && counter, VX_ERR_NULL_POINTER, "vx_dots_pr_fin: NULL pointer");
+    return launch_dots_pr("vx_dots_pr_fin", prec, zprec, n, r, zn, zo, partials, op, S, counter, stream);
+}
+
+extern "C" int64_t vx_jacobi_step_partials(int64_t n) { return n > 0 ? 2 * step_ctas(n) : 2; }
+
+extern "C" int vx_jacobi_step(int64_t n, double* S, double* x, const double* p, double* r, const double* q,
+                              const double* inv_diag, double* z, int update, double* partials, unsigned* counter,
+                              cudaStream_t stream) {
+    VX_CHECK_ARG(n > 0, VX_ERR_INVALID_ARGUMENT, "vx_jacobi_step: n must be positive");
+    VX_CHECK_ARG(S && r && inv_diag && z && partials && counter && (!update || (x && p && q)), VX_ERR_NULL_POINTER,
+                 "vx_jacobi_step: NULL pointer");
+    vx::launch(jacobi_step_kernel, unsigned(step_ctas(n)), FT, 0, stream, n, S, x, p, r, q, inv_diag, z, update, partials,
+               counter);
+    VX_CHECK_LAUNCH("vx_jacobi_step");
+    return VX_OK;
+}
+
+extern "C" int64_t vx_small_cg_limit(void) { return SMALL_CTAS * FT; }
+
+extern "C" int vx_small_step(int64_t n, int64_t G, const double* pq, double* S, double* x, const double* p, double* r,
+                             const double* q, const double* inv_diag, double* z, int fin, int step, double* partials,
+                             cudaStream_t stream) {
+    VX_CHECK_ARG(n > 0 && n <= SMALL_CTAS * FT && (fin || step) && (!fin || G > 0), VX_ERR_INVALID_ARGUMENT,
+                 "vx_small_step: bad sizes");
+    VX_CHECK_ARG(S && (!fin || (pq && x && p)) && (!step || (r && inv_diag && z && partials)) && (!(fin && step) || q),
+                 VX_ERR_NULL_POINTER, "vx_small_step: NULL pointer");
+    vx::launch(small_step_kernel, unsigned(step_ctas(n)), FT, 0, stream, n, G, pq, S, x, p, r, q, inv_diag, z, fin, step,
+               partials);
+    VX_CHECK_LAUNCH("vx_small_step");
+    return VX_OK;
+}
+
+extern "C" int vx_small_direction(int64_t n, const double* partials, double* S, const double* z, double* p,
+                                  cudaStream_t stream) {
+    VX_CHECK_ARG(n > 0 && n <= SMALL_CTAS * FT, VX_ERR_INVALID_ARGUMENT, "vx_small_direction: bad size");
+    VX_CHECK_ARG(partials && S && z && p, VX_ERR_NULL_POINTER, "vx_small_direction: NULL pointer");
+    vx::launch(small_direction_kernel, unsigned(step_ctas(n)), FT, 0, stream, n, partials, S, z, p);
+    VX_CHECK_LAUNCH("vx_small_direction");
     return VX_OK;
 }
 
@@ -530,10 +644,10 @@ extern "C" int vx_batch_dots_pr(int zprec, int64_t n, int slots, int64_t stride,
     const unsigned G = unsigned(fixed_ctas(n));
     if (zprec == VX_F64)
         vx::launch(dots_pr_kernel<double, double>, dim3(G, slots), FT, 0, stream, n, r, (const double*)zn,
-                   (const double*)zo, partials, stride);
+                   (const double*)zo, partials, stride, 0, (double*)nullptr, (unsigned*)nullptr);
     else if (zprec == VX_F32)
         vx::launch(dots_pr_kernel<double, float>, dim3(G, slots), FT, 0, stream, n, r, (const float*)zn,
-                   (const float*)zo, partials, stride);
+                   (const float*)zo, partials, stride, 0, (double*)nullptr, (unsigned*)nullptr);
     else { set_error("vx_batch_dots_pr: unsupported precision %d", zprec); return VX_ERR_INVALID_ARGUMENT; }
     VX_CHECK_LAUNCH("vx_batch_dots_pr");
     return VX_OK;

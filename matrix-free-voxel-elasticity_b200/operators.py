@@ -172,6 +172,20 @@ class VoxelOperator:
                   self._vec(x, "x"), self._vec(b, "b"), self._vec(res, "res"),
                   _ptr(partials, "partials", torch.float64), stream_ptr())
 
+    def apply_dot_fin(self, p, E, node_mask, q, partials, S, counter, fin):
+        """apply_dot followed by the finalisation `fin` of its sum into the solver scalars S; counter: one
+        zeroed int32, zero again afterwards."""
+        _lib.call("vx_apply_dot_fin", fin, self._sel, *self.shape, self._bp, self._E(E), self._mask(node_mask),
+                  self._vec(p, "p"), self._vec(q, "q"), _ptr(partials, "partials", torch.float64),
+                  _ptr(S, "S", torch.float64), _ptr(counter, "counter", torch.int32), stream_ptr())
+
+    def true_residual_fin(self, x, b, E, node_mask, res, partials, S, counter, fin):
+        """true_residual followed by the finalisation `fin` of its sum into S."""
+        _lib.call("vx_true_residual_fin", fin, self._sel, *self.shape, self._bp, self._E(E), self._mask(node_mask),
+                  self._vec(x, "x"), self._vec(b, "b"), self._vec(res, "res"),
+                  _ptr(partials, "partials", torch.float64), _ptr(S, "S", torch.float64),
+                  _ptr(counter, "counter", torch.int32), stream_ptr())
+
     def energy(self, u, rho=None, emin=1e-9, emax=1.0, penal=3.0, ce=None, dc=None):
         """ce_e = u_e^T ke u_e (FP64); with rho also dc_e = -p rho^(p-1) (emax-emin) ce_e."""
         ce = torch.empty(self.n_elem, dtype=torch.float64, device="cuda") if ce is None else ce

@@ -502,7 +502,9 @@ class FCGSolver:
         self.p = torch.zeros(n, **f64)
         self.q = torch.zeros(n, **f64)
         self.z_old = torch.zeros(n, dtype=precond.dtype, device="cuda")     # z's own storage: an exact copy
-        self.S = torch.zeros(16, **f64)
+        scalars = torch.zeros(17, **f64)
+        self.S = scalars[:16]
+        self.counter = scalars[16:].view(torch.int32)[:1]     # arrivals of the fused reductions, 0 between them
         self.S_host = torch.zeros(16, dtype=torch.float64, pin_memory=True)
         # f . x after a launched solve (launch(..., dot_with=f)): device value and its pinned copy
         self.dot_partials = torch.zeros(int(_lib.load().vx_partials_size(n)), **f64)
@@ -512,7 +514,11 @@ class FCGSolver:
         self.last_dot = None
         self.G_op = op64.partials_size
         self.G_vec = int(_lib.load().vx_solver_partials(n))
-        self.partials = torch.zeros(max(self.G_op, 2 * self.G_vec), **f64)
+        steps = int(_lib.load().vx_jacobi_step_partials(n))
+        self.partials = torch.empty(max(self.G_op, 2 * self.G_vec, steps), **f64)
+        self._jacobi = type(precond) is JacobiPreconditioner
+        self._small = self._jacobi and n <= int(_lib.load().vx_small_cg_limit())
+        self.step_partials = torch.empty(steps, **f64) if self._small else None
         self.zprec = PREC[precond.dtype]
         self.stream = torch.cuda.Stream()
         self.use_graph = bool(graph)
@@ -525,27 +531,51 @@ class FCGSolver:
         return 6 * self.n * 8 + self.M.footprint_bytes() + self.E.numel() * 8
 
     # ------------------------------------------------------------------ kernel emission
-    def _fin(self, op, G):
-        _lib.call("vx_solver_finalize", op, G, self.partials.data_ptr(), self.S.data_ptr(), _s())
+    def _true_residual(self, out):
+        """out = b - A x and the true relative residual in S."""
+        self.op.true_residual_fin(self.x, self.b, self.E, self.mask, out, self.partials, self.S, self.counter, FIN_TRUE)
+
+    def _dots(self, fin, prec, a, b, c=None):
+        """a . b (and a . (b - c)), finalised into S."""
+        _lib.call("vx_dots_pr_fin", fin, _lib.VX_F64, prec, self.n, a.data_ptr(), b.data_ptr(),
+                  None if c is None else c.data_ptr(), self.partials.data_ptr(), self.S.data_ptr(),
+                  self.counter.data_ptr(), _s())
+
+    def _small_iteration(self, check: bool):
+        """One Jacobi-preconditioned iteration on a small system: three launches, five at a check."""
+        S, M, pq, sp = self.S.data_ptr(), self.M, self.partials.data_ptr(), self.step_partials.data_ptr()
+        x, r, p, q, d, z = (t.data_ptr() for t in (self.x, self.r, self.p, self.q, M.invd, M.z))
+        self.op.apply_dot(self.p, self.E, self.mask, self.q, self.partials)      # q = A p, p.q
+        if check:
+            _lib.call("vx_small_step", self.n, self.G_op, pq, S, x, p, None, None, None, None, 1, 0, None, _s())
+            self._true_residual(self.r)
+        _lib.call("vx_small_step", self.n, self.G_op, pq, S, x, p, r, q, d, z, 0 if check else 1, 1, sp, _s())
+        _lib.call("vx_small_direction", self.n, sp, S, z, p, _s())
 
     def _iteration(self, check: bool):
+        if self._small:
+            return self._small_iteration(check)
         op, S, pp = self.op, self.S.data_ptr(), self.partials.data_ptr()
         # Off the check iterations the updates ride on kernels that stream the same vectors anyway:
-        # r -= alpha q in the preconditioner's first kernel, x += alpha p in the direction update.
+        # r -= alpha q in the preconditioner's first kernel, x += alpha p in the direction update (both in
+        # the one step kernel of a Jacobi preconditioner).
         # At a check iteration x is updated here and r is replaced by b - A x.
         fuse = not check and getattr(self.M, "fuses_residual_update", False)
-        op.apply_dot(self.p, self.E, self.mask, self.q, self.partials)          # q = A p, p.q
-        self._fin(FIN_PQ, self.G_op)
-        if not fuse:
+        op.apply_dot_fin(self.p, self.E, self.mask, self.q, self.partials, self.S, self.counter, FIN_PQ)   # q = A p, p.q
+        if not fuse and (check or not self._jacobi):
             _lib.call("vx_cg_update", _lib.VX_F64, self.n, S, self.x.data_ptr(), self.p.data_ptr(),
                       self.r.data_ptr(), self.q.data_ptr(), 0 if check else 1, _s())
         if check:                                                                # r = b - A x (replacement)
-            op.true_residual(self.x, self.b, self.E, self.mask, self.r, self.partials)
-            self._fin(FIN_TRUE, self.G_op)
+            self._true_residual(self.r)
+        if self._jacobi:                                                         # z = M r over the previous z
+            z = self.M.z
+            _lib.call("vx_jacobi_step", self.n, S, self.x.data_ptr(), self.p.data_ptr(), self.r.data_ptr(),
+                      self.q.data_ptr(), self.M.invd.data_ptr(), z.data_ptr(), 0 if check else 1, pp,
+                      self.counter.data_ptr(), _s())
+            _lib.call("vx_cg_direction", _lib.VX_F64, self.zprec, self.n, S, z.data_ptr(), self.p.data_ptr(), None, _s())
+            return
         z = self.M.emit(self.r, update=(self.q, self.S)) if fuse else self.M.emit(self.r)
-        _lib.call("vx_dots_pr", _lib.VX_F64, self.zprec, self.n, self.r.data_ptr(), z.data_ptr(),
-                  self.z_old.data_ptr(), pp, _s())
-        self._fin(FIN_BETA_PR, self.G_vec)
+        self._dots(FIN_BETA_PR, self.zprec, self.r, z, self.z_old)
         if fuse:
             _lib.call("vx_cg_direction_update", self.zprec, self.n, S, z.data_ptr(), self.p.data_ptr(),
                       self.z_old.data_ptr(), self.x.data_ptr(), _s())
@@ -563,20 +593,15 @@ class FCGSolver:
         self.p.zero_()
         _lib.call("vx_set_scalars", S, 0, 16, 0.0, _s())
         _lib.call("vx_set_scalars", S, S_TOL, 1, self.tol if self.fixed is None else -1.0, _s())
-        _lib.call("vx_dots_pr", _lib.VX_F64, _lib.VX_F64, self.n, self.b.data_ptr(), self.b.data_ptr(), None,
-                  self.partials.data_ptr(), _s())
-        self._fin(FIN_NB, self.G_vec)
+        self._dots(FIN_NB, _lib.VX_F64, self.b, self.b)
         if x0 is None:
             self.x.zero_()
             self.r.copy_(self.b)
         else:                                                   # warm start: r = b - A x0
             self.x.copy_(x0)
-            self.op.true_residual(self.x, self.b, self.E, self.mask, self.r, self.partials)
-            self._fin(FIN_TRUE, self.G_op)
+            self._true_residual(self.r)
         z = self.M.emit(self.r)
-        _lib.call("vx_dots_pr", _lib.VX_F64, self.zprec, self.n, self.r.data_ptr(), z.data_ptr(), None,
-                  self.partials.data_ptr(), _s())
-        self._fin(FIN_RZ, self.G_vec)
+        self._dots(FIN_RZ, self.zprec, self.r, z)
         _lib.call("vx_cg_direction", _lib.VX_F64, self.zprec, self.n, S, z.data_ptr(), self.p.data_ptr(),
                   self.z_old.data_ptr(), _s())                                  # p = z (beta = 0), z_old = z
 
@@ -658,8 +683,7 @@ class FCGSolver:
                 s = self._read()
                 done, it = bool(s[S_DONE]), int(s[S_IT])
             if not done:                                                       # final true residual (voxel_mg.py:213-216)
-                self.op.true_residual(self.x, self.b, self.E, self.mask, self.q, self.partials)
-                self._fin(FIN_TRUE, self.G_op)
+                self._true_residual(self.q)
                 s = self._read()
             if self._dot_with is not None:
                 if int(s[S_IT]) != int(s_launch[S_IT]):                      # x moved after the dot: redo it
