@@ -85,29 +85,31 @@ __global__ void band_load_kernel(int n, int bw, const __grid_constant__ FactorBa
 // inverse goes to dinv (CB x CB, row-major, lower triangle), and the block column's rows below it
 // (the A values band_update turns into the panel) to apanel ((bw + 1) x CB), so that band_update
 // can store finished panel rows in place while other tiles still read the originals.
-// The block's CB pivots are a chain of dependent steps, so it is factored by four warps with the
-// rows in registers (right-looking; threads i and CB + i hold the even and the odd columns of row i;
-// per pivot: the pivot thread's reciprocal square root (the pivot is d rsqrt(d)), a named barrier of
-// the four warps, the column through shared memory, a rank-1 update of the row in registers, split
-// between the two threads of the row).  Three variants measured no faster: one barrier per pivot
-// with every row forming the reciprocal square root from a double-buffered column (+8%), a
-// look-ahead in which row j + 1 forms the next pivot before finishing its update (+2%), and (with
-// two factoring warps) the update of a whole row by one thread.  Meanwhile warps 4-7 copy the
-// panel rows; a block smaller than CB (the last) is padded with the identity.
-// The inverse X = L^-1 goes by 32 x 32 blocks: warps 0 and 1 run the forward substitutions of
-// X11 and X22 (lane = column, in registers, four partial sums per row), then all eight warps form
-// X21 = -X22 (L21 X11).  Every loop is unrolled, so the row and column registers are addressed at
-// compile time (a variant with the pivot loop rolled and the row shifted through the registers ran
-// slower).
-constexpr int HB = CB / 2, HBP = HB + 1;   // half blocks of the block inverse
-constexpr int FT = 2 * CB;     // factoring threads: a row's even and odd columns
-__device__ __forceinline__ void potrf_bar() { asm volatile("bar.sync 1, %0;" ::"n"(FT) : "memory"); }
+// The block's CB pivots are a chain of dependent steps.  Warp 0 walks it through the two HB x HB diagonal
+// blocks with a row per lane in registers (right-looking; per pivot: the pivot to every lane by a shuffle, its
+// reciprocal square root formed by every lane -- the pivot is d rsqrt(d) --, the column and its rank-1 update,
+// the column's entries again by shuffles: no barrier and no shared memory on the chain).  It hands its
+// columns over PC at a time through named barriers to warp 1 (the rows L21 below, right-looking too) and
+// warp 2 (the forward substitution of the block's inverse), which trail it by one group; the four warps then
+// apply the 32 updates of L22 and warp 0 goes on, while warps 1 and 3 form L21 X11.  Each entry meets the
+// same operations in the same order as in a plain right-looking factorisation by rows.  Warps 4-7 copy the
+// panel rows meanwhile; a block smaller than CB (the last) is padded with the identity.
+// The inverse X = L^-1 goes by 32 x 32 blocks: X11 and X22 by forward substitution (lane = column, in
+// registers, four partial sums per row), then X21 = -X22 (L21 X11) by all eight warps.
+// The form it replaces, four factoring warps with three barriers a pivot, took 38k cycles for the 64 pivots.
+// Measured (whole factorisation, inverse included): n = 4131, bw = 275 3.11 -> 2.61 ms; n = 5700, bw = 335 4.81 -> 4.12 ms,
+// bit for bit the same factor.
+constexpr int HB = CB / 2, HBP = HB + 1;   // half blocks
+constexpr int PC = 8;                      // pivots handed over at a time
+constexpr int FT = 2 * CB;                 // threads of warps 0-3
+template <int COUNT> __device__ __forceinline__ void potrf_sync(int id) { asm volatile("bar.sync %0, %1;" ::"r"(id), "n"(COUNT) : "memory"); }
+template <int COUNT> __device__ __forceinline__ void potrf_arrive(int id) { asm volatile("bar.arrive %0, %1;" ::"r"(id), "n"(COUNT) : "memory"); }
 
 // FACTOR = false: the band already holds a Cholesky factor; only the diagonal block's inverse is
 // formed (block k0 = blockIdx.x CB, every block in one launch; no panel copy, nothing written back).
 template <bool FACTOR>
 __global__ void __launch_bounds__(POTRF_T) band_potrf_kernel(int n, int bw, int k0, const __grid_constant__ FactorBatch fb) {
-    static_assert(CB == 64 && POTRF_T > FT, "four factoring warps, the others copy");
+    static_assert(CB == 64 && POTRF_T > FT, "warps 0-3 factor, the others copy");
     vx::pdl_begin();
     if constexpr (!FACTOR) k0 = blockIdx.x * CB;
     const FactorPtrs P = fptrs(fb, n, bw);
@@ -116,7 +118,7 @@ __global__ void __launch_bounds__(POTRF_T) band_potrf_kernel(int n, int bw, int 
     double* __restrict__ apanel = P.apanel;
     int* __restrict__ info = P.info;
     extern __shared__ __align__(16) double psm[];
-    __shared__ double colj[CB], rinv[CB];
+    __shared__ double rinv[CB];
     double (*D)[CBP] = reinterpret_cast<double (*)[CBP]>(psm);
     double (*X)[CBP] = reinterpret_cast<double (*)[CBP]>(psm + CB * CBP);
     double (*Tm)[HBP] = reinterpret_cast<double (*)[HBP]>(psm + 2 * CB * CBP);   // L21 X11
@@ -138,47 +140,118 @@ __global__ void __launch_bounds__(POTRF_T) band_potrf_kernel(int n, int bw, int 
         }
     }
     __syncthreads();
-    if (!FACTOR && t < CB) rinv[t] = 1.0 / D[t][t];
-    if (FACTOR && t < FT) {
-        // row t % CB; warps 0-1 hold its even columns, warps 2-3 its odd ones (H = t / CB)
-        const int row = t % CB;
-        auto factor_rows = [&](auto hc) {
-            constexpr int H = decltype(hc)::value;
-            double a[CB / 2];                          // a[i] = row, column 2 i + H
+    const int lane = t & 31, wid = t >> 5;
+    // rows [r0, r1) of the block inverse at offset o (lane = column); x: the rows above
+    auto substitute = [&](int o, auto r0c, double (&x)[HB]) {
+        constexpr int R0 = decltype(r0c)::value;
+        #pragma unroll
+        for (int r = R0; r < R0 + PC; ++r) {
+            double s[4] = {0.0, 0.0, 0.0, 0.0};
             #pragma unroll
-            for (int i = 0; i < CB / 2; ++i) a[i] = D[row][2 * i + H];
-            #pragma unroll
-            for (int j = 0; j < CB; ++j) {
-                if ((j & 1) == H && row == j) {
-                    double d = a[j / 2];
+            for (int p = 0; p < r; ++p) s[p & 3] += D[o + r][o + p] * x[p];
+            x[r] = ((r == lane ? 1.0 : 0.0) - ((s[0] + s[1]) + (s[2] + s[3]))) * rinv[o + r];
+            X[o + r][o + lane] = x[r];
+        }
+    };
+    using Q0 = std::integral_constant<int, 0>;
+    using Q1 = std::integral_constant<int, PC>;
+    using Q2 = std::integral_constant<int, 2 * PC>;
+    using Q3 = std::integral_constant<int, 3 * PC>;
+    if (!FACTOR) {
+        if (t < CB) rinv[t] = 1.0 / D[t][t];
+        __syncthreads();
+        if (wid < 2) {
+            double x[HB];
+            const int o = wid * HB;
+            substitute(o, Q0{}, x);
+            substitute(o, Q1{}, x);
+            substitute(o, Q2{}, x);
+            substitute(o, Q3{}, x);
+        } else {
+            for (int i = t - 2 * 32; i < HB * HB; i += POTRF_T - 2 * 32) X[i / HB][HB + i % HB] = 0.0;
+        }
+    } else if (wid < 4) {
+        #pragma unroll 1
+        for (int h = 0; h < 2; ++h) {                  // the diagonal block at offset o = 0, then HB
+            const int o = h * HB, id = 1 + 4 * h;      // barriers 1-4 (three warps), 5-8 (two), 9 (four)
+            if (wid == 0) {
+                double a[HB];
+                #pragma unroll
+                for (int c = 0; c < HB; ++c) a[c] = D[o + lane][o + c];
+                #pragma unroll
+                for (int j = 0; j < HB; ++j) {
+                    double d = __shfl_sync(0xffffffffu, a[j], j);
                     if (!(d > 0.0)) {                  // not positive definite: flag, keep finite
-                        if (j < w) atomicCAS(info, 0, k0 + j + 1);
+                        if (lane == 0 && o + j < w) atomicCAS(info, 0, k0 + o + j + 1);
                         d = 1.0;
                     }
                     const double ri = rsqrt(d);
-                    a[j / 2] = d * ri;
-                    rinv[j] = ri;
-                }
-                potrf_bar();
-                if ((j & 1) == H && row > j) {
-                    a[j / 2] *= rinv[j];               // L[row][j]
-                    colj[row] = a[j / 2];
-                }
-                potrf_bar();
-                if (row > j) {
-                    const double l = colj[row];
+                    a[j] = lane == j ? d * ri : a[j] * ri;
+                    if (lane == 0) rinv[o + j] = ri;
+                    D[o + lane][o + j] = a[j];         // rows above j: never read
                     #pragma unroll
-                    for (int c = j + 1; c < CB; ++c)   // c > row: never read (upper part)
-                        if ((c & 1) == H) a[c / 2] -= l * colj[c];
+                    for (int c = j + 1; c < HB; ++c) a[c] = fma(-a[j], __shfl_sync(0xffffffffu, a[j], c), a[c]);
+                    if (j % PC == PC - 1) {
+                        if (h == 0) potrf_arrive<96>(id + j / PC);
+                        else potrf_arrive<64>(id + j / PC);
+                    }
                 }
-                potrf_bar();                           // colj is rewritten by the next pivot
+            } else if (wid == 1 && h == 0) {           // L21: row HB + lane
+                double a[HB];
+                #pragma unroll
+                for (int c = 0; c < HB; ++c) a[c] = D[HB + lane][c];
+                #pragma unroll
+                for (int j = 0; j < HB; ++j) {
+                    if (j % PC == 0) potrf_sync<96>(id + j / PC);
+                    a[j] *= rinv[j];
+                    D[HB + lane][j] = a[j];
+                    #pragma unroll
+                    for (int c = j + 1; c < HB; ++c) a[c] = fma(-a[j], D[c][j], a[c]);
+                }
+            } else if (wid == 2) {
+                double x[HB];
+                auto group = [&](auto r0c) {
+                    if (h == 0) potrf_sync<96>(id + decltype(r0c)::value / PC);
+                    else potrf_sync<64>(id + decltype(r0c)::value / PC);
+                    substitute(o, r0c, x);
+                };
+                group(Q0{});
+                group(Q1{});
+                group(Q2{});
+                group(Q3{});
+            } else if (h == 0) {                       // warp 3: X is lower triangular
+                for (int i = lane; i < HB * HB; i += 32) X[i / HB][HB + i % HB] = 0.0;
+            } else {                                   // warps 1 and 3: Tm = L21 X11, 16 rows each
+                const int r0 = wid == 1 ? 0 : HB / 2;
+                double s[HB / 2];
+                #pragma unroll
+                for (int m = 0; m < HB / 2; ++m) s[m] = 0.0;
+                #pragma unroll 4
+                for (int p = 0; p < HB; ++p) {
+                    const double xv = X[p][lane];
+                    #pragma unroll
+                    for (int m = 0; m < HB / 2; ++m) s[m] = fma(D[HB + r0 + m][p], xv, s[m]);
+                }
+                #pragma unroll
+                for (int m = 0; m < HB / 2; ++m) Tm[r0 + m][lane] = s[m];
             }
-            #pragma unroll
-            for (int i = 0; i < CB / 2; ++i) D[row][2 * i + H] = 2 * i + H <= row ? a[i] : 0.0;
-        };
-        if (t < CB) factor_rows(std::integral_constant<int, 0>{});
-        else factor_rows(std::integral_constant<int, 1>{});
-    } else if (FACTOR) {                               // meanwhile warps 4-7 copy the panel rows
+            potrf_sync<FT>(9);
+            if (h == 0) {                              // the HB updates of L22: lane = row, columns wid + 4 m
+                double s[HB / 4];
+                #pragma unroll
+                for (int m = 0; m < HB / 4; ++m) s[m] = D[HB + lane][HB + wid + 4 * m];
+                #pragma unroll 4
+                for (int j = 0; j < HB; ++j) {
+                    const double l = D[HB + lane][j];
+                    #pragma unroll
+                    for (int m = 0; m < HB / 4; ++m) s[m] = fma(-l, D[HB + wid + 4 * m][j], s[m]);
+                }
+                #pragma unroll
+                for (int m = 0; m < HB / 4; ++m) D[HB + lane][HB + wid + 4 * m] = s[m];
+                potrf_sync<FT>(9);
+            }
+        }
+    } else {                                           // meanwhile warps 4-7 copy the panel rows
         // in batches whose loads are all issued before their stores: the band and the panel share
         // one workspace, so the compiler may not move a load above an earlier store by itself
         constexpr int CPB = 16, CPT = POTRF_T - FT;
@@ -196,28 +269,10 @@ __global__ void __launch_bounds__(POTRF_T) band_potrf_kernel(int n, int bw, int 
         }
     }
     __syncthreads();
-    // X = L^-1 by 32 x 32 blocks: X11 (warp 0) and X22 (warp 1) by forward substitution, lane = column,
-    // in registers; then X21 = -X22 (L21 X11) by all threads
-    if (t < 2 * HB) {
-        const int o = (t / HB) * HB, c = t % HB;
-        double x[HB];
-        #pragma unroll
-        for (int r = 0; r < HB; ++r) {
-            double s[4] = {0.0, 0.0, 0.0, 0.0};
-            #pragma unroll
-            for (int p = 0; p < r; ++p) s[p & 3] += D[o + r][o + p] * x[p];
-            x[r] = ((r == c ? 1.0 : 0.0) - ((s[0] + s[1]) + (s[2] + s[3]))) * rinv[o + r];
-        }
-        #pragma unroll
-        for (int r = 0; r < HB; ++r) X[o + r][o + c] = x[r];
-    } else {
-        for (int i = t - 2 * HB; i < HB * HB; i += POTRF_T - 2 * HB) X[i / HB][HB + i % HB] = 0.0;
-    }
-    __syncthreads();
     const int tc = t % HB, tr = t / HB;                // column and first row of this thread's outputs
     constexpr int NR = HB * HB / POTRF_T;              // outputs per thread, rows tr + RS m
     constexpr int RS = POTRF_T / HB;
-    {
+    if (!FACTOR) {
         double s[NR];
         #pragma unroll
         for (int m = 0; m < NR; ++m) s[m] = 0.0;
