@@ -165,19 +165,28 @@ HOST_ONLY = {"vx_last_error", "vx_version", "vx_element_matrix", "vx_element", "
 launches = 0          # kernels launched directly (graph launches are counted by the solvers)
 
 
-_FNS = {}             # name -> bound entry point (getattr on a CDLL is not free)
+_FNS = {}             # name -> (bound entry point, its kernels per call; None: counted from its arguments)
+
+
+def _bind(name: str):
+    count = KERNELS_PER_CALL.get(name, 0 if name in HOST_ONLY else 1)
+    if name in ("vx_coarse_factor", "vx_batch_coarse_factor"):
+        count = None
+    entry = _FNS[name] = (getattr(load(), name), count)
+    return entry
 
 
 def call(name: str, *args) -> None:
+    """One library call.  A small operator launch costs the host more than the device, so the way through
+    here is short: one look-up, the call, the launch count."""
     global launches
-    fn = _FNS.get(name)
-    if fn is None:
-        fn = _FNS[name] = getattr(load(), name)
-    check(fn(*args), name)
-    if name in ("vx_coarse_factor", "vx_batch_coarse_factor"):   # load, a factor and an update per block, inverse
-        launches += 2 * ((int(args[0]) + 63) // 64) + 1
-    elif name not in HOST_ONLY:
-        launches += KERNELS_PER_CALL.get(name, 1)
+    fn, count = _FNS.get(name) or _bind(name)
+    status = fn(*args)
+    if status:
+        check(status, name)
+    if count is None:                     # load, a factor and an update per block, inverse
+        count = 2 * ((int(args[0]) + 63) // 64) + 1
+    launches += count
     if CAPTURE_STREAM is not None and _lib.vx_capture_status(CAPTURE_STREAM) == 2:
         raise RuntimeError(f"{name} invalidated the stream capture")
 

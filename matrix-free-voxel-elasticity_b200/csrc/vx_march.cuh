@@ -423,6 +423,7 @@ inline int march_cx(const Grid& g, int tiles, int slots) {
         const int64_t ctas = int64_t(tiles) * ((planes + cx - 1) / cx);
         const int64_t c = (ctas + slots - 1) / slots * (cx + 2);
         if (c < cost) { cost = c; best = cx; }
+        if (cx == 1) break;                                  // more waves split no further
     }
     return best;
 }

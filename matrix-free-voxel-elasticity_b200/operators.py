@@ -27,18 +27,26 @@ STORAGE = {(torch.float64, torch.float64): _lib.VX_F64, (torch.float32, torch.fl
 
 _RAW_STREAM = getattr(torch._C, "_cuda_getCurrentRawStream", None)
 _CUR_DEVICE = getattr(torch._C, "_cuda_getDevice", None)
+_initialized = False          # CUDA's initialisation is for the life of the process
 
 
 def stream_ptr(device=None) -> int:
     """cudaStream_t of the current stream (of the current device when `device` is None).  The
     host-driven loops ask for it once per launch, so on the current device it is read with torch's
     raw-stream accessor, without building a Stream object and resolving the device index."""
-    if device is None and _RAW_STREAM is not None and _CUR_DEVICE is not None and torch.cuda.is_initialized():
-        return _RAW_STREAM(_CUR_DEVICE())
+    global _initialized
+    if device is None and _RAW_STREAM is not None and _CUR_DEVICE is not None:
+        if _initialized or torch.cuda.is_initialized():
+            _initialized = True
+            return _RAW_STREAM(_CUR_DEVICE())
     return torch.cuda.current_stream(device).cuda_stream
 
 
 def _ptr(t, what, dtype=None, numel=None, allow_none=False):
+    """Device address of a contiguous CUDA tensor (of `dtype` and `numel` entries), else ValueError."""
+    if (t.__class__ is torch.Tensor and t.is_cuda and t.is_contiguous() and (dtype is None or t.dtype is dtype)
+            and (numel is None or t.numel() == numel)):
+        return t.data_ptr()
     if t is None:
         if allow_none:
             return None
@@ -94,6 +102,7 @@ class VoxelOperator:
         self.nodes = n_nodes(self.shape)
         self.ndof = 3 * self.nodes
         self.n_elem = n_elems(self.shape)
+        self._ydtype = torch.float32 if dtype == torch.bfloat16 else dtype     # of vx_matvec's result
         self._bp = _lib.dptr(self.blocks)
         self._kp = _lib.dptr(self.ke)
 
@@ -121,10 +130,11 @@ class VoxelOperator:
     # --------------------------------------------------------------- products
     def matvec(self, u, E, node_mask=None, out=None):
         """y = K u (node_mask None) or y = M K (M u) + (I - M) u."""
-        y = self._out(out)
-        _lib.call("vx_matvec", self._sel, *self.shape, self._bp, self._E(E), self._vec(u, "u"),
-                  _ptr(y, "y", torch.float32 if self.dtype == torch.bfloat16 else self.dtype, self.ndof),
-                  self._mask(node_mask), stream_ptr())
+        y = self._out(None) if out is None else out
+        nx, ny, nz = self.shape
+        _lib.call("vx_matvec", self._sel, nx, ny, nz, self._bp, _ptr(E, "E", self.aux_dtype, self.n_elem),
+                  _ptr(u, "u", self.dtype, self.ndof), _ptr(y, "y", self._ydtype, self.ndof),
+                  None if node_mask is None else _ptr(node_mask, "node_mask", torch.uint8, self.nodes), stream_ptr())
         return y
 
     def matvec_dense(self, u, E, out=None):
