@@ -9,6 +9,7 @@
 // convergence, on breakdown or at maxiter.
 #include "vx_finalize.cuh"
 #include <algorithm>
+#include <type_traits>
 
 namespace vx {
 
@@ -20,15 +21,60 @@ __global__ void __launch_bounds__(FT) finalize_kernel(int op, int64_t G, const d
     fin_reduce(op, G, partials + pstride * int64_t(blockIdx.y), S + S_COUNT * int64_t(blockIdx.y));
 }
 
+// The vector kernels move W consecutive entries per thread: 4 (16-byte accesses, two for doubles) on long
+// aligned vectors, where one entry per thread left HBM at 84 to 88% for want of bytes in flight, else 1.
+// The same operations either way.  576x288x288 (us, W = 1 -> 4, FP32 z): direction with
+// the x update 1006 -> 850 (6.8 TB/s), V-cycle entry with the r update 920 -> 762, direction 600 -> 506, entry
+// 590 -> 424, x and r update 1077 -> 988.
+constexpr int64_t WIDE_MIN = 1 << 20;      // below this, 4 entries a thread leave SMs without CTAs
+template <int W, typename T>
+__device__ __forceinline__ void ldv(const T* p, T (&v)[W]) {
+    if constexpr (W == 1) v[0] = p[0];
+    else if constexpr (sizeof(T) == 8) {
+        const double2 a = reinterpret_cast<const double2*>(p)[0], b = reinterpret_cast<const double2*>(p)[1];
+        v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
+    } else if constexpr (sizeof(T) == 4) {
+        const float4 a = *reinterpret_cast<const float4*>(p);
+        v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+    } else {
+        union { uint2 u; T t[4]; } a;
+        a.u = *reinterpret_cast<const uint2*>(p);
+        for (int k = 0; k < 4; ++k) v[k] = a.t[k];
+    }
+}
+template <int W, typename T>
+__device__ __forceinline__ void stv(T* p, const T (&v)[W]) {
+    if constexpr (W == 1) p[0] = v[0];
+    else if constexpr (sizeof(T) == 8) {
+        reinterpret_cast<double2*>(p)[0] = make_double2(v[0], v[1]);
+        reinterpret_cast<double2*>(p)[1] = make_double2(v[2], v[3]);
+    } else if constexpr (sizeof(T) == 4) {
+        *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]);
+    } else {
+        union { uint2 u; T t[4]; } a;
+        for (int k = 0; k < 4; ++k) a.t[k] = v[k];
+        *reinterpret_cast<uint2*>(p) = a.u;
+    }
+}
+// Runs f(i, integral_constant<W>) for this thread's entries: the W at i, or the last few one by one.
+template <int W, typename F>
+__device__ __forceinline__ void for_entries(int64_t n, F&& f) {
+    const int64_t i = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) * W;
+    if (i + W <= n) f(i, std::integral_constant<int, W>{});
+    else if constexpr (W > 1)
+        for (int64_t k = i; k < n; ++k) f(k, std::integral_constant<int, 1>{});
+}
+template <typename... T> bool wide(int64_t n, const T*... p) {
+    return n >= WIDE_MIN && ((p == nullptr || aligned(p, 4 * sizeof(T) > 16 ? 16 : 4 * sizeof(T))) && ...);
+}
+
 // x += alpha p; r -= alpha q (r update skipped when it is about to be replaced by b - A x).
 // Nothing moves once the loop has converged or broken down.
 // Vector kernels of a batch: slot blockIdx.y works on its n entries at slot * vs and on S + 16 slot.
-template <typename T>
+template <int W, typename T>
 __global__ void cg_update_kernel(int64_t n, const double* __restrict__ S, T* __restrict__ x, const T* __restrict__ p,
                                  T* __restrict__ r, const T* __restrict__ q, int update_r, int64_t vs) {
     vx::pdl_begin();
-    const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i >= n) return;
     const int64_t o = vs * int64_t(blockIdx.y);
     S += S_COUNT * int64_t(blockIdx.y);
     x += o;
@@ -36,41 +82,71 @@ __global__ void cg_update_kernel(int64_t n, const double* __restrict__ S, T* __r
     if (update_r) { r += o; q += o; }
     if (S[S_DONE] != 0.0 || S[S_BREAK] != 0.0) return;
     const T a = T(S[S_ALPHA]);
-    x[i] = x[i] + a * p[i];
-    if (update_r) r[i] = r[i] - a * q[i];
+    for_entries<W>(n, [&](int64_t i, auto wc) {
+        constexpr int V = decltype(wc)::value;
+        T xv[V], pv[V], rv[V], qv[V];
+        ldv<V>(x + i, xv);
+        ldv<V>(p + i, pv);
+        if (update_r) { ldv<V>(r + i, rv); ldv<V>(q + i, qv); }
+        #pragma unroll
+        for (int k = 0; k < V; ++k) {
+            xv[k] = xv[k] + a * pv[k];
+            if (update_r) rv[k] = rv[k] - a * qv[k];
+        }
+        stv<V>(x + i, xv);
+        if (update_r) stv<V>(r + i, rv);
+    });
 }
 
 // p = z + beta p and, when z_old is given, z_old = z; z and z_old in the preconditioner's storage TZ
 // (a copy in z's own type is exact and moves half the bytes of an FP64 copy of an FP32 z)
-template <typename T, typename TZ>
+template <int W, typename T, typename TZ>
 __global__ void cg_direction_kernel(int64_t n, const double* __restrict__ S, const TZ* __restrict__ z, T* __restrict__ p,
                                     TZ* __restrict__ z_old, int64_t vs) {
     vx::pdl_begin();
-    const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i >= n) return;
     const int64_t o = vs * int64_t(blockIdx.y);
     S += S_COUNT * int64_t(blockIdx.y);
     z += o;
     p += o;
     if (z_old) z_old += o;
-    const TZ zr = z[i];
-    p[i] = T(Storage<TZ>::cvt(zr)) + T(S[S_BETA]) * p[i];
-    if (z_old) z_old[i] = zr;
+    const T beta = T(S[S_BETA]);
+    for_entries<W>(n, [&](int64_t i, auto wc) {
+        constexpr int V = decltype(wc)::value;
+        TZ zr[V];
+        T pv[V];
+        ldv<V>(z + i, zr);
+        ldv<V>(p + i, pv);
+        #pragma unroll
+        for (int k = 0; k < V; ++k) pv[k] = T(Storage<TZ>::cvt(zr[k])) + beta * pv[k];
+        stv<V>(p + i, pv);
+        if (z_old) stv<V>(z_old + i, zr);
+    });
 }
 
 // The same direction update preceded by the deferred x += alpha p of this iteration (p still the old
 // direction), skipped once the loop has converged or broken down: one read of p serves both.
-template <typename T, typename TZ>
+template <int W, typename T, typename TZ>
 __global__ void cg_direction_update_kernel(int64_t n, const double* __restrict__ S, const TZ* __restrict__ z,
                                            T* __restrict__ p, TZ* __restrict__ z_old, T* __restrict__ x) {
     vx::pdl_begin();
-    const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const T pi = p[i];
-    if (S[S_DONE] == 0.0 && S[S_BREAK] == 0.0) x[i] = x[i] + T(S[S_ALPHA]) * pi;
-    const TZ zr = z[i];
-    p[i] = T(Storage<TZ>::cvt(zr)) + T(S[S_BETA]) * pi;
-    if (z_old) z_old[i] = zr;
+    const bool move = S[S_DONE] == 0.0 && S[S_BREAK] == 0.0;
+    const T alpha = T(S[S_ALPHA]), beta = T(S[S_BETA]);
+    for_entries<W>(n, [&](int64_t i, auto wc) {
+        constexpr int V = decltype(wc)::value;
+        T pv[V], xv[V];
+        TZ zr[V];
+        ldv<V>(p + i, pv);
+        if (move) ldv<V>(x + i, xv);
+        ldv<V>(z + i, zr);
+        #pragma unroll
+        for (int k = 0; k < V; ++k) {
+            xv[k] = xv[k] + alpha * pv[k];
+            pv[k] = T(Storage<TZ>::cvt(zr[k])) + beta * pv[k];
+        }
+        if (move) stv<V>(x + i, xv);
+        stv<V>(p + i, pv);
+        if (z_old) stv<V>(z_old + i, zr);
+    });
 }
 
 // partials for r . zn and r . (zn - zo), fixed grid G (a function of n), fixed order
@@ -251,38 +327,37 @@ __global__ void __launch_bounds__(FT) jacobi_precond_dot_kernel(int64_t n, const
     if (threadIdx.x == 0) partials[blockIdx.x] = a;
 }
 
-// V-cycle entry: r_mg = (TM) r64 (skipped when r_mg is NULL), x = omega * invd * r_mg
-// V-cycle entry: r_mg = r64 in auxiliary storage, x = omega * invd * r_mg (the first pre-sweep from x = 0)
-template <typename TX, typename TR>
-__global__ void vcycle_entry_kernel(int64_t n, const double* __restrict__ r64, TR* __restrict__ rmg,
+// V-cycle entry: r_mg = r64 in auxiliary storage (skipped when r_mg is NULL), x = omega * invd * r_mg (the first
+// pre-sweep from x = 0).  With UPDATE it is preceded by the CG residual update r64 -= alpha q (alpha =
+// S[S_ALPHA]), which is skipped, like vx_cg_update's, once the loop has converged or broken down.
+template <int W, bool UPDATE, typename TX, typename TR>
+__global__ void vcycle_entry_kernel(int64_t n, const double* __restrict__ S, const double* __restrict__ r_in,
+                                    double* __restrict__ r_out, const double* __restrict__ q, TR* __restrict__ rmg,
                                     const TR* __restrict__ invd, double omega, TX* __restrict__ x) {
     vx::pdl_begin();
     using A = arith_t<TX>;
-    const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const A r = A(Storage<TR>::round(arith_t<TR>(r64[i])));   // the level residual as stored
-    if (rmg) Storage<TR>::store(rmg + i, r);
-    Storage<TX>::store(x + i, A(omega) * A(Storage<TR>::load(invd + i)) * r);
-}
-
-// The same entry preceded by the CG residual update r64 -= alpha q (alpha = S[S_ALPHA]), which is
-// skipped, like vx_cg_update's, once the loop has converged or broken down.
-template <typename TX, typename TR>
-__global__ void vcycle_entry_update_kernel(int64_t n, const double* __restrict__ S, double* __restrict__ r64,
-                                           const double* __restrict__ q, TR* __restrict__ rmg,
-                                           const TR* __restrict__ invd, double omega, TX* __restrict__ x) {
-    vx::pdl_begin();
-    using A = arith_t<TX>;
-    const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    double rv = r64[i];
-    if (S[S_DONE] == 0.0 && S[S_BREAK] == 0.0) {
-        rv = rv - S[S_ALPHA] * q[i];
-        r64[i] = rv;
-    }
-    const A r = A(Storage<TR>::round(arith_t<TR>(rv)));
-    if (rmg) Storage<TR>::store(rmg + i, r);
-    Storage<TX>::store(x + i, A(omega) * A(Storage<TR>::load(invd + i)) * r);
+    const bool move = UPDATE && S[S_DONE] == 0.0 && S[S_BREAK] == 0.0;
+    const double alpha = UPDATE ? S[S_ALPHA] : 0.0;
+    const double* const rp = UPDATE ? r_out : r_in;
+    for_entries<W>(n, [&](int64_t i, auto wc) {
+        constexpr int V = decltype(wc)::value;
+        double rv[V], qv[V];
+        TR dv[V], mv[V];
+        TX xv[V];
+        ldv<V>(rp + i, rv);
+        if (move) ldv<V>(q + i, qv);
+        ldv<V>(invd + i, dv);
+        #pragma unroll
+        for (int k = 0; k < V; ++k) {
+            if (move) rv[k] = rv[k] - alpha * qv[k];
+            const A r = A(Storage<TR>::round(arith_t<TR>(rv[k])));   // the level residual as stored
+            Storage<TR>::store(&mv[k], r);
+            Storage<TX>::store(&xv[k], A(omega) * A(Storage<TR>::cvt(dv[k])) * r);
+        }
+        if (move) stv<V>(r_out + i, rv);
+        if (rmg) stv<V>(rmg + i, mv);
+        stv<V>(x + i, xv);
+    });
 }
 
 // out = omega * a * b: a, b auxiliary, out an iterate
@@ -353,12 +428,14 @@ extern "C" int vx_cg_update(int prec, int64_t n, const double* S, void* x, const
                             int update_r, cudaStream_t stream) {
     VX_CHECK_ARG(n > 0, VX_ERR_INVALID_ARGUMENT, "vx_cg_update: n must be positive");
     VX_CHECK_ARG(S && x && p && (!update_r || (r && q)), VX_ERR_NULL_POINTER, "vx_cg_update: NULL pointer");
-    if (prec == VX_F64)
-        vx::launch(cg_update_kernel<double>, nb(n, 256), 256, 0, stream, n, S, (double*)x, (const double*)p, (double*)r,
-                                                                 (const double*)q, update_r, int64_t(0));
-    else if (prec == VX_F32)
-        vx::launch(cg_update_kernel<float>, nb(n, 256), 256, 0, stream, n, S, (float*)x, (const float*)p, (float*)r,
-                                                                (const float*)q, update_r, int64_t(0));
+    auto go = [&](auto t) {
+        using T = decltype(t);
+        const bool w = wide(n, (const T*)x, (const T*)p, update_r ? (const T*)r : nullptr, update_r ? (const T*)q : nullptr);
+        vx::launch(w ? cg_update_kernel<4, T> : cg_update_kernel<1, T>, nb(n, w ? 1024 : 256), 256, 0, stream, n, S, (T*)x,
+                   (const T*)p, (T*)r, (const T*)q, update_r, int64_t(0));
+    };
+    if (prec == VX_F64) go(double());
+    else if (prec == VX_F32) go(float());
     else { set_error("vx_cg_update: unsupported precision %d", prec); return VX_ERR_INVALID_ARGUMENT; }
     VX_CHECK_LAUNCH("vx_cg_update");
     return VX_OK;
@@ -368,15 +445,17 @@ extern "C" int vx_cg_direction(int prec, int zprec, int64_t n, const double* S, 
                                cudaStream_t stream) {
     VX_CHECK_ARG(n > 0, VX_ERR_INVALID_ARGUMENT, "vx_cg_direction: n must be positive");
     VX_CHECK_ARG(S && z && p, VX_ERR_NULL_POINTER, "vx_cg_direction: NULL pointer");
-    if (prec == VX_F64 && zprec == VX_F64)
-        vx::launch(cg_direction_kernel<double, double>, nb(n, 256), 256, 0, stream, n, S, (const double*)z, (double*)p, (double*)z_old, int64_t(0));
-    else if (prec == VX_F64 && zprec == VX_F32)
-        vx::launch(cg_direction_kernel<double, float>, nb(n, 256), 256, 0, stream, n, S, (const float*)z, (double*)p, (float*)z_old, int64_t(0));
-    else if (prec == VX_F64 && zprec == VX_BF16_F32)
-        vx::launch(cg_direction_kernel<double, __nv_bfloat16>, nb(n, 256), 256, 0, stream, n, S, (const __nv_bfloat16*)z, (double*)p,
-                                                                                   (__nv_bfloat16*)z_old, int64_t(0));
-    else if (prec == VX_F32 && zprec == VX_F32)
-        vx::launch(cg_direction_kernel<float, float>, nb(n, 256), 256, 0, stream, n, S, (const float*)z, (float*)p, (float*)z_old, int64_t(0));
+    auto go = [&](auto t, auto tz) {
+        using T = decltype(t);
+        using TZ = decltype(tz);
+        const bool w = wide(n, (const TZ*)z, (const T*)p, (const TZ*)z_old);
+        vx::launch(w ? cg_direction_kernel<4, T, TZ> : cg_direction_kernel<1, T, TZ>, nb(n, w ? 1024 : 256), 256, 0, stream, n,
+                   S, (const TZ*)z, (T*)p, (TZ*)z_old, int64_t(0));
+    };
+    if (prec == VX_F64 && zprec == VX_F64) go(double(), double());
+    else if (prec == VX_F64 && zprec == VX_F32) go(double(), float());
+    else if (prec == VX_F64 && zprec == VX_BF16_F32) go(double(), __nv_bfloat16());
+    else if (prec == VX_F32 && zprec == VX_F32) go(float(), float());
     else { set_error("vx_cg_direction: unsupported precisions %d/%d", prec, zprec); return VX_ERR_INVALID_ARGUMENT; }
     VX_CHECK_LAUNCH("vx_cg_direction");
     return VX_OK;
@@ -388,7 +467,9 @@ extern "C" int vx_cg_direction_update(int zprec, int64_t n, const double* S, con
     VX_CHECK_ARG(S && z && p && x, VX_ERR_NULL_POINTER, "vx_cg_direction_update: NULL pointer");
     const bool ok = dispatch_prec(zprec, [&](auto t) {
         using X = typename decltype(t)::X;
-        vx::launch(cg_direction_update_kernel<double, X>, nb(n, 256), 256, 0, stream, n, S, (const X*)z, p, (X*)z_old, x);
+        const bool w = wide(n, (const X*)z, (const double*)p, (const X*)z_old, (const double*)x);
+        vx::launch(w ? cg_direction_update_kernel<4, double, X> : cg_direction_update_kernel<1, double, X>,
+                   nb(n, w ? 1024 : 256), 256, 0, stream, n, S, (const X*)z, p, (X*)z_old, x);
     });
     VX_CHECK_ARG(ok, VX_ERR_INVALID_ARGUMENT, "vx_cg_direction_update: unsupported precision %d", zprec);
     VX_CHECK_LAUNCH("vx_cg_direction_update");
@@ -488,7 +569,10 @@ extern "C" int vx_vcycle_entry(int prec, int64_t n, const double* r64, void* r_m
     const bool ok = dispatch_prec(prec, [&](auto t) {
         using X = typename decltype(t)::X;
         using R = typename decltype(t)::R;
-        vx::launch(vcycle_entry_kernel<X, R>, nb(n, 256), 256, 0, stream, n, r64, (R*)r_mg, (const R*)inv_diag, omega, (X*)x);
+        const bool w = wide(n, r64, (const R*)r_mg, (const R*)inv_diag, (const X*)x);
+        vx::launch(w ? vcycle_entry_kernel<4, false, X, R> : vcycle_entry_kernel<1, false, X, R>, nb(n, w ? 1024 : 256), 256, 0,
+                   stream, n, (const double*)nullptr, r64, (double*)nullptr, (const double*)nullptr, (R*)r_mg,
+                   (const R*)inv_diag, omega, (X*)x);
     });
     VX_CHECK_ARG(ok, VX_ERR_INVALID_ARGUMENT, "vx_vcycle_entry: unsupported precision %d", prec);
     VX_CHECK_LAUNCH("vx_vcycle_entry");
@@ -502,8 +586,9 @@ extern "C" int vx_vcycle_entry_update(int prec, int64_t n, const double* S, doub
     const bool ok = dispatch_prec(prec, [&](auto t) {
         using X = typename decltype(t)::X;
         using R = typename decltype(t)::R;
-        vx::launch(vcycle_entry_update_kernel<X, R>, nb(n, 256), 256, 0, stream, n, S, r64, q, (R*)r_mg, (const R*)inv_diag,
-                                                                         omega, (X*)x);
+        const bool w = wide(n, (const double*)r64, q, (const R*)r_mg, (const R*)inv_diag, (const X*)x);
+        vx::launch(w ? vcycle_entry_kernel<4, true, X, R> : vcycle_entry_kernel<1, true, X, R>, nb(n, w ? 1024 : 256), 256, 0,
+                   stream, n, S, (const double*)nullptr, r64, q, (R*)r_mg, (const R*)inv_diag, omega, (X*)x);
     });
     VX_CHECK_ARG(ok, VX_ERR_INVALID_ARGUMENT, "vx_vcycle_entry_update: unsupported precision %d", prec);
     VX_CHECK_LAUNCH("vx_vcycle_entry_update");
@@ -615,7 +700,7 @@ extern "C" int vx_batch_cg_update(int prec, int64_t n, int slots, int64_t stride
     VX_CHECK_ARG(n > 0 && slots >= 1 && slots <= 65535, VX_ERR_INVALID_ARGUMENT, "vx_batch_cg_update: bad n/slots");
     VX_CHECK_ARG(S && x && p && (!update_r || (r && q)), VX_ERR_NULL_POINTER, "vx_batch_cg_update: NULL pointer");
     VX_CHECK_ARG(prec == VX_F64, VX_ERR_INVALID_ARGUMENT, "vx_batch_cg_update: unsupported precision %d", prec);
-    vx::launch(cg_update_kernel<double>, dim3(nb(n, 256), slots), 256, 0, stream, n, S, (double*)x, (const double*)p,
+    vx::launch(cg_update_kernel<1, double>, dim3(nb(n, 256), slots), 256, 0, stream, n, S, (double*)x, (const double*)p,
                (double*)r, (const double*)q, update_r, stride);
     VX_CHECK_LAUNCH("vx_batch_cg_update");
     return VX_OK;
@@ -626,10 +711,10 @@ extern "C" int vx_batch_cg_direction(int zprec, int64_t n, int slots, int64_t st
     VX_CHECK_ARG(n > 0 && slots >= 1 && slots <= 65535, VX_ERR_INVALID_ARGUMENT, "vx_batch_cg_direction: bad n/slots");
     VX_CHECK_ARG(S && z && p, VX_ERR_NULL_POINTER, "vx_batch_cg_direction: NULL pointer");
     if (zprec == VX_F64)
-        vx::launch(cg_direction_kernel<double, double>, dim3(nb(n, 256), slots), 256, 0, stream, n, S, (const double*)z, p,
+        vx::launch(cg_direction_kernel<1, double, double>, dim3(nb(n, 256), slots), 256, 0, stream, n, S, (const double*)z, p,
                    (double*)z_old, stride);
     else if (zprec == VX_F32)
-        vx::launch(cg_direction_kernel<double, float>, dim3(nb(n, 256), slots), 256, 0, stream, n, S, (const float*)z, p,
+        vx::launch(cg_direction_kernel<1, double, float>, dim3(nb(n, 256), slots), 256, 0, stream, n, S, (const float*)z, p,
                    (float*)z_old, stride);
     else { set_error("vx_batch_cg_direction: unsupported precision %d", zprec); return VX_ERR_INVALID_ARGUMENT; }
     VX_CHECK_LAUNCH("vx_batch_cg_direction");
