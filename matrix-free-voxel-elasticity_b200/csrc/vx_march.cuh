@@ -19,13 +19,13 @@
 // plane e are written before it; their readers (rows above and below) come after it.  The operand ring
 // has three planes (own read of plane e, neighbour read of e + 1, write of e + 2), the contributions two.
 //
-// What bounds it: the FP64 forms the double-precision pipe (138 of about 300 issued instructions an
-// element row, 45% busy) together with the latency between its barriers, the FP32 sweep HBM and issue.
-// Eight warps and two CTAs an SM (128 registers, no spills) let one CTA compute while the other waits at
-// its barrier; measured at 576x288x288 (us, matvec FP64 / FP32, Jacobi FP64 / FP32): 2 x 8 warps
-// 1040 / 512 / 1195 / 606, 1 x 12 warps 1137 / 562 / 1242 / 685, 1 x 16 warps 1193 / 550 / 1250 / 610;
-// named barriers between neighbouring rows instead of the CTA barrier gave 1102 / 551 with 2 x 8 warps.
-// parity_stream_xp: 1405 / 638 / 1615 / 732.
+// What bounds it: the FP64 forms the double-precision pipe (133 of about 270 issued instructions an element
+// row, half busy) together with the latency between its barriers, the FP32 sweep HBM, issue and registers.
+// Eight warps and two CTAs an SM (128 registers) let one CTA compute while the other waits at its barrier;
+// measured at 576x288x288 (us, matvec FP64 / FP32, Jacobi FP64 / FP32) with one step loop and nine constants
+// more: 2 x 8 warps 1053 / 513 / 1193 / 606, 1 x 12 warps 1137 / 562 / 1242 / 685, 1 x 16 warps 1193 / 550 /
+// 1250 / 610, named barriers between neighbouring rows 1102 / 551 (matvecs); as it is now 1017 / 483 / 1149 /
+// 606 (2.7, 3.3, 3.9 and 4.2 TB/s).  parity_stream_xp: 1405 / 638 / 1615 / 732.
 #pragma once
 
 namespace vx {
@@ -64,36 +64,36 @@ template <typename TC> constexpr size_t march_smem() { return size_t(5) * 3 * Ma
 template <typename TC, bool CUBIC, int PY, int PZ, typename P, typename Args>
 __device__ __forceinline__ void march_blocks(const Args& args, P (&s)[3], P (&d)[3]) {
     if constexpr (CUBIC) {
-        const auto& K = args.K;
+        const auto& K = args.M;
         if constexpr (PY == 0 && PZ == 0) {
             const P bs = cmul2(K.b0, add2(add2(d[0], s[1]), s[2]));          // g0: x@1 y@2 z@4
             d[0] = cfma2(K.amb0, d[0], bs);
             s[1] = cfma2(K.amb0, s[1], bs);
             s[2] = cfma2(K.amb0, s[2], bs);
             const P a1 = d[1], a2 = d[2];                                    // g1: y@3 z@5
-            d[1] = cfma2(K.d1, a2, cmul2(K.c1, a1));
-            d[2] = cfma2(K.d1, a1, cmul2(K.c1, a2));
+            d[1] = cfma2(K.d, a2, a1);
+            d[2] = cfma2(K.d, a1, a2);
         } else if constexpr (PY == 1 && PZ == 0) {
             const P a0 = d[0], a2 = s[2];                                    // g2: x@3 z@6
-            d[0] = cfma2(K.d2, a2, cmul2(K.c2, a0));
-            s[2] = cfma2(K.d2, a0, cmul2(K.c2, a2));
-            const P t = cmul2(K.e3, add2(s[0], d[1]));                       // g3: x@2 y@1, z@7
+            d[0] = cfma2(K.d, a2, a0);
+            s[2] = cfma2(K.d, a0, a2);
+            const P t = cmul2(K.e, add2(s[0], d[1]));                        // g3: x@2 y@1, z@7
             s[0] = t;
             d[1] = t;
-            d[2] = cmul2(K.f3, d[2]);
+            d[2] = cmul2(K.f, d[2]);
         } else if constexpr (PY == 0 && PZ == 1) {
             const P a0 = d[0], a1 = s[1];                                    // g4: x@5 y@6
-            d[0] = cfma2(K.d4, a1, cmul2(K.c4, a0));
-            s[1] = cfma2(K.d4, a0, cmul2(K.c4, a1));
-            const P t = cmul2(K.e5, add2(s[0], d[2]));                       // g5: x@4 z@1, y@7
+            d[0] = cfma2(K.d, a1, a0);
+            s[1] = cfma2(K.d, a0, a1);
+            const P t = cmul2(K.e, add2(s[0], d[2]));                        // g5: x@4 z@1, y@7
             s[0] = t;
             d[2] = t;
-            d[1] = cmul2(K.f5, d[1]);
+            d[1] = cmul2(K.f, d[1]);
         } else {
-            const P t = cmul2(K.e6, add2(s[1], s[2]));                       // g6: y@4 z@2, x@7
+            const P t = cmul2(K.e, add2(s[1], s[2]));                        // g6: y@4 z@2, x@7
             s[1] = t;
             s[2] = t;
-            d[0] = cmul2(K.f6, d[0]);
+            d[0] = cmul2(K.f, d[0]);
             const P ks = cmul2(K.k7, add2(add2(s[0], d[1]), d[2]));          // g7: x@6 y@5 z@3
             s[0] = cfma2(K.hmk7, s[0], ks);
             d[1] = cfma2(K.hmk7, d[1], ks);
@@ -135,6 +135,11 @@ parity_march(const __grid_constant__ OpArgs2<TC, TU, TE, TY, TR> args) {
     constexpr bool HAS_D = EPI == EPI_JACOBI;
     // does the epilogue read the operand at the output node?
     constexpr bool USES_X = EPI == EPI_JACOBI || EPI == EPI_APPLY_DOT;
+    // The FP32 forms with the most epilogue operands have no registers left: they keep one step loop.  The others
+    // run the planes inside the grid in a loop without tests (FP32 matvec 513 -> 483 us, FP64 true residual 1147 ->
+    // 1067 at 576x288x288; in the FP32 sweep that loop spills, 603 -> 701), and in FP32 test a warp's masks by a
+    // vote (in FP64 the vote costs 3%).
+    constexpr bool LEAN = N == 2 && (EPI == EPI_JACOBI || EPI == EPI_TRUE_RES), VOTE = N == 2 && !LEAN;
     const auto& a = args.a;
     const int lane = threadIdx.x & 31;
     const int row = threadIdx.x >> 5;
@@ -174,8 +179,8 @@ parity_march(const __grid_constant__ OpArgs2<TC, TU, TE, TY, TR> args) {
     uint8_t um[N];
     typename Storage<TE>::raw_t er[N];                       // modulus of the next element plane
     // loads of node plane ix (then moves on to ix + 1) and of element plane ex (then ex + 1)
-    auto load_u = [&](int ix) {
-        const int step = ix >= 0 && ix < g.nx ? plane_nodes : 0;
+    auto load_u = [&](int ix, bool inside = false) {
+        const int step = inside || (ix >= 0 && ix < g.nx) ? plane_nodes : 0;
         #pragma unroll
         for (int c = 0; c < N; ++c) {
             const TU* p = a.u + 3 * n_in[c];
@@ -185,8 +190,8 @@ parity_march(const __grid_constant__ OpArgs2<TC, TU, TE, TY, TR> args) {
             n_in[c] += step;
         }
     };
-    auto load_e = [&](int ex) {
-        const bool in = ex >= 0 && ex < g.nx;
+    auto load_e = [&](int ex, bool inside = false) {
+        const bool in = inside || (ex >= 0 && ex < g.nx);
         #pragma unroll
         for (int c = 0; c < N; ++c) {
             er[c] = typename Storage<TE>::raw_t(0.0f);
@@ -204,7 +209,7 @@ parity_march(const __grid_constant__ OpArgs2<TC, TU, TE, TY, TR> args) {
             for (int c = 0; c < N; ++c) v[k][c] = TC(Storage<TU>::cvt(ur[c][k]));
         if constexpr (MASK == MASK_NODE) {
             bits = N == 2 ? unsigned(um[0]) | unsigned(um[N - 1]) << 8 : unsigned(um[0]) | 0x0700u;
-            if ((bits & 0x0707u) != 0x0707u) {               // some DOF is fixed
+            if (!VOTE ? (bits & 0x0707u) != 0x0707u : !__all_sync(0xffffffffu, (bits & 0x0707u) == 0x0707u)) {   // a fixed DOF
                 #pragma unroll
                 for (int k = 0; k < 3; ++k)
                     #pragma unroll
@@ -257,15 +262,19 @@ parity_march(const __grid_constant__ OpArgs2<TC, TU, TE, TY, TR> args) {
     double acc = 0.0;
 
     // element plane e, output node plane e (the first element plane only feeds node plane x0)
-    auto step = [&](int e, auto first) {
-        constexpr bool FIRST = decltype(first)::value;
+    // BULK: planes e + 3 and e + 1 are inside the grid and needed, so nothing is tested
+    auto step = [&](int e, auto first, auto bulk) {
+        constexpr bool FIRST = decltype(first)::value, BULK = decltype(bulk)::value;
         TC ev[N];
         #pragma unroll
-        for (int c = 0; c < N; ++c) ev[c] = TC(Storage<TE>::cvt(er[c]));
-        if (e + 2 <= x1) {
+        for (int c = 0; c < N; ++c) {
+            ev[c] = TC(Storage<TE>::cvt(er[c]));
+            if constexpr (CUBIC) ev[c] *= args.M.scale;
+        }
+        if (BULK || e + 2 <= x1) {
             bits2 = put_u(at2);
-            if (e + 3 <= x1) load_u(e + 3);
-            load_e(e + 1);
+            if (BULK || e + 3 <= x1) load_u(e + 3, BULK);
+            load_e(e + 1, BULK);
         }
         typename Storage<TR>::raw_t rr[N][3], dd[N][3];
         if constexpr (HAS_R && !FIRST) {
@@ -348,46 +357,61 @@ parity_march(const __grid_constant__ OpArgs2<TC, TU, TE, TY, TR> args) {
                 for (int k = 0; k < 3; ++k) xv[k] = us[at0 + own_at + 32 * k];
             }
             const bool sums = e >= a.dot_x0 && e < a.dot_x1;
+            TC xr[N][3], ax[N][3];
             #pragma unroll
-            for (int c = 0; c < N; ++c) {
-                if (!owner[c]) continue;
-                const TU* un = a.u + 3 * n_out[c];
-                const unsigned bb = MASK == MASK_NODE ? bits0 >> (8 * c) : 7u;
-                TC xr[3], ax[3];
+            for (int c = 0; c < N; ++c)
                 #pragma unroll
                 for (int k = 0; k < 3; ++k) {
-                    ax[k] = C::get(yv[k], c);
-                    xr[k] = USES_X ? C::get(xv[k], c) : TC(0);
+                    ax[c][k] = C::get(yv[k], c);
+                    xr[c][k] = USES_X ? C::get(xv[k], c) : TC(0);
                 }
-                if constexpr (MASK == MASK_NODE && EPI != EPI_RESIDUAL) {
-                    if ((bb & 7u) != 7u) {                   // a fixed DOF passes its unmasked operand through
-                        #pragma unroll
-                        for (int k = 0; k < 3; ++k)
-                            if (!((bb >> k) & 1u)) ax[k] = xr[k] = TC(Storage<TU>::load(un + k));
-                    }
-                }
+            auto fix = [&](int c) {                          // fixed DOFs: the unmasked operand, or a zero residual
                 #pragma unroll
                 for (int k = 0; k < 3; ++k) {
-                    TC o;
-                    if constexpr (EPI == EPI_RAW) {
-                        o = ax[k];
-                    } else if constexpr (EPI == EPI_APPLY_DOT) {
-                        o = ax[k];
-                        if (sums) acc += double(xr[k]) * double(ax[k]);
+                    if ((bits0 >> (8 * c + k)) & 1u) continue;
+                    if constexpr (EPI == EPI_RESIDUAL) {
+                        rr[c][k] = typename Storage<TR>::raw_t(0.0f);
+                        ax[c][k] = TC(0);
                     } else {
-                        const TC r_ = TC(Storage<TR>::cvt(rr[c][k]));
-                        if constexpr (EPI == EPI_JACOBI) {
-                            o = xr[k] + a.omega * TC(Storage<TR>::cvt(dd[c][k])) * (r_ - ax[k]);
-                        } else if constexpr (EPI == EPI_RESIDUAL) {
-                            o = r_ - ax[k];
-                            if (MASK == MASK_NODE && !((bb >> k) & 1u)) o = TC(0);
-                        } else {
-                            o = r_ - ax[k];
-                            if (sums) acc += double(o) * double(o);
-                        }
+                        ax[c][k] = xr[c][k] = TC(Storage<TU>::load(a.u + 3 * n_out[c] + k));
                     }
-                    Storage<TY>::store(a.y + 3 * n_out[c] + k, o);
                 }
+            };
+            auto put = [&](int c) {
+                TC o[3];
+                #pragma unroll
+                for (int k = 0; k < 3; ++k) {
+                    if constexpr (EPI == EPI_RAW || EPI == EPI_APPLY_DOT) o[k] = ax[c][k];
+                    else {
+                        const TC r_ = TC(Storage<TR>::cvt(rr[c][k]));
+                        if constexpr (EPI == EPI_JACOBI)
+                            o[k] = xr[c][k] + a.omega * TC(Storage<TR>::cvt(dd[c][k])) * (r_ - ax[c][k]);
+                        else o[k] = r_ - ax[c][k];
+                    }
+                }
+                if (!owner[c]) return;
+                #pragma unroll
+                for (int k = 0; k < 3; ++k) {
+                    Storage<TY>::store(a.y + 3 * n_out[c] + k, o[k]);
+                    if constexpr (EPI == EPI_APPLY_DOT || EPI == EPI_TRUE_RES) {
+                        if (sums) acc += double(EPI == EPI_TRUE_RES ? o[k] : xr[c][k]) * double(o[k]);
+                    }
+                }
+            };
+            if constexpr (!VOTE) {
+                #pragma unroll
+                for (int c = 0; c < N; ++c) {
+                    if (!owner[c]) continue;
+                    if (MASK == MASK_NODE && ((bits0 >> (8 * c)) & 7u) != 7u) fix(c);
+                    put(c);
+                }
+            } else {
+                if (MASK == MASK_NODE && !__all_sync(0xffffffffu, (bits0 & 0x0707u) == 0x0707u)) {
+                    #pragma unroll
+                    for (int c = 0; c < N; ++c) fix(c);
+                }
+                #pragma unroll
+                for (int c = 0; c < N; ++c) put(c);
             }
         }
         #pragma unroll
@@ -397,9 +421,12 @@ parity_march(const __grid_constant__ OpArgs2<TC, TU, TE, TY, TR> args) {
         hat = RING - hat;
         bits0 = bits1; bits1 = bits2;
     };
-    step(x0 - 1, std::true_type{});
+    step(x0 - 1, std::true_type{}, std::false_type{});
+    int e = x0;
     #pragma unroll 1
-    for (int e = x0; e < x1; ++e) step(e, std::false_type{});
+    for (const int eb = LEAN ? x0 : min(x1, g.nx - 1) - 2; e < eb; ++e) step(e, std::false_type{}, std::true_type{});
+    #pragma unroll 1
+    for (; e < x1; ++e) step(e, std::false_type{}, std::false_type{});
     if constexpr (EPI == EPI_TRUE_RES || EPI == EPI_APPLY_DOT) {
         const int64_t bid = (int64_t(blockIdx.z) * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;
         block_sum_store<NWS * 32>(acc, a.partials + bid);

@@ -56,6 +56,7 @@ struct OpArgs {
     double emin, de, penal;   // SIMP modulus E = emin + de * rho^penal
     int cx;                   // owned node planes per CTA (x chunk)
     bool cubic;               // host side: the blocks have the cube pattern (CubeK)
+    const double* blocks;     // host side: the 72 parity coefficients
     bool xp;                  // host side: parity_stream_xp instead of parity_march (VX_STREAM_XP)
     BlocksT<TC> C;
 };
@@ -319,11 +320,20 @@ template <typename TC> struct CubeK {
     typename Coef<TC>::type amb0, b0, c1, d1, c2, d2, c4, d4, e3, f3, e5, f5, e6, f6, hmk7, k7;
 };
 
+// The same with all edges equal for parity_march: the three axes' blocks agree (g1 = g2 = g4, g3 = g5 = g6), and
+// the modulus is scaled by c so that [c d; d c] becomes [1 d/c; d/c 1].  Seven constants: each one held in the
+// constant bank costs its moves to registers every step.
+template <typename TC> struct MarchK {
+    typename Coef<TC>::type amb0, b0, d, e, f, hmk7, k7;
+    TC scale;
+};
+
 template <typename TC, typename TU, typename TE, typename TY, typename TR = TY>
 struct OpArgs2 {
     OpArgs<TC, TU, TE, TY, TR> a;
     Blocks2<TC> C2;
     CubeK<TC> K;
+    MarchK<TC> M;
 };
 }  // namespace vx
 
@@ -374,6 +384,34 @@ CubeK<TC> cube_constants(const BlocksT<TC>& C) {
     K.e6 = k(B(6, 1, 1)); K.f6 = k(B(6, 0, 0));
     K.hmk7 = k(B(7, 0, 0) - B(7, 0, 1)); K.k7 = k(B(7, 0, 1));
     return K;
+}
+
+// true if the cube pattern holds and the blocks agree between the axes (to 1e-14 of the largest)
+inline bool cube_symmetric(const double* c) {
+    double m = 0;
+    for (int i = 0; i < 72; ++i) m = std::max(m, std::fabs(c[i]));
+    auto B = [&](int g, int r, int col) { return c[9 * g + 3 * r + col]; };
+    auto eq = [&](double x, double y) { return std::fabs(x - y) <= 1e-14 * m; };
+    return B(1, 1, 1) != 0.0 && eq(B(1, 1, 1), B(2, 0, 0)) && eq(B(1, 1, 1), B(4, 0, 0)) && eq(B(1, 1, 2), B(2, 0, 2)) &&
+           eq(B(1, 1, 2), B(4, 0, 1)) && eq(B(3, 0, 0), B(5, 0, 0)) && eq(B(3, 0, 0), B(6, 1, 1)) &&
+           eq(B(3, 2, 2), B(5, 1, 1)) && eq(B(3, 2, 2), B(6, 0, 0));
+}
+
+template <typename TC>
+MarchK<TC> march_constants(const double* c) {
+    auto k = [](double v) {
+        if constexpr (std::is_same<TC, float>::value) return make_float2(float(v), float(v));
+        else return v;
+    };
+    auto B = [&](int g, int r, int col) { return c[9 * g + 3 * r + col]; };
+    const double s = B(1, 1, 1);
+    MarchK<TC> M;
+    M.amb0 = k((B(0, 0, 0) - B(0, 0, 1)) / s); M.b0 = k(B(0, 0, 1) / s);
+    M.d = k(B(1, 1, 2) / s);
+    M.e = k(B(3, 0, 0) / s); M.f = k(B(3, 2, 2) / s);
+    M.hmk7 = k((B(7, 0, 0) - B(7, 0, 1)) / s); M.k7 = k(B(7, 0, 1) / s);
+    M.scale = TC(s);
+    return M;
 }
 
 // ============================================================================= parity_stream_xp
@@ -799,7 +837,10 @@ OpArgs2<TC, TU, TE, TY, TR> packed_args(const OpArgs<TC, TU, TE, TY, TR>& a) {
         if constexpr (std::is_same<TC, float>::value) a2.C2.c[i] = make_float2(a.C.c[i], a.C.c[i]);
         else a2.C2.c[i] = a.C.c[i];
     }
-    if (a.cubic) a2.K = cube_constants<TC>(a.C);
+    if (a.cubic) {
+        a2.K = cube_constants<TC>(a.C);
+        a2.M = march_constants<TC>(a.blocks);
+    }
     return a2;
 }
 
@@ -843,8 +884,9 @@ int launch_stream(const OpArgs<TC, TU, TE, TY, TR>& a_in, cudaStream_t s, const 
                       size_t(2) * XpCfg<TC>::NW * 6 * 32 * sizeof(V2<TC>));
         }
         const dim3 grid = march_grid<TC>(a.g, &a.cx);
-        return go(cubic ? parity_march<TC, TU, TE, TY, TR, EPI, MASK, true> : parity_march<TC, TU, TE, TY, TR, EPI, MASK, false>,
-                  configured[cubic ? 1 : 0], grid, March<TC>::NW * 32, march_smem<TC>());
+        const bool cube = cubic && cube_symmetric(a.blocks);
+        return go(cube ? parity_march<TC, TU, TE, TY, TR, EPI, MASK, true> : parity_march<TC, TU, TE, TY, TR, EPI, MASK, false>,
+                  configured[cube ? 1 : 0], grid, March<TC>::NW * 32, march_smem<TC>());
     } else {
         const Tiling t = tiling(VX_F64, false);
         a.cx = stream_cx(a.g, t);
@@ -998,6 +1040,7 @@ extern "C" int vx_matvec(int sel, int nx, int ny, int nz, const double* blocks, 
         a.g = Grid{nx, ny, nz}; a.u = (const X*)u; a.E = (const M*)E; a.y = (TC*)y; a.node_mask = node_mask;
         a.C = convert_blocks<TC>(blocks);
         a.cubic = cube_pattern(blocks);
+            a.blocks = blocks;
         a.xp = sel & VX_STREAM_XP;
         rc = node_mask ? launch_stream<TC, X, M, TC, EPI_RAW, MASK_NODE, false, false>(a, stream, "vx_matvec")
                        : launch_stream<TC, X, M, TC, EPI_RAW, MASK_NONE, false, false>(a, stream, "vx_matvec");
@@ -1168,6 +1211,7 @@ int fused_dispatch(const char* what, int sel, int nx, int ny, int nz, const doub
             a.fin = fin; a.S = S; a.counter = counter;
             a.C = convert_blocks<TC>(blocks);
             a.cubic = cube_pattern(blocks);
+            a.blocks = blocks;
             a.xp = sel & VX_STREAM_XP;
             rc = node_mask ? launch_stream<TC, X, M, TY, EPI, MASK_NODE, false, false, R>(a, stream, what)
                            : launch_stream<TC, X, M, TY, EPI, MASK_NONE, false, false, R>(a, stream, what);
