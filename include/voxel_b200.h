@@ -295,6 +295,19 @@ int vx_tc_element_product(int nx, int ny, int nz, const double* ke, const float*
 /* Fault flag of vx_tc_element_product's bounded accumulator wait, as vx_device_status. */
 int vx_tc_status(int* status, int clear);
 
+/* The coarsest system of an (nx, ny, nz) grid factored from its dense matrix A (n x n, n = 3 nodes) with its
+ * planes split at the middle one: the two halves side by side, then the plane.  vx_split_factor_size and
+ * vx_split_workspace give the doubles of `factor` and `work` (0 when the grid does not split: fewer than
+ * five node planes, or a band wider than a half); info: 3 ints, non-zero where a matrix is not positive
+ * definite.  vx_split_apply: z = A^-1 r, masked; y: n + 3 (ny + 1)(nz + 1) doubles of work.  Replaces
+ * src/voxel_mg.py:107-116,152-159 like vx_coarse_factor / vx_coarse_apply_factor. */
+int64_t vx_split_factor_size(int nx, int ny, int nz);
+int64_t vx_split_workspace(int nx, int ny, int nz);
+int vx_split_factor(int nx, int ny, int nz, const double* A, double* factor, double* work, int* info,
+                    cudaStream_t stream);
+int vx_split_apply(int prec, int nx, int ny, int nz, const double* factor, const void* r,
+                   const uint8_t* node_mask, double* y, void* z, cudaStream_t stream);
+
 /* The coarsest level's exact solve, set up without library calls (replaces the host Cholesky and the
  * two triangular solves of src/voxel_mg.py:152-159, experiments/session_i/run_gpu.py:281-286).
  * A: the dense n x n constrained matrix (vx_assemble_dense, row-major, symmetric positive definite),

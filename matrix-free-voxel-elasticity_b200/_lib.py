@@ -67,6 +67,10 @@ SIGNATURES = {
     "vx_tc_element_product": (c_int, [c_int, c_int, c_int, _D, c_void_p, c_void_p, c_void_p, c_void_p, c_int,
                                       c_void_p]),
     "vx_tc_status": (c_int, [POINTER(c_int), c_int]),
+    "vx_split_factor_size": (c_int64, [c_int, c_int, c_int]),
+    "vx_split_workspace": (c_int64, [c_int, c_int, c_int]),
+    "vx_split_factor": (c_int, [c_int, c_int, c_int, _P, _P, _P, _P, _P]),
+    "vx_split_apply": (c_int, [c_int, c_int, c_int, c_int, _P, _P, _P, _P, _P, _P]),
     "vx_coarse_factor_workspace": (c_int64, [c_int, c_int]),
     "vx_coarse_factor": (c_int, [c_int, c_int, _P, _P, _P, _P, _P]),
     "vx_batch_coarse_factor": (c_int, [c_int, c_int, c_int, POINTER(c_int), _P, _P, _P, _P, _P]),
@@ -154,13 +158,13 @@ CAPTURE_STREAM = None
 
 # Kernel launches issued by each entry point (entry points not listed launch none or one:
 # host-only entry points are in HOST_ONLY).  Used to count this library's launches.
-KERNELS_PER_CALL = {"vx_tc_element_product": 1, "vx_coarse_pack_factor": 3, "vx_dots": 2, "vx_assemble_dense": 1, "vx_true_residual_noalloc": 2, "vx_coarse_apply_factor": 2,
+KERNELS_PER_CALL = {"vx_tc_element_product": 1, "vx_coarse_pack_factor": 3, "vx_dots": 2, "vx_assemble_dense": 1, "vx_true_residual_noalloc": 2, "vx_coarse_apply_factor": 2, "vx_split_apply": 2,
                     "vx_batch_coarse_apply_factor": 2}
 HOST_ONLY = {"vx_last_error", "vx_version", "vx_element_matrix", "vx_element", "vx_parity_blocks",
              "vx_operator_partials", "vx_partials_size", "vx_jacobi_step_partials", "vx_small_cg_limit", "vx_solver_slots", "vx_solver_partials",
              "vx_graph_while_begin", "vx_graph_destroy", "vx_capture_status", "vx_graph_launch",
              "vx_oc_partials", "vx_graph_body_nodes", "vx_plane_fix_partials", "vx_device_status",
-             "vx_coarse_factor_workspace", "vx_set_stream_kernel",
+             "vx_coarse_factor_workspace", "vx_split_factor_size", "vx_split_workspace", "vx_set_stream_kernel",
              "vx_tc_status"}
 launches = 0          # kernels launched directly (graph launches are counted by the solvers)
 
@@ -170,7 +174,7 @@ _FNS = {}             # name -> (bound entry point, its kernels per call; None: 
 
 def _bind(name: str):
     count = KERNELS_PER_CALL.get(name, 0 if name in HOST_ONLY else 1)
-    if name in ("vx_coarse_factor", "vx_batch_coarse_factor"):
+    if name in ("vx_coarse_factor", "vx_batch_coarse_factor", "vx_split_factor"):
         count = None
     entry = _FNS[name] = (getattr(load(), name), count)
     return entry
@@ -184,7 +188,10 @@ def call(name: str, *args) -> None:
     status = fn(*args)
     if status:
         check(status, name)
-    if count is None:                     # load, a factor and an update per block, inverse
+    if count is None and name == "vx_split_factor":    # two chains as below, four products
+        planes, p = int(args[0]) + 1, 3 * (int(args[1]) + 1) * (int(args[2]) + 1)
+        count = 2 * ((planes // 2 * p + 63) // 64) + 2 * ((p + 63) // 64) + 6
+    elif count is None:                   # load, a factor and an update per block, inverse
         count = 2 * ((int(args[0]) + 63) // 64) + 1
     launches += count
     if CAPTURE_STREAM is not None and _lib.vx_capture_status(CAPTURE_STREAM) == 2:

@@ -721,6 +721,41 @@ extern "C" int64_t vx_coarse_factor_workspace(int n, int bw) {
     return int64_t(n) * (bw + 1) + nblk * CB * CB + int64_t(bw + 1) * CB;
 }
 
+// The chain of block factorisations and trailing updates, and the inverse factor, of B loaded bands.
+static void launch_chain(int n, int bw, unsigned B, const FactorBatch& fb, cudaStream_t stream) {
+    const size_t psm = size_t(2 * CB * CBP + HB * HBP) * sizeof(double);
+    const size_t usm = size_t(CB + 2 * UQ) * CBP * sizeof(double);
+    for (int k0 = 0; k0 < n; k0 += CB) {
+        vx::launch(band_potrf_kernel<true>, dim3(1, B), POTRF_T, psm, stream, n, bw, k0, fb);
+        const int w = std::min(CB, n - k0);
+        const int rows = std::min(n, k0 + w + bw) - (k0 + w);
+        if (rows <= 0) continue;
+        const int T = (rows + CB - 1) / CB;
+        vx::launch(band_update_kernel, dim3(unsigned(4 * (T * (T + 1) / 2)), B), UPDATE_T, usm, stream, n, bw, k0, T, fb);
+    }
+}
+static void launch_inverse(int n, int bw, unsigned B, int nw, const FactorBatch& fb, cudaStream_t stream) {
+    const InvbLayout<INV_TC> il(bw);
+    if (il.bytes <= 227 * 1024) {
+        vx::launch(band_inverse_blocked_kernel<INV_TC>, dim3(unsigned((n + INV_TC - 1) / INV_TC), B), INVB_T, il.bytes, stream, n,
+                   bw, fb);
+    } else {
+        const size_t ism = size_t(INV_STAGES + nw) * (bw + 1) * sizeof(double);
+        vx::launch(band_inverse_kernel, dim3(unsigned((n + nw - 1) / nw), B), unsigned(nw * 32), ism, stream, n, bw,
+                   fb);
+    }
+}
+static int opt_in_factor(const char* what) {
+    const size_t psm = size_t(2 * CB * CBP + HB * HBP) * sizeof(double);
+    const size_t usm = size_t(CB + 2 * UQ) * CBP * sizeof(double);
+    static std::atomic<uint64_t> opt_p, opt_u, opt_i, opt_b;
+    int st = smem_opt_in(opt_p, (const void*)band_potrf_kernel<true>, psm, what);
+    if (!st) st = smem_opt_in(opt_u, (const void*)band_update_kernel, usm, what);
+    if (!st) st = smem_opt_in(opt_i, (const void*)band_inverse_kernel, 227 * 1024, what);
+    if (!st) st = smem_opt_in(opt_b, (const void*)band_inverse_blocked_kernel<INV_TC>, 227 * 1024, what);
+    return st;
+}
+
 // count factorisations of one size (matrix slots slots[0..count) of A, packed and info; workspace m
 // of work for the m-th), every launch covering all of them (blockIdx.y).
 static int coarse_factor_batch(const char* what, int n, int bw, int count, const int* slots, const double* A,
@@ -750,34 +785,13 @@ static int coarse_factor_batch(const char* what, int n, int bw, int count, const
             return VX_ERR_CUDA;
         }
     }
-    const size_t psm = size_t(2 * CB * CBP + HB * HBP) * sizeof(double);
-    const size_t usm = size_t(CB + 2 * UQ) * CBP * sizeof(double);
-    const size_t ism = size_t(INV_STAGES + nw) * (bw + 1) * sizeof(double);
-    static std::atomic<uint64_t> opt_p, opt_u, opt_i, opt_b;
-    int st = smem_opt_in(opt_p, (const void*)band_potrf_kernel<true>, psm, what);
-    if (!st) st = smem_opt_in(opt_u, (const void*)band_update_kernel, usm, what);
-    if (!st) st = smem_opt_in(opt_i, (const void*)band_inverse_kernel, 227 * 1024, what);
-    if (!st) st = smem_opt_in(opt_b, (const void*)band_inverse_blocked_kernel<INV_TC>, 227 * 1024, what);
+    const int st = opt_in_factor(what);
     if (st) return st;
     const unsigned B = unsigned(count);
     const int64_t band = int64_t(n) * (bw + 1);
     vx::launch(band_load_kernel, dim3(unsigned((band + 255) / 256), B), 256, 0, stream, n, bw, fb);
-    for (int k0 = 0; k0 < n; k0 += CB) {
-        vx::launch(band_potrf_kernel<true>, dim3(1, B), POTRF_T, psm, stream, n, bw, k0, fb);
-        const int w = std::min(CB, n - k0);
-        const int rows = std::min(n, k0 + w + bw) - (k0 + w);
-        if (rows <= 0) continue;
-        const int T = (rows + CB - 1) / CB;
-        vx::launch(band_update_kernel, dim3(unsigned(4 * (T * (T + 1) / 2)), B), UPDATE_T, usm, stream, n, bw, k0, T, fb);
-    }
-    const InvbLayout<INV_TC> il(bw);
-    if (il.bytes <= 227 * 1024) {
-        vx::launch(band_inverse_blocked_kernel<INV_TC>, dim3(unsigned((n + INV_TC - 1) / INV_TC), B), INVB_T, il.bytes, stream, n,
-                   bw, fb);
-    } else {
-        vx::launch(band_inverse_kernel, dim3(unsigned((n + nw - 1) / nw), B), unsigned(nw * 32), ism, stream, n, bw,
-                   fb);
-    }
+    launch_chain(n, bw, B, fb, stream);
+    launch_inverse(n, bw, B, nw, fb, stream);
     VX_CHECK_LAUNCH(what);
     return VX_OK;
 }
@@ -843,5 +857,314 @@ extern "C" int vx_coarse_pack_factor(int n, int bw, const double* L, double* pac
                    fb);
     }
     VX_CHECK_LAUNCH(what);
+    return VX_OK;
+}
+
+// ----------------------------------------------------------------------------- split coarse system
+// The coarsest system split at a middle node plane.  The planes left of it and, in reverse order, those right
+// of it are two independent banded systems X = L, R of one size (an even number of planes: R is padded with a
+// decoupled plane of identity rows at its far end); eliminating both first and the plane s last,
+//     W_X = [Linv_X's last p x p block] B_X     (B_X: the coupling of X's last plane with s, p DOFs a plane)
+//     S   = A_ss - W_L^T W_L - W_R^T W_R = L_s L_s^T
+//     M_X = -Linv_s W_X^T [Linv_X's last p rows]
+// the inverse factor is [Linv_L; Linv_R; M_L M_R Linv_s]: half the chain of dependent block factorisations
+// (34 + 4 blocks of 64 instead of 65 for 17 planes of 243) and 0.56 of the bytes of the dense triangles, which
+// then stay in L2.  Factor, and a solve (one band -> split): n = 4131 2.61 -> 1.58 ms, 36 -> 21 us; n = 5700 4.12 ->
+// 2.57 ms, 63 -> 40 us; n = 1911 1.11 -> 0.73 ms, 17 -> 10 us.
+namespace vx {
+
+struct SplitShape {
+    int n, p, n2, pad, sep;      // DOFs, DOFs a plane, DOFs of a half, padded DOFs of R, first DOF of the plane s
+    int bw;                      // half-bandwidth of a half
+};
+static bool split_shape(int nx, int ny, int nz, SplitShape* sh) {
+    const int planes = nx + 1;
+    sh->p = 3 * (ny + 1) * (nz + 1);
+    sh->n = planes * sh->p;
+    sh->n2 = planes / 2 * sh->p;
+    sh->pad = planes % 2 ? 0 : sh->p;
+    sh->sep = sh->n2;
+    sh->bw = 3 * ((ny + 1) * (nz + 1) + (nz + 1) + 1) + 2;
+    return planes >= 5 && sh->bw < sh->n2 && inverse_warps(sh->bw) > 0;
+}
+// global DOF of entry i of half X (i >= pad for R)
+__host__ __device__ __forceinline__ int split_dof(const SplitShape& s, int X, int i) { return X ? s.n - 1 - (i - s.pad) : i; }
+
+__global__ void split_load_kernel(SplitShape s, const double* __restrict__ A, const __grid_constant__ FactorBatch fb) {
+    vx::pdl_begin();
+    const FactorPtrs P = fptrs(fb, s.n2, s.bw);
+    const int X = blockIdx.y;
+    const int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+    if (t >= int64_t(s.n2) * (s.bw + 1)) return;
+    const int i = int(t / (s.bw + 1)), j = i - s.bw + int(t % (s.bw + 1)), pad = X ? s.pad : 0;
+    double v = 0.0;
+    if (i < pad) v = i == j ? 1.0 : 0.0;
+    else if (j >= pad) v = A[int64_t(split_dof(s, X, i)) * s.n + split_dof(s, X, j)];
+    P.lb[t] = v;
+}
+
+// C = alpha op(A) op(B) + D for m x n results and depth k, elements by row and column strides; lower_a / lower_b:
+// entries of A right of its diagonal, of B right of column k0b + row, count as zero.  blockIdx.z adds the z
+// offsets.  64 x 64 tiles, a 4 x 4 register tile a thread; a few us each, none of them is worth more.
+struct SplitGemm {
+    int m, n, k, lower_a, lower_b, k0b;
+    double alpha;
+    const double *a, *b, *d;
+    double *c, *ct;
+    int64_t ar, ac, az, br, bc, bz, dr, dc, cr, cc, cz, ctr, ctc, ctz;
+};
+__global__ void __launch_bounds__(256) split_gemm_kernel(const __grid_constant__ SplitGemm g) {
+    vx::pdl_begin();
+    __shared__ double As[16][65], Bs[16][65];
+    const int t = threadIdx.x, i0 = blockIdx.y * 64, j0 = blockIdx.x * 64, tr = t / 16, tc = t % 16;
+    const double* a = g.a + g.az * blockIdx.z;
+    const double* b = g.b + (blockIdx.z ? g.bz : 0);
+    const int64_t br = blockIdx.z && g.lower_b < 0 ? -g.br : g.br;
+    double acc[4][4] = {};
+    for (int k0 = 0; k0 < g.k; k0 += 16) {
+        #pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const int q = t + 256 * u;
+            // the faster index of the stage runs along the unit stride
+            const int ka = g.ac == 1 ? q % 16 : q / 64, ia = g.ac == 1 ? q / 16 : q % 64;
+            const int kb = g.br == 1 ? q % 16 : q / 64, jb = g.br == 1 ? q / 16 : q % 64;
+            const int i = i0 + ia, j = j0 + jb, k1 = k0 + ka, k2 = k0 + kb;
+            As[ka][ia] = i < g.m && k1 < g.k && !(g.lower_a && k1 > i) ? a[i * g.ar + k1 * g.ac] : 0.0;
+            Bs[kb][jb] = j < g.n && k2 < g.k && !(g.lower_b > 0 && j > g.k0b + k2) ? b[k2 * br + j * g.bc] : 0.0;
+        }
+        __syncthreads();
+        #pragma unroll
+        for (int k = 0; k < 16; ++k) {
+            double av[4], bv[4];
+            #pragma unroll
+            for (int x = 0; x < 4; ++x) { av[x] = As[k][tr + 16 * x]; bv[x] = Bs[k][tc + 16 * x]; }
+            #pragma unroll
+            for (int x = 0; x < 4; ++x)
+                #pragma unroll
+                for (int y = 0; y < 4; ++y) acc[x][y] = fma(av[x], bv[y], acc[x][y]);
+        }
+        __syncthreads();
+    }
+    #pragma unroll
+    for (int x = 0; x < 4; ++x)
+        #pragma unroll
+        for (int y = 0; y < 4; ++y) {
+            const int i = i0 + tr + 16 * x, j = j0 + tc + 16 * y;
+            if (i >= g.m || j >= g.n) continue;
+            double v = g.alpha * acc[x][y];
+            if (g.d) v += g.d[i * g.dr + j * g.dc];
+            g.c[g.cz * blockIdx.z + i * g.cr + j * g.cc] = v;
+            if (g.ct) g.ct[g.ctz * blockIdx.z + i * g.ctr + j * g.ctc] = v;
+        }
+}
+static void launch_gemm(const SplitGemm& g, int z, cudaStream_t stream) {
+    vx::launch(split_gemm_kernel, dim3(unsigned((g.n + 63) / 64), unsigned((g.m + 63) / 64), unsigned(z)), 256, 0, stream, g);
+}
+
+// factor: [packed_L][packed_R] (n2 x n2), [packed_s] (p x p), [M_L][M_R] (p x n2), [M_L^T][M_R^T] (n2 x p)
+struct SplitFactor { int64_t ps, m, mt, total; };
+static SplitFactor split_factor_layout(const SplitShape& s) {
+    SplitFactor f;
+    f.ps = 2 * int64_t(s.n2) * s.n2;
+    f.m = f.ps + int64_t(s.p) * s.p;
+    f.mt = f.m + 2 * int64_t(s.p) * s.n2;
+    f.total = f.mt + 2 * int64_t(s.p) * s.n2;
+    return f;
+}
+
+// sum of a CTA's threads' s, valid in thread 0 (the order of coarse_lower_kernel's row sums)
+constexpr int ST = 256;
+__device__ __forceinline__ double split_sum(double s) {
+    __shared__ double red[ST / 32];
+    #pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
+    __syncthreads();
+    double t = 0.0;
+    if (threadIdx.x == 0)
+        for (int k = 0; k < ST / 32; ++k) t += red[k];
+    return t;
+}
+
+// y = Linv r in the split order: rows of L, of R, of s (y[0 .. 2 n2 + p)), one CTA per row.
+template <typename TR>
+__global__ void __launch_bounds__(ST) split_lower_kernel(SplitShape s, SplitFactor f, const double* __restrict__ F,
+                                                         const TR* __restrict__ r, double* __restrict__ y) {
+    vx::pdl_begin();
+    const int row = blockIdx.x, t = threadIdx.x;
+    auto rv = [&](int X, int j) { return double(Storage<TR>::load(r + split_dof(s, X, j))); };
+    double v = 0.0;
+    if (row < 2 * s.n2) {
+        const int X = row >= s.n2, i = row - X * s.n2;
+        const double* m = F + (int64_t(X) * s.n2 + i) * s.n2;
+        for (int j = (X ? s.pad : 0) + t; j <= i; j += ST) v = fma(m[j], rv(X, j), v);
+    } else {
+        const int k = row - 2 * s.n2;
+        const double* m = F + f.ps + int64_t(k) * s.p;
+        for (int j = t; j <= k; j += ST) v = fma(m[j], double(Storage<TR>::load(r + s.sep + j)), v);
+        for (int X = 0; X < 2; ++X) {
+            const double* c = F + f.m + (int64_t(X) * s.p + k) * s.n2;
+            for (int j = (X ? s.pad : 0) + t; j < s.n2; j += ST) v = fma(c[j], rv(X, j), v);
+        }
+    }
+    v = split_sum(v);
+    if (t == 0) y[row] = v;
+}
+
+// z = Linv^T y, masked, in DOF order
+template <typename T>
+__global__ void __launch_bounds__(ST) split_upper_kernel(SplitShape s, SplitFactor f, const double* __restrict__ F,
+                                                         const double* __restrict__ y, const uint8_t* __restrict__ mask,
+                                                         T* __restrict__ z) {
+    vx::pdl_begin();
+    using A = arith_t<T>;
+    const int row = blockIdx.x, t = threadIdx.x;
+    const double* ys = y + 2 * s.n2;
+    double v = 0.0;
+    int dof;
+    if (row < 2 * s.n2) {
+        const int X = row >= s.n2, i = row - X * s.n2;
+        if (X && i < s.pad) return;
+        dof = split_dof(s, X, i);
+        const double* m = F + (int64_t(X) * s.n2 + i) * s.n2;
+        const double* c = F + f.mt + (int64_t(X) * s.n2 + i) * s.p;
+        for (int j = i + t; j < s.n2; j += ST) v = fma(m[j], y[X * s.n2 + j], v);
+        for (int k = t; k < s.p; k += ST) v = fma(c[k], ys[k], v);
+    } else {
+        const int k = row - 2 * s.n2;
+        dof = s.sep + k;
+        const double* m = F + f.ps + int64_t(k) * s.p;
+        for (int j = k + t; j < s.p; j += ST) v = fma(m[j], ys[j], v);
+    }
+    v = split_sum(v);
+    if (t == 0) {
+        const bool fr = mask ? ((mask[dof / 3] >> (dof % 3)) & 1u) : true;
+        Storage<T>::store(z + dof, fr ? A(v) : A(0));
+    }
+}
+
+}  // namespace vx
+
+extern "C" int64_t vx_split_factor_size(int nx, int ny, int nz) {
+    SplitShape s;
+    if (check_grid(nx, ny, nz) || !split_shape(nx, ny, nz, &s)) return 0;
+    return split_factor_layout(s).total;
+}
+
+extern "C" int64_t vx_split_workspace(int nx, int ny, int nz) {
+    SplitShape s;
+    if (check_grid(nx, ny, nz) || !split_shape(nx, ny, nz, &s)) return 0;
+    const int64_t pp = int64_t(s.p) * s.p;
+    return 2 * vx_coarse_factor_workspace(s.n2, s.bw) + vx_coarse_factor_workspace(s.p, s.p - 1) + 5 * pp;
+}
+
+extern "C" int vx_split_factor(int nx, int ny, int nz, const double* A, double* factor, double* work, int* info,
+                               cudaStream_t stream) {
+    const char* what = "vx_split_factor";
+    int st = check_grid(nx, ny, nz);
+    if (st) return st;
+    VX_CHECK_ARG(A && factor && work && info, VX_ERR_NULL_POINTER, "%s: NULL pointer", what);
+    SplitShape s;
+    VX_CHECK_ARG(split_shape(nx, ny, nz, &s), VX_ERR_INVALID_ARGUMENT, "%s: grid (%d, %d, %d) does not split", what, nx, ny, nz);
+    const SplitFactor f = split_factor_layout(s);
+    st = opt_in_factor(what);
+    if (st) return st;
+    cudaError_t e = cudaMemsetAsync(info, 0, 3 * sizeof(int), stream);
+    if (e != cudaSuccess) {
+        set_error("%s: memset: %s", what, cudaGetErrorString(e));
+        return VX_ERR_CUDA;
+    }
+    const int p = s.p, n2 = s.n2;
+    const int64_t pp = int64_t(p) * p;
+    FactorBatch h{};
+    h.packed = factor;
+    h.work = work;
+    h.info = info;
+    h.mat = int64_t(n2) * n2;
+    h.ws = vx_coarse_factor_workspace(n2, s.bw);
+    h.nblk = (n2 + CB - 1) / CB;
+    h.slot[0] = 0;
+    h.slot[1] = 1;
+    double* const swork = work + 2 * h.ws;
+    double* const W = swork + vx_coarse_factor_workspace(p, p - 1);
+    double* const S = W + 2 * pp;
+    double* const G = S + pp;
+    const int64_t band = int64_t(n2) * (s.bw + 1);
+    vx::launch(split_load_kernel, dim3(unsigned((band + 255) / 256), 2), 256, 0, stream, s, A, h);
+    launch_chain(n2, s.bw, 2, h, stream);
+    launch_inverse(n2, s.bw, 2, inverse_warps(s.bw), h, stream);
+
+    const int last = n2 - p;                                     // first entry of a half's last plane
+    SplitGemm g{};                                               // W_X = (last block of Linv_X) B_X
+    g.m = g.n = g.k = p;
+    g.lower_a = 1;
+    g.lower_b = -1;                                              // R's rows run down the DOFs: stride -n
+    g.alpha = 1.0;
+    g.a = factor + int64_t(last) * n2 + last; g.ar = n2; g.ac = 1; g.az = h.mat;
+    g.b = A + int64_t(split_dof(s, 0, last)) * s.n + s.sep; g.br = s.n; g.bc = 1;
+    g.bz = int64_t(split_dof(s, 1, last) - split_dof(s, 0, last)) * s.n;
+    g.c = W; g.cr = p; g.cc = 1; g.cz = pp;
+    launch_gemm(g, 2, stream);
+    g = SplitGemm{};                                             // S = A_ss - [W_L; W_R]^T [W_L; W_R]
+    g.m = g.n = p;
+    g.k = 2 * p;
+    g.alpha = -1.0;
+    g.a = W; g.ar = 1; g.ac = p;
+    g.b = W; g.br = p; g.bc = 1;
+    g.d = A + int64_t(s.sep) * s.n + s.sep; g.dr = s.n; g.dc = 1;
+    g.c = S; g.cr = p; g.cc = 1;
+    launch_gemm(g, 1, stream);
+    FactorBatch q{};
+    q.A = S;
+    q.packed = factor + f.ps;
+    q.work = swork;
+    q.info = info + 2;
+    q.mat = pp;
+    q.ws = vx_coarse_factor_workspace(p, p - 1);
+    q.nblk = (p + CB - 1) / CB;
+    vx::launch(band_load_kernel, dim3(unsigned((pp + 255) / 256), 1), 256, 0, stream, p, p - 1, q);
+    launch_chain(p, p - 1, 1, q, stream);
+    launch_inverse(p, p - 1, 1, inverse_warps(p - 1), q, stream);
+    g = SplitGemm{};                                             // G_X = -Linv_s W_X^T
+    g.m = g.n = g.k = p;
+    g.lower_a = 1;
+    g.alpha = -1.0;
+    g.a = factor + f.ps; g.ar = p; g.ac = 1;
+    g.b = W; g.br = 1; g.bc = p; g.bz = pp;
+    g.c = G; g.cr = p; g.cc = 1; g.cz = pp;
+    launch_gemm(g, 2, stream);
+    g = SplitGemm{};                                             // M_X = G_X (last p rows of Linv_X), and M_X^T
+    g.m = g.k = p;
+    g.n = n2;
+    g.lower_b = 1;
+    g.k0b = last;
+    g.alpha = 1.0;
+    g.a = G; g.ar = p; g.ac = 1; g.az = pp;
+    g.b = factor + int64_t(last) * n2; g.br = n2; g.bc = 1; g.bz = h.mat;
+    g.c = factor + f.m; g.cr = n2; g.cc = 1; g.cz = int64_t(p) * n2;
+    g.ct = factor + f.mt; g.ctr = 1; g.ctc = p; g.ctz = int64_t(p) * n2;
+    launch_gemm(g, 2, stream);
+    VX_CHECK_LAUNCH(what);
+    return VX_OK;
+}
+
+extern "C" int vx_split_apply(int prec, int nx, int ny, int nz, const double* factor, const void* r,
+                              const uint8_t* node_mask, double* y, void* z, cudaStream_t stream) {
+    int st = check_grid(nx, ny, nz);
+    if (st) return st;
+    VX_CHECK_ARG(factor && r && y && z, VX_ERR_NULL_POINTER, "vx_split_apply: NULL pointer");
+    SplitShape s;
+    VX_CHECK_ARG(split_shape(nx, ny, nz, &s), VX_ERR_INVALID_ARGUMENT, "vx_split_apply: grid (%d, %d, %d) does not split",
+                 nx, ny, nz);
+    const SplitFactor f = split_factor_layout(s);
+    const unsigned rows = unsigned(2 * s.n2 + s.p);
+    const bool ok = dispatch_prec(prec, [&](auto t) {             // r auxiliary, z an iterate
+        using R = typename decltype(t)::R;
+        using X = typename decltype(t)::X;
+        vx::launch(split_lower_kernel<R>, rows, ST, 0, stream, s, f, factor, (const R*)r, y);
+        vx::launch(split_upper_kernel<X>, rows, ST, 0, stream, s, f, factor, y, node_mask, (X*)z);
+    });
+    VX_CHECK_ARG(ok, VX_ERR_INVALID_ARGUMENT, "vx_split_apply: unsupported precision %d", prec);
+    VX_CHECK_LAUNCH("vx_split_apply");
     return VX_OK;
 }

@@ -132,6 +132,7 @@ class MGHierarchy:
             self.levels.append(L)
         c = self.levels[-1]
         self.blocks = int(coarse_blocks) if coarse_blocks else 0
+        self._split = None
         if self.blocks:
             nxc, nyc, nzc = c.shape
             if (nxc + 1) % self.blocks:
@@ -150,8 +151,17 @@ class MGHierarchy:
             _lib.call("vx_assemble_dense", *c.shape, _lib.dptr(np.ascontiguousarray(self.ke * 2 ** (len(self.shapes) - 1))),
                       _ptr(c.E64, "E"), _ptr(c.mask, "mask"), A.data_ptr(), _s())
             self.A_coarse = A
-            self.coarse_packed = torch.empty_like(A)              # tril(L^-1) + triu(L^-T, 1)
-            self._coarse_y = torch.zeros(c.n, dtype=torch.float64, device="cuda")
+            # The coarsest planes split at the middle one where that is possible (half the factor's chain, 0.56
+            # of the bytes of a solve); small grids keep the one band (small_grid_stream)
+            size = 0 if small_grid_stream(self.shapes[0]) else int(_lib.load().vx_split_factor_size(*c.shape))
+            f64 = dict(dtype=torch.float64, device="cuda")
+            if size:
+                self._split = torch.empty(size, **f64)
+                self._factor_work = torch.empty(int(_lib.load().vx_split_workspace(*c.shape)), **f64)
+                self._factor_info = torch.zeros(3, dtype=torch.int32, device="cuda")
+            else:
+                self.coarse_packed = torch.empty_like(A)          # tril(L^-1) + triu(L^-T, 1)
+            self._coarse_y = torch.zeros(c.n + (c.n // (c.shape[0] + 1) if size else 0), **f64)
         # the same calls as update_modulus, so a refreshed pooled hierarchy and a fresh one are
         # bitwise identical; the factorisation is checked once here (the check synchronises)
         info = self._coarse_inverse()
@@ -265,6 +275,10 @@ class MGHierarchy:
             return self._factor_info
         n = self.A_coarse.shape[0]
         nx, ny, nz = self.levels[-1].shape
+        if self._split is not None:
+            _lib.call("vx_split_factor", nx, ny, nz, self.A_coarse.data_ptr(), self._split.data_ptr(),
+                      self._factor_work.data_ptr(), self._factor_info.data_ptr(), _s())
+            return self._factor_info
         bw = min(n - 1, 3 * ((ny + 1) * (nz + 1) + (nz + 1) + 1) + 2)
         if getattr(self, "_factor_work", None) is None:
             need = int(_lib.load().vx_coarse_factor_workspace(n, bw))
@@ -289,7 +303,8 @@ class MGHierarchy:
                 b += 0 if t is None else t.numel() * t.element_size()
             b += L.E64.numel() * 8 + L.mask.numel()
         work = getattr(self, "_factor_work", None)
-        return b + self.coarse_packed.numel() * 8 * 2 + (0 if work is None else work.numel() * 8)   # A, packed, band
+        factor = self.coarse_packed if self._split is None else self._split
+        return b + (self.A_coarse.numel() + factor.numel() + (0 if work is None else work.numel())) * 8
 
     def spectral_omegas(self, iterations=30, seed=20260923):
         """omega_l = 4 / (3 lambda_l), lambda_l from a seeded FP64 power iteration on D^-1 A over the
@@ -371,6 +386,9 @@ class MGHierarchy:
             nb_ = self.A_coarse.shape[1]
             _lib.call("vx_batch_coarse_apply_factor", self.prec, nb_, self.blocks, nb_, self.coarse_packed.data_ptr(),
                       r.data_ptr(), L.mask.data_ptr(), self._coarse_y.data_ptr(), L.x.data_ptr(), _s())
+        elif self._split is not None:
+            _lib.call("vx_split_apply", self.prec, *L.shape, self._split.data_ptr(), r.data_ptr(), L.mask.data_ptr(),
+                      self._coarse_y.data_ptr(), L.x.data_ptr(), _s())
         else:
             _lib.call("vx_coarse_apply_factor", self.prec, L.n, self.coarse_packed.data_ptr(), r.data_ptr(),
                       L.mask.data_ptr(), self._coarse_y.data_ptr(), L.x.data_ptr(), _s())
