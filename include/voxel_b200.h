@@ -233,6 +233,11 @@ int vx_oc_probe(int64_t n, const double* x, const double* dc, const double* dv, 
 int vx_oc_finalize(int64_t n, const double* partials, double* S, cudaStream_t stream);
 int vx_oc_apply(int64_t n, const double* x, const double* dc, const double* dv, double move, const double* S,
                 double* x_new, cudaStream_t stream);
+/* The probe in one launch: ratio = -dc / dv (vx_oc_ratio, once per update), and the CTA that arrives last does
+ * vx_oc_finalize's step.  *counter (device, 4 bytes) is 0 before and after.  The same bits as vx_oc_probe. */
+int vx_oc_ratio(int64_t n, const double* dc, const double* dv, double* ratio, cudaStream_t stream);
+int vx_oc_probe_fin(int64_t n, const double* x, const double* ratio, const double* w, double move, double* S,
+                    double* partials, unsigned* counter, cudaStream_t stream);
 
 /* Operator forms fused with the outer Krylov loop (FP64/FP32, author layout, node mask optional):
  *   vx_apply_dot:     q = A p and partials[cta] = sum p.q over the CTA's owned nodes

@@ -109,6 +109,8 @@ SIGNATURES = {
     "vx_cone_filter": (c_int, [c_int, c_int, c_int, c_double, _P, _P, c_int, _P, _P]),
     "vx_oc_partials": (c_int64, [c_int64]),
     "vx_oc_probe": (c_int, [c_int64, _P, _P, _P, _P, c_double, _P, _P, _P]),
+    "vx_oc_ratio": (c_int, [c_int64, _P, _P, _P, _P]),
+    "vx_oc_probe_fin": (c_int, [c_int64, _P, _P, _P, c_double, _P, _P, _P, _P]),
     "vx_oc_finalize": (c_int, [c_int64, _P, _P, _P]),
     "vx_oc_apply": (c_int, [c_int64, _P, _P, _P, c_double, _P, _P, _P]),
     # x-slab decomposition

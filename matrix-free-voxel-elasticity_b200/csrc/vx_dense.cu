@@ -361,38 +361,33 @@ __global__ void __launch_bounds__(UPDATE_T) band_update_kernel(int n, int bw, in
         #pragma unroll
         for (int b = 0; b < 4; ++b) { oi[a][b] = 0.0; oj[a][b] = 0.0; }
     }
-    if (same) {
+    // (X is lower triangular: column block b of the panel takes p < 16 (b + 1) only; the skipped terms are zero)
+    auto panel = [&](auto b0c) {
+        constexpr int B0 = decltype(b0c)::value;
         #pragma unroll 4
-        for (int p = 0; p < CB; ++p) {
-            double ai[2], x[4];
-            #pragma unroll
-            for (int a = 0; a < 2; ++a) ai[a] = PI[tr + 16 * a][p];
-            #pragma unroll
-            for (int b = 0; b < 4; ++b) x[b] = Xi[tc + 16 * b][p];
-            #pragma unroll
-            for (int a = 0; a < 2; ++a) {
-                #pragma unroll
-                for (int b = 0; b < 4; ++b) oi[a][b] = fma(ai[a], x[b], oi[a][b]);
-            }
-        }
-    } else {
-        #pragma unroll 4
-        for (int p = 0; p < CB; ++p) {
+        for (int p = 16 * B0; p < 16 * B0 + 16; ++p) {
             double ai[2], aj[2], x[4];
             #pragma unroll
-            for (int a = 0; a < 2; ++a) { ai[a] = PI[tr + 16 * a][p]; aj[a] = PJ[tr + 16 * a][p]; }
+            for (int a = 0; a < 2; ++a) {
+                ai[a] = PI[tr + 16 * a][p];
+                aj[a] = same ? 0.0 : PJ[tr + 16 * a][p];
+            }
             #pragma unroll
-            for (int b = 0; b < 4; ++b) x[b] = Xi[tc + 16 * b][p];
+            for (int b = B0; b < 4; ++b) x[b] = Xi[tc + 16 * b][p];
             #pragma unroll
             for (int a = 0; a < 2; ++a) {
                 #pragma unroll
-                for (int b = 0; b < 4; ++b) {
+                for (int b = B0; b < 4; ++b) {
                     oi[a][b] = fma(ai[a], x[b], oi[a][b]);
-                    oj[a][b] = fma(aj[a], x[b], oj[a][b]);
+                    if (!same) oj[a][b] = fma(aj[a], x[b], oj[a][b]);
                 }
             }
         }
-    }
+    };
+    panel(std::integral_constant<int, 0>{});
+    panel(std::integral_constant<int, 1>{});
+    panel(std::integral_constant<int, 2>{});
+    panel(std::integral_constant<int, 3>{});
     __syncthreads();
     #pragma unroll
     for (int a = 0; a < 2; ++a) {
@@ -869,8 +864,8 @@ extern "C" int vx_coarse_pack_factor(int n, int bw, const double* L, double* pac
 //     M_X = -Linv_s W_X^T [Linv_X's last p rows]
 // the inverse factor is [Linv_L; Linv_R; M_L M_R Linv_s]: half the chain of dependent block factorisations
 // (34 + 4 blocks of 64 instead of 65 for 17 planes of 243) and 0.56 of the bytes of the dense triangles, which
-// then stay in L2.  Factor, and a solve (one band -> split): n = 4131 2.61 -> 1.58 ms, 36 -> 21 us; n = 5700 4.12 ->
-// 2.57 ms, 63 -> 40 us; n = 1911 1.11 -> 0.73 ms, 17 -> 10 us.
+// then stay in L2.  Factor, and a solve (one band -> split): n = 4131 2.61 -> 1.49 ms, 36 -> 21 us; n = 5700 4.12 ->
+// 2.48 ms, 63 -> 40 us; n = 1911 1.11 -> 0.65 ms, 17 -> 10 us.
 namespace vx {
 
 struct SplitShape {
@@ -905,7 +900,9 @@ __global__ void split_load_kernel(SplitShape s, const double* __restrict__ A, co
 
 // C = alpha op(A) op(B) + D for m x n results and depth k, elements by row and column strides; lower_a / lower_b:
 // entries of A right of its diagonal, of B right of column k0b + row, count as zero.  blockIdx.z adds the z
-// offsets.  64 x 64 tiles, a 4 x 4 register tile a thread; a few us each, none of them is worth more.
+// offsets.  The products sit on the factor's chain and most have only p x p results, so tiles are small (32 x 32,
+// 64 CTAs for p = 243) and the next 32 of the depth are in flight during a step (64 x 64 tiles without: four
+// products 200 -> 110 us, n = 4131).
 struct SplitGemm {
     int m, n, k, lower_a, lower_b, k0b;
     double alpha;
@@ -913,42 +910,53 @@ struct SplitGemm {
     double *c, *ct;
     int64_t ar, ac, az, br, bc, bz, dr, dc, cr, cc, cz, ctr, ctc, ctz;
 };
+constexpr int GT = 32;
 __global__ void __launch_bounds__(256) split_gemm_kernel(const __grid_constant__ SplitGemm g) {
     vx::pdl_begin();
-    __shared__ double As[16][65], Bs[16][65];
-    const int t = threadIdx.x, i0 = blockIdx.y * 64, j0 = blockIdx.x * 64, tr = t / 16, tc = t % 16;
+    __shared__ double As[GT][GT + 1], Bs[GT][GT + 1];
+    const int t = threadIdx.x, i0 = blockIdx.y * GT, j0 = blockIdx.x * GT, tr = t / 16, tc = t % 16;
     const double* a = g.a + g.az * blockIdx.z;
     const double* b = g.b + (blockIdx.z ? g.bz : 0);
     const int64_t br = blockIdx.z && g.lower_b < 0 ? -g.br : g.br;
-    double acc[4][4] = {};
-    for (int k0 = 0; k0 < g.k; k0 += 16) {
+    // stage slots of this thread: the faster index runs along the unit stride
+    const int u0 = t % GT, u1 = t / GT;                          // + 8 per slot
+    const bool a_row = g.ac == 1, b_col = g.bc == 1;
+    double ra[4], rb[4];
+    auto load = [&](int k0) {
         #pragma unroll
         for (int u = 0; u < 4; ++u) {
-            const int q = t + 256 * u;
-            // the faster index of the stage runs along the unit stride
-            const int ka = g.ac == 1 ? q % 16 : q / 64, ia = g.ac == 1 ? q / 16 : q % 64;
-            const int kb = g.br == 1 ? q % 16 : q / 64, jb = g.br == 1 ? q / 16 : q % 64;
-            const int i = i0 + ia, j = j0 + jb, k1 = k0 + ka, k2 = k0 + kb;
-            As[ka][ia] = i < g.m && k1 < g.k && !(g.lower_a && k1 > i) ? a[i * g.ar + k1 * g.ac] : 0.0;
-            Bs[kb][jb] = j < g.n && k2 < g.k && !(g.lower_b > 0 && j > g.k0b + k2) ? b[k2 * br + j * g.bc] : 0.0;
+            const int v = u1 + 8 * u;
+            const int ka = k0 + (a_row ? u0 : v), i = i0 + (a_row ? v : u0);
+            const int kb = k0 + (b_col ? v : u0), j = j0 + (b_col ? u0 : v);
+            ra[u] = i < g.m && ka < g.k && !(g.lower_a && ka > i) ? a[i * g.ar + ka * g.ac] : 0.0;
+            rb[u] = j < g.n && kb < g.k && !(g.lower_b > 0 && j > g.k0b + kb) ? b[kb * br + j * g.bc] : 0.0;
+        }
+    };
+    double acc[2][2] = {};
+    load(0);
+    for (int k0 = 0; k0 < g.k; k0 += GT) {
+        #pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const int v = u1 + 8 * u;
+            As[a_row ? u0 : v][a_row ? v : u0] = ra[u];
+            Bs[b_col ? v : u0][b_col ? u0 : v] = rb[u];
         }
         __syncthreads();
-        #pragma unroll
-        for (int k = 0; k < 16; ++k) {
-            double av[4], bv[4];
-            #pragma unroll
-            for (int x = 0; x < 4; ++x) { av[x] = As[k][tr + 16 * x]; bv[x] = Bs[k][tc + 16 * x]; }
-            #pragma unroll
-            for (int x = 0; x < 4; ++x)
-                #pragma unroll
-                for (int y = 0; y < 4; ++y) acc[x][y] = fma(av[x], bv[y], acc[x][y]);
+        if (k0 + GT < g.k) load(k0 + GT);
+        #pragma unroll 8
+        for (int k = 0; k < GT; ++k) {
+            const double a0 = As[k][tr], a1 = As[k][tr + 16], b0 = Bs[k][tc], b1 = Bs[k][tc + 16];
+            acc[0][0] = fma(a0, b0, acc[0][0]);
+            acc[0][1] = fma(a0, b1, acc[0][1]);
+            acc[1][0] = fma(a1, b0, acc[1][0]);
+            acc[1][1] = fma(a1, b1, acc[1][1]);
         }
         __syncthreads();
     }
     #pragma unroll
-    for (int x = 0; x < 4; ++x)
+    for (int x = 0; x < 2; ++x)
         #pragma unroll
-        for (int y = 0; y < 4; ++y) {
+        for (int y = 0; y < 2; ++y) {
             const int i = i0 + tr + 16 * x, j = j0 + tc + 16 * y;
             if (i >= g.m || j >= g.n) continue;
             double v = g.alpha * acc[x][y];
@@ -958,7 +966,7 @@ __global__ void __launch_bounds__(256) split_gemm_kernel(const __grid_constant__
         }
 }
 static void launch_gemm(const SplitGemm& g, int z, cudaStream_t stream) {
-    vx::launch(split_gemm_kernel, dim3(unsigned((g.n + 63) / 64), unsigned((g.m + 63) / 64), unsigned(z)), 256, 0, stream, g);
+    vx::launch(split_gemm_kernel, dim3(unsigned((g.n + GT - 1) / GT), unsigned((g.m + GT - 1) / GT), unsigned(z)), 256, 0, stream, g);
 }
 
 // factor: [packed_L][packed_R] (n2 x n2), [packed_s] (p x p), [M_L][M_R] (p x n2), [M_L^T][M_R^T] (n2 x p)

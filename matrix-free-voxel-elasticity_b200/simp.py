@@ -21,6 +21,7 @@ from .solver import _GraphLoop
 
 OC_L1, OC_L2, OC_LMID, OC_VOL, OC_VOLFRAC, OC_TOL, OC_NEL = range(7)
 OC_DONE, OC_IT, OC_MAXIT, OC_BREAK, OC_CHECK = 10, 11, 12, 14, 15
+OC_PROBES = 8          # bisection probes per turn of the WHILE graph
 
 
 class ConeFilter:
@@ -91,16 +92,23 @@ class OCUpdater:
         self.dc = torch.zeros(n, dtype=torch.float64, device="cuda")
         self.dv = torch.zeros(n, dtype=torch.float64, device="cuda")
         self.x_new = torch.zeros(n, dtype=torch.float64, device="cuda")
+        self.ratio = torch.zeros(n, dtype=torch.float64, device="cuda")        # -dc / dv
+        self.counter = torch.zeros(1, dtype=torch.int32, device="cuda")
         self.move = None
         self.stream = torch.cuda.Stream()
         self.use_graph = graph
         self._graph = None
         self.probes = 0
 
+    def _probe(self):
+        _lib.call("vx_oc_probe_fin", self.n, self.x.data_ptr(), self.ratio.data_ptr(), self.w.data_ptr(), self.move,
+                  self.S.data_ptr(), self.partials.data_ptr(), self.counter.data_ptr(), stream_ptr())
+
     def _body(self):
-        _lib.call("vx_oc_probe", self.n, self.x.data_ptr(), self.dc.data_ptr(), self.dv.data_ptr(), self.w.data_ptr(),
-                  self.move, self.S.data_ptr(), self.partials.data_ptr(), stream_ptr())
-        _lib.call("vx_oc_finalize", self.n, self.partials.data_ptr(), self.S.data_ptr(), stream_ptr())
+        # several probes a turn of the WHILE graph (a turn costs about as much as a probe); past the end of
+        # the bisection a probe does nothing
+        for _ in range(OC_PROBES):
+            self._probe()
 
     def __call__(self, x, dc, dv, volfrac, move, tol=1e-3, l2=1e9, max_probes=400):
         """x_new of oc_top88(x, dc, dv, volfrac, move, density=filter.forward, l2, tol)."""
@@ -113,21 +121,22 @@ class OCUpdater:
             self.x.copy_(x)
             self.dc.copy_(dc)
             self.dv.copy_(dv)
+            _lib.call("vx_oc_ratio", self.n, self.dc.data_ptr(), self.dv.data_ptr(), self.ratio.data_ptr(), stream_ptr())
         if self.use_graph and self._graph is None:
             self._graph = _GraphLoop(self.stream, self.S, self._body)
         with torch.cuda.stream(self.stream):
             init = torch.zeros(16, dtype=torch.float64)
             init[OC_L1], init[OC_L2], init[OC_VOLFRAC], init[OC_TOL] = 0.0, float(l2), float(volfrac), float(tol)
-            init[OC_NEL], init[OC_MAXIT], init[OC_CHECK] = float(self.n), float(max_probes), 1.0
+            init[OC_NEL], init[OC_MAXIT], init[OC_CHECK] = float(self.n), float(max_probes), float(OC_PROBES)
             self.S.copy_(init, non_blocking=False)
-            if self.use_graph:
+            graph = self.use_graph and max_probes >= OC_PROBES
+            if graph:
                 self._graph.launch(self.stream)
-            else:
-                for _ in range(max_probes):
-                    self._body()
+            if not graph or max_probes % OC_PROBES:            # probes past the last whole body
+                self.S_host.copy_(self.S)
+                while not self.S_host[OC_DONE] and self.S_host[OC_IT] < max_probes:
+                    self._probe()
                     self.S_host.copy_(self.S)
-                    if self.S_host[OC_DONE]:
-                        break
             _lib.call("vx_oc_apply", self.n, self.x.data_ptr(), self.dc.data_ptr(), self.dv.data_ptr(), self.move,
                       self.S.data_ptr(), self.x_new.data_ptr(), stream_ptr())
             self.S_host.copy_(self.S, non_blocking=True)
@@ -135,7 +144,7 @@ class OCUpdater:
         caller.wait_stream(self.stream)
         self.probes = int(self.S_host[OC_IT])
         if self.use_graph:
-            self._graph.account(self.probes)
+            self._graph.account(-(-self.probes // OC_PROBES))
         if not self.S_host[OC_DONE]:
             raise RuntimeError(f"OC bisection did not reach tol {tol} in {max_probes} probes")
         return self.x_new.clone()
