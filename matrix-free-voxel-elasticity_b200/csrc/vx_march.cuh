@@ -8,9 +8,9 @@
 // way back.  Per element that is half the shuffles' and half the shared-memory traffic of the order
 // x, y, z (parity_stream_xp: 6 through shared memory, 12 by shuffles each way).
 //
-// A thread owns one z column of one node row in FP64, and of two node rows NW apart in FP32, whose values
-// travel as packed f32x2 pairs that are never taken apart: only the warps at the seam between the two
-// halves swap a half when they read a neighbour row.  Rows 0 and NROW-1 and lanes 0 and 31 are halo.
+// A thread owns one z column of one node row in FP64, and of two node rows half a tile apart in FP32, whose
+// values travel as packed f32x2 pairs that are never taken apart: only the rows at the seam between the two
+// halves swap a half when they read a neighbour row.  A tile's outer rows and columns are halo.
 //
 // The parity blocks couple the x, y and z components of one (py, pz) class only with their own px = 0, 1
 // values, so each class is finished before the next one starts: six block inputs are live, not 24.
@@ -22,10 +22,10 @@
 // What bounds it: the FP64 forms the double-precision pipe (133 of about 270 issued instructions an element
 // row, half busy) together with the latency between its barriers, the FP32 sweep HBM, issue and registers.
 // Eight warps and two CTAs an SM (128 registers) let one CTA compute while the other waits at its barrier;
-// measured at 576x288x288 (us, matvec FP64 / FP32, Jacobi FP64 / FP32) with one step loop and nine constants
-// more: 2 x 8 warps 1053 / 513 / 1193 / 606, 1 x 12 warps 1137 / 562 / 1242 / 685, 1 x 16 warps 1193 / 550 /
-// 1250 / 610, named barriers between neighbouring rows 1102 / 551 (matvecs); as it is now 1017 / 483 / 1149 /
-// 606 (2.7, 3.3, 3.9 and 4.2 TB/s).  parity_stream_xp: 1405 / 638 / 1615 / 732.
+// measured at 576x288x288 (us, matvec FP64 / FP32, Jacobi FP64 / FP32) before the changes noted below: 2 x 8
+// warps 1053 / 513 / 1193 / 606, 1 x 12 warps 1137 / 562 / 1242 / 685, 1 x 16 warps 1193 / 550 / 1250 / 610, named
+// barriers between neighbouring rows 1102 / 551 (matvecs).  As it is now: 898 / 484 / 1131 / 606 (3.1, 3.3, 4.0
+// and 4.2 TB/s); parity_stream_xp: 1405 / 638 / 1615 / 732.
 #pragma once
 
 namespace vx {
@@ -38,8 +38,17 @@ __device__ __forceinline__ V1 mul2(V1 a, V1 b) { return {a.x * b.x}; }
 __device__ __forceinline__ V1 fma2(V1 a, V1 b, V1 c) { return {fma(a.x, b.x, c.x)}; }
 __device__ __forceinline__ V1 cmul2(double c, V1 a) { return {c * a.x}; }
 __device__ __forceinline__ V1 cfma2(double c, V1 a, V1 acc) { return {fma(c, a.x, acc.x)}; }
-__device__ __forceinline__ V1 shfl_down2(V1 a, int d) { return {__shfl_down_sync(0xffffffffu, a.x, d)}; }
-__device__ __forceinline__ V1 shfl_up2(V1 a, int d) { return {__shfl_up_sync(0xffffffffu, a.x, d)}; }
+// exchange with the next / previous lane of a row of LZ lanes (its last / first lane keeps its own value)
+template <int LZ> __device__ __forceinline__ V1 next_lane(V1 a) { return {__shfl_down_sync(0xffffffffu, a.x, 1, LZ)}; }
+template <int LZ> __device__ __forceinline__ V1 prev_lane(V1 a) { return {__shfl_up_sync(0xffffffffu, a.x, 1, LZ)}; }
+template <int LZ> __device__ __forceinline__ V2<float> next_lane(V2<float> a) {
+    const unsigned long long b = __shfl_down_sync(0xffffffffu, *reinterpret_cast<const unsigned long long*>(&a.v), 1, LZ);
+    return {*reinterpret_cast<const float2*>(&b)};
+}
+template <int LZ> __device__ __forceinline__ V2<float> prev_lane(V2<float> a) {
+    const unsigned long long b = __shfl_up_sync(0xffffffffu, *reinterpret_cast<const unsigned long long*>(&a.v), 1, LZ);
+    return {*reinterpret_cast<const float2*>(&b)};
+}
 
 template <typename TC, int N> struct MarchPack;
 template <typename TC> struct MarchPack<TC, 1> {
@@ -53,9 +62,14 @@ template <typename TC> struct MarchPack<TC, 2> {
     __device__ static __forceinline__ TC get(P p, int c) { return c ? p.hi() : p.lo(); }
 };
 template <typename TC> struct March;
-template <> struct March<double> : MarchPack<double, 1> { static constexpr int N = 1, NW = 8, MINB = 2; };
-template <> struct March<float> : MarchPack<float, 2> { static constexpr int N = 2, NW = 8, MINB = 2; };
-template <typename TC> constexpr int march_rows() { return March<TC>::N * March<TC>::NW; }
+// Lanes per node row.  A row of 32 lanes owns 30 columns; in FP64, where a CTA has only eight warps of single
+// rows, rows of 16 lanes (two a warp) make the tile 14 x 14 of 16 x 16 nodes instead of 6 x 30 of 8 x 32: 77%
+// of the lanes own a node instead of 70%, and the node counts 2^k + 1 waste less of the last tile (128x64x64
+// 21.5 -> 16.1 us, 192x96x96 57 -> 38, 576x288x288 1017 -> 898; rows of 8 lanes 23.5, 62, 1068).  The FP32 tile
+// is 14 x 30 of 16 x 32 either way round; 32 lanes coalesce better (484 us against 508).
+template <> struct March<double> : MarchPack<double, 1> { static constexpr int N = 1, NW = 8, MINB = 2, LZ = 16; };
+template <> struct March<float> : MarchPack<float, 2> { static constexpr int N = 2, NW = 8, MINB = 2, LZ = 32; };
+template <typename TC> constexpr int march_rows() { return March<TC>::N * March<TC>::NW * 32 / March<TC>::LZ; }
 template <typename TC> constexpr size_t march_smem() { return size_t(5) * 3 * March<TC>::NW * 32 * sizeof(typename March<TC>::P); }
 
 // The block products of class (py, pz): s[c], d[c] are the px = 0 and px = 1 inputs of component c (at the
@@ -130,21 +144,21 @@ parity_march(const __grid_constant__ OpArgs2<TC, TU, TE, TY, TR> args) {
     vx::pdl_begin();
     using C = March<TC>;
     using P = typename C::P;
-    constexpr int N = C::N, NWS = C::NW, OWN = N * NWS - 2;
+    constexpr int N = C::N, LZ = C::LZ, ROWS = C::NW * 32 / LZ, OWN = N * ROWS - 2, OWNZ = LZ - 2;
     constexpr bool HAS_R = EPI == EPI_JACOBI || EPI == EPI_RESIDUAL || EPI == EPI_TRUE_RES;
     constexpr bool HAS_D = EPI == EPI_JACOBI;
     // does the epilogue read the operand at the output node?
     constexpr bool USES_X = EPI == EPI_JACOBI || EPI == EPI_APPLY_DOT;
-    // The FP32 forms with the most epilogue operands have no registers left: they keep one step loop.  The others
-    // run the planes inside the grid in a loop without tests (FP32 matvec 513 -> 483 us, FP64 true residual 1147 ->
-    // 1067 at 576x288x288; in the FP32 sweep that loop spills, 603 -> 701), and in FP32 test a warp's masks by a
-    // vote (in FP64 the vote costs 3%).
-    constexpr bool LEAN = N == 2 && (EPI == EPI_JACOBI || EPI == EPI_TRUE_RES), VOTE = N == 2 && !LEAN;
+    // Most forms run the planes inside the grid in a loop without tests (FP32 matvec 513 -> 483 us at
+    // 576x288x288) and, in FP32, test a warp's masks by a vote.  The forms that have no registers left for a
+    // second step loop keep one (FP32 sweep 603 us, with it 701; FP64 apply 976, with it 1000).
+    constexpr bool LEAN = N == 2 ? EPI == EPI_JACOBI || EPI == EPI_TRUE_RES : EPI == EPI_APPLY_DOT;
+    constexpr bool VOTE = N == 2 && !LEAN;
     const auto& a = args.a;
-    const int lane = threadIdx.x & 31;
-    const int row = threadIdx.x >> 5;
+    const int lane = threadIdx.x % LZ;                       // node column of the row
+    const int row = threadIdx.x / LZ;
     const Grid g = a.g;
-    const int iz = blockIdx.x * TZ - 1 + lane;
+    const int iz = blockIdx.x * OWNZ - 1 + lane;
     const int x0 = blockIdx.z * a.cx;
     const int x1 = min(x0 + a.cx, g.nx + 1);                 // owned node planes [x0, x1)
     const int plane_nodes = (g.ny + 1) * (g.nz + 1);
@@ -158,22 +172,22 @@ parity_march(const __grid_constant__ OpArgs2<TC, TU, TE, TY, TR> args) {
     const int pl0 = max(x0 - 1, 0);
     #pragma unroll
     for (int c = 0; c < N; ++c) {
-        const int rr = row + c * NWS, iy = blockIdx.y * OWN - 1 + rr;
-        owner[c] = iy >= 0 && iy <= g.ny && iz >= 0 && iz <= g.nz && lane >= 1 && lane <= TZ && rr >= 1 && rr <= OWN;
-        elem_ok[c] = iy >= 0 && iy < g.ny && iz >= 0 && iz < g.nz && lane < 31 && rr < N * NWS - 1;
+        const int rr = row + c * ROWS, iy = blockIdx.y * OWN - 1 + rr;
+        owner[c] = iy >= 0 && iy <= g.ny && iz >= 0 && iz <= g.nz && lane >= 1 && lane <= OWNZ && rr >= 1 && rr <= OWN;
+        elem_ok[c] = iy >= 0 && iy < g.ny && iz >= 0 && iz < g.nz && lane < LZ - 1 && rr < N * ROWS - 1;
         const int cn = min(max(iy, 0), g.ny) * (g.nz + 1) + min(max(iz, 0), g.nz);
         n_in[c] = pl0 * plane_nodes + cn;
         n_out[c] = (x0 - 1) * plane_nodes + cn;              // plane x0 - 1 is never stored
         e_in[c] = (x0 - 1) * plane_elems + min(max(iy, 0), g.ny - 1) * g.nz + min(max(iz, 0), g.nz - 1);
     }
-    const bool compute = N == 2 || row < NWS - 1;            // warp-uniform
+    const bool compute = N == 2 || LZ < 32 || row < ROWS - 1;    // warp-uniform
 
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    P* const us = reinterpret_cast<P*>(smem_raw);            // operand ring: 3 planes x NWS rows x 3 x 32
-    P* const hs = us + 3 * NWS * 96;                         // inverse-y contributions: 2 planes
-    const int own_at = row * 96 + lane;
-    const int up_at = (row + 1 < NWS ? row + 1 : (N == 2 ? 0 : row)) * 96 + lane;
-    const int dn_at = (row > 0 ? row - 1 : (N == 2 ? NWS - 1 : 0)) * 96 + lane;
+    P* const us = reinterpret_cast<P*>(smem_raw);            // operand ring: 3 planes x ROWS x 3 x LZ
+    P* const hs = us + 3 * ROWS * 3 * LZ;                         // inverse-y contributions: 2 planes
+    const int own_at = row * 3 * LZ + lane;
+    const int up_at = (row + 1 < ROWS ? row + 1 : (N == 2 ? 0 : row)) * 3 * LZ + lane;
+    const int dn_at = (row > 0 ? row - 1 : (N == 2 ? ROWS - 1 : 0)) * 3 * LZ + lane;
 
     typename Storage<TU>::raw_t ur[N][3];                    // operand of the plane in flight
     uint8_t um[N];
@@ -218,22 +232,22 @@ parity_march(const __grid_constant__ OpArgs2<TC, TU, TE, TY, TR> args) {
             }
         }
         #pragma unroll
-        for (int k = 0; k < 3; ++k) us[at + own_at + 32 * k] = C::make(v[k]);
+        for (int k = 0; k < 3; ++k) us[at + own_at + LZ * k] = C::make(v[k]);
         return bits;
     };
     // y stage of a ring plane: ya[c][py] at this row's face
     auto y_stage = [&](int at, P (&ya)[3][2]) {
         #pragma unroll
         for (int k = 0; k < 3; ++k) {
-            const P o = us[at + own_at + 32 * k];
-            P n = us[at + up_at + 32 * k];
-            if constexpr (N == 2) { if (row == NWS - 1) n = mk2(n.hi(), n.hi()); }   // row NWS is the other half's row 0
+            const P o = us[at + own_at + LZ * k];
+            P n = us[at + up_at + LZ * k];
+            if constexpr (N == 2) { if (row == ROWS - 1) n = mk2(n.hi(), n.hi()); }   // row ROWS is the other half's row 0
             ya[k][0] = add2(o, n);
             ya[k][1] = sub2(o, n);
         }
     };
 
-    constexpr int RING = NWS * 96;
+    constexpr int RING = ROWS * 3 * LZ;
     P pp[3][2][2];                                           // y-z transformed operand of node plane e
     P gg[3][2][2];                                           // element plane e-1's contributions to node plane e
     unsigned bits0, bits1, bits2 = 0;                        // mask bits of node planes e, e+1, e+2
@@ -251,7 +265,7 @@ parity_march(const __grid_constant__ OpArgs2<TC, TU, TE, TY, TR> args) {
         for (int k = 0; k < 3; ++k)
             #pragma unroll
             for (int py = 0; py < 2; ++py) {
-                const P yb = shfl_down2(ya[k][py], 1);
+                const P yb = next_lane<LZ>(ya[k][py]);
                 pp[k][py][0] = add2(ya[k][py], yb);
                 pp[k][py][1] = sub2(ya[k][py], yb);
                 const TC z[2] = {TC(0), TC(0)};
@@ -296,7 +310,7 @@ parity_march(const __grid_constant__ OpArgs2<TC, TU, TE, TY, TR> args) {
             #pragma unroll
             for (int k = 0; k < 3; ++k)
                 #pragma unroll
-                for (int py = 0; py < 2; ++py) yb[k][py] = shfl_down2(ya[k][py], 1);
+                for (int py = 0; py < 2; ++py) yb[k][py] = next_lane<LZ>(ya[k][py]);
             P fx[3][2][2];                                   // totals of node plane e's faces
             auto cls = [&](auto PYc, auto PZc) {
                 constexpr int PY = decltype(PYc)::value, PZ = decltype(PZc)::value;
@@ -336,10 +350,10 @@ parity_march(const __grid_constant__ OpArgs2<TC, TU, TE, TY, TR> args) {
                 #pragma unroll
                 for (int py = 0; py < 2; ++py) {
                     const P f0 = fx[k][py][0], f1 = fx[k][py][1];
-                    fz[py] = add2(add2(f0, f1), shfl_up2(sub2(f0, f1), 1));
+                    fz[py] = add2(add2(f0, f1), prev_lane<LZ>(sub2(f0, f1)));
                 }
                 hown[k] = add2(fz[0], fz[1]);
-                hs[hat + own_at + 32 * k] = sub2(fz[0], fz[1]);
+                hs[hat + own_at + LZ * k] = sub2(fz[0], fz[1]);
             }
         }
         __syncthreads();
@@ -347,14 +361,14 @@ parity_march(const __grid_constant__ OpArgs2<TC, TU, TE, TY, TR> args) {
             P yv[3];
             #pragma unroll
             for (int k = 0; k < 3; ++k) {
-                P h = hs[hat + dn_at + 32 * k];
-                if constexpr (N == 2) { if (row == 0) h = mk2(h.lo(), h.lo()); }     // row NWS gets row NWS - 1's
+                P h = hs[hat + dn_at + LZ * k];
+                if constexpr (N == 2) { if (row == 0) h = mk2(h.lo(), h.lo()); }     // row ROWS gets row ROWS - 1's
                 yv[k] = add2(hown[k], h);
             }
             P xv[3];
             if constexpr (USES_X) {
                 #pragma unroll
-                for (int k = 0; k < 3; ++k) xv[k] = us[at0 + own_at + 32 * k];
+                for (int k = 0; k < 3; ++k) xv[k] = us[at0 + own_at + LZ * k];
             }
             const bool sums = e >= a.dot_x0 && e < a.dot_x1;
             TC xr[N][3], ax[N][3];
@@ -429,9 +443,9 @@ parity_march(const __grid_constant__ OpArgs2<TC, TU, TE, TY, TR> args) {
     for (; e < x1; ++e) step(e, std::false_type{}, std::false_type{});
     if constexpr (EPI == EPI_TRUE_RES || EPI == EPI_APPLY_DOT) {
         const int64_t bid = (int64_t(blockIdx.z) * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;
-        block_sum_store<NWS * 32>(acc, a.partials + bid);
+        block_sum_store<C::NW * 32>(acc, a.partials + bid);
         if (a.counter) {
-            static_assert(NWS * 32 == FT, "the last CTA finishes the reduction with FT threads");
+            static_assert(C::NW * 32 == FT, "the last CTA finishes the reduction with FT threads");
             finalize_last(a.fin, int64_t(gridDim.x) * gridDim.y * gridDim.z, a.partials, a.S, a.counter);
         }
     }

@@ -794,7 +794,7 @@ inline ZpGrid zp_grid_for(const Grid& g) {
 
 template <typename TC>
 dim3 march_grid(const Grid& g, int* cx) {
-    const int tz = (g.nz + 1 + TZ - 1) / TZ, own = march_rows<TC>() - 2, ty = (g.ny + 1 + own - 1) / own;
+    const int ownz = March<TC>::LZ - 2, tz = (g.nz + 1 + ownz - 1) / ownz, own = march_rows<TC>() - 2, ty = (g.ny + 1 + own - 1) / own;
     *cx = march_cx(g, tz * ty, March<TC>::MINB * sm_count());
     return dim3(tz, ty, (g.nx + 1 + *cx - 1) / *cx);
 }
