@@ -79,26 +79,30 @@ template <typename TC, bool CUBIC, int PY, int PZ, typename P, typename Args>
 __device__ __forceinline__ void march_blocks(const Args& args, P (&s)[3], P (&d)[3]) {
     if constexpr (CUBIC) {
         const auto& K = args.M;
+        auto cd = [&](P other, P self) {                     // a row of [c d; d c]
+            if constexpr (MarchK<TC>::SCALED) return cfma2(K.d, other, self);
+            else return cfma2(K.d, other, cmul2(K.c, self));
+        };
         if constexpr (PY == 0 && PZ == 0) {
             const P bs = cmul2(K.b0, add2(add2(d[0], s[1]), s[2]));          // g0: x@1 y@2 z@4
             d[0] = cfma2(K.amb0, d[0], bs);
             s[1] = cfma2(K.amb0, s[1], bs);
             s[2] = cfma2(K.amb0, s[2], bs);
             const P a1 = d[1], a2 = d[2];                                    // g1: y@3 z@5
-            d[1] = cfma2(K.d, a2, a1);
-            d[2] = cfma2(K.d, a1, a2);
+            d[1] = cd(a2, a1);
+            d[2] = cd(a1, a2);
         } else if constexpr (PY == 1 && PZ == 0) {
             const P a0 = d[0], a2 = s[2];                                    // g2: x@3 z@6
-            d[0] = cfma2(K.d, a2, a0);
-            s[2] = cfma2(K.d, a0, a2);
+            d[0] = cd(a2, a0);
+            s[2] = cd(a0, a2);
             const P t = cmul2(K.e, add2(s[0], d[1]));                        // g3: x@2 y@1, z@7
             s[0] = t;
             d[1] = t;
             d[2] = cmul2(K.f, d[2]);
         } else if constexpr (PY == 0 && PZ == 1) {
             const P a0 = d[0], a1 = s[1];                                    // g4: x@5 y@6
-            d[0] = cfma2(K.d, a1, a0);
-            s[1] = cfma2(K.d, a0, a1);
+            d[0] = cd(a1, a0);
+            s[1] = cd(a0, a1);
             const P t = cmul2(K.e, add2(s[0], d[2]));                        // g5: x@4 z@1, y@7
             s[0] = t;
             d[2] = t;
@@ -283,7 +287,7 @@ parity_march(const __grid_constant__ OpArgs2<TC, TU, TE, TY, TR> args) {
         #pragma unroll
         for (int c = 0; c < N; ++c) {
             ev[c] = TC(Storage<TE>::cvt(er[c]));
-            if constexpr (CUBIC) ev[c] *= args.M.scale;
+            if constexpr (CUBIC && MarchK<TC>::SCALED) ev[c] *= args.M.scale;
         }
         if (BULK || e + 2 <= x1) {
             bits2 = put_u(at2);

@@ -320,11 +320,13 @@ template <typename TC> struct CubeK {
     typename Coef<TC>::type amb0, b0, c1, d1, c2, d2, c4, d4, e3, f3, e5, f5, e6, f6, hmk7, k7;
 };
 
-// The same with all edges equal for parity_march: the three axes' blocks agree (g1 = g2 = g4, g3 = g5 = g6), and
-// the modulus is scaled by c so that [c d; d c] becomes [1 d/c; d/c 1].  Seven constants: each one held in the
-// constant bank costs its moves to registers every step.
+// The same for parity_march, whose cube form also needs the three axes' blocks to agree (g1 = g2 = g4, g3 = g5 =
+// g6): each constant held in the constant bank costs its moves to registers every step.  In FP64 the modulus is
+// scaled by c, so that [c d; d c] becomes [1 d/c; d/c 1]: a constant and five multiplications less (apply 1019 ->
+// 947 us at 576x288x288).  FP32 keeps c: the scaled modulus would be rounded once more.
 template <typename TC> struct MarchK {
-    typename Coef<TC>::type amb0, b0, d, e, f, hmk7, k7;
+    static constexpr bool SCALED = std::is_same<TC, double>::value;
+    typename Coef<TC>::type amb0, b0, c, d, e, f, hmk7, k7;
     TC scale;
 };
 
@@ -404,8 +406,9 @@ MarchK<TC> march_constants(const double* c) {
         else return v;
     };
     auto B = [&](int g, int r, int col) { return c[9 * g + 3 * r + col]; };
-    const double s = B(1, 1, 1);
+    const double s = MarchK<TC>::SCALED ? B(1, 1, 1) : 1.0;
     MarchK<TC> M;
+    M.c = k(B(1, 1, 1));
     M.amb0 = k((B(0, 0, 0) - B(0, 0, 1)) / s); M.b0 = k(B(0, 0, 1) / s);
     M.d = k(B(1, 1, 2) / s);
     M.e = k(B(3, 0, 0) / s); M.f = k(B(3, 2, 2) / s);
