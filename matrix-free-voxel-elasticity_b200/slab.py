@@ -32,7 +32,7 @@ from . import _lib
 from .element import quadrature
 from .operators import PREC, STORAGE, VoxelOperator, node_mask_from_dofs, stream_ptr
 from .solver import (FIN_BETA_PR, FIN_NB, FIN_PQ, FIN_RZ, FIN_TRUE, S_BREAK, S_CHECK, S_DONE, S_IT, S_MAXIT,
-                     S_MV, S_REL, S_TOL, SolveResult, _GraphLoop, hierarchy_shapes)
+                     S_MV, S_REL, S_TOL, SolveResult, _GraphLoop, hierarchy_shapes, small_grid_stream)
 
 PLANE_APPLY, PLANE_JACOBI, PLANE_RESIDUAL, PLANE_TRUE_RES = range(4)
 _ARITH = {torch.float64: torch.float64, torch.float32: torch.float32, torch.bfloat16: torch.float32}
@@ -352,19 +352,26 @@ class SlabHierarchy:
         kc = np.ascontiguousarray(self.ke * 2 ** l)
         A = torch.empty(self.nc, self.nc, dtype=torch.float64, device="cuda")
         _lib.call("vx_assemble_dense", *cs, _lib.dptr(kc), Eg.data_ptr(), mg.data_ptr(), A.data_ptr(), _s())
-        # banded Cholesky and the packed inverse factor in the library's own kernels (as MGHierarchy)
-        bw = min(self.nc - 1, 3 * ((cs[1] + 1) * (cs[2] + 1) + (cs[2] + 1) + 1) + 2)
-        work = torch.empty(int(_lib.load().vx_coarse_factor_workspace(self.nc, bw)), dtype=torch.float64, device="cuda")
-        info = torch.zeros(1, dtype=torch.int32, device="cuda")
-        self.coarse_packed = torch.empty_like(A)
-        _lib.call("vx_coarse_factor", self.nc, bw, A.data_ptr(), self.coarse_packed.data_ptr(), work.data_ptr(),
-                  info.data_ptr(), _s())
-        if int(info) != 0:
-            raise ValueError(f"coarsest-level matrix is not positive definite (pivot {int(info)})")
+        # the factor in the library's own kernels, the coarsest planes split where MGHierarchy splits them
+        size = 0 if small_grid_stream(self.shapes[0]) else int(_lib.load().vx_split_factor_size(*cs))
+        info = torch.zeros(3, dtype=torch.int32, device="cuda")
+        self._split = self.coarse_packed = None
+        if size:
+            self._split = torch.empty(size, dtype=torch.float64, device="cuda")
+            work = torch.empty(int(_lib.load().vx_split_workspace(*cs)), dtype=torch.float64, device="cuda")
+            _lib.call("vx_split_factor", *cs, A.data_ptr(), self._split.data_ptr(), work.data_ptr(), info.data_ptr(), _s())
+        else:
+            bw = min(self.nc - 1, 3 * (Pc + (cs[2] + 1) + 1) + 2)
+            work = torch.empty(int(_lib.load().vx_coarse_factor_workspace(self.nc, bw)), dtype=torch.float64, device="cuda")
+            self.coarse_packed = torch.empty_like(A)
+            _lib.call("vx_coarse_factor", self.nc, bw, A.data_ptr(), self.coarse_packed.data_ptr(), work.data_ptr(),
+                      info.data_ptr(), _s())
+        if int(info.abs().max()) != 0:
+            raise ValueError(f"coarsest-level matrix is not positive definite (pivot {info.tolist()})")
         del A, work
         self._rc = torch.zeros(self.nc, dtype=self.aux_dtype, device="cuda")
         self._zc = torch.zeros(self.nc, dtype=self.dtype, device="cuda")
-        self._yc = torch.zeros(self.nc, dtype=torch.float64, device="cuda")
+        self._yc = torch.zeros(self.nc + 3 * Pc, dtype=torch.float64, device="cuda")
 
     def spectral_omegas(self, iterations=30, seed=20260923):
         """omega_l = 4 / (3 lambda_l), lambda_l from the seeded FP64 power iteration on D^-1 A over the
@@ -462,8 +469,12 @@ class SlabHierarchy:
     def _coarse(self):
         l = len(self.shapes) - 1
         self.comm.gather([L.r[:L.n_own] for _, L in self._level(l)], self._rc)
-        _lib.call("vx_coarse_apply_factor", self.prec, self.nc, self.coarse_packed.data_ptr(), self._rc.data_ptr(),
-                  self.coarse_mask.data_ptr(), self._yc.data_ptr(), self._zc.data_ptr(), _s())
+        if self._split is not None:
+            _lib.call("vx_split_apply", self.prec, *self.shapes[l], self._split.data_ptr(), self._rc.data_ptr(),
+                      self.coarse_mask.data_ptr(), self._yc.data_ptr(), self._zc.data_ptr(), _s())
+        else:
+            _lib.call("vx_coarse_apply_factor", self.prec, self.nc, self.coarse_packed.data_ptr(), self._rc.data_ptr(),
+                      self.coarse_mask.data_ptr(), self._yc.data_ptr(), self._zc.data_ptr(), _s())
         for _, L in self._level(l):
             lo = 3 * L.a * L.P
             L.x.copy_(self._zc[lo:lo + L.n])
