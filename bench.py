@@ -151,8 +151,8 @@ def build_inputs(name, device="cuda"):
 # DRAM bytes per grid node of one launch, from single-kernel ncu captures of the same kernels on the
 # 256x128x128 grid (4,276,737 nodes): dram__bytes_read.sum + dram__bytes_write.sum / nodes.  Scaled by
 # the node count of the measured launch (the traffic of these streaming kernels grows with the nodes).
-NCU_TRAFFIC_PER_NODE = {"jacobi_sweep_f32": (175.528960e6 + 36.767744e6) / 4276737,
-                        "apply_dot_f64": (140.506880e6 + 71.061504e6) / 4276737}
+NCU_TRAFFIC_PER_NODE = {"jacobi_sweep_f32": (177.938944e6 + 35.143424e6) / 4276737,
+                        "apply_dot_f64": (140.538112e6 + 67.077376e6) / 4276737}
 NCU_TRAFFIC_SOURCE = "ncu dram bytes of the same kernel on 256x128x128, per node, scaled by nodes"
 
 
