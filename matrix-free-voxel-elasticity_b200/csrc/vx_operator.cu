@@ -1370,7 +1370,11 @@ extern "C" int vx_true_residual_noalloc(int prec, int nx, int ny, int nz, const 
                  "vx_true_residual_noalloc: NULL pointer");
     VX_CHECK_ARG(prec == VX_F64 || prec == VX_F32, VX_ERR_INVALID_ARGUMENT,
                  "vx_true_residual_noalloc: unsupported precision %d", prec);
-    const int64_t G = stream_ctas(Grid{nx, ny, nz}, prec);
+    // parity_march's 14 x 14 FP64 tiles are more than parity_stream_xp's 6 x 30 on a grid a few nodes thin
+    // in y and very long in z (28572 against 13334 on 1x5x400000): such a grid still fits by the latter
+    int sel = prec;
+    int64_t G = stream_ctas(Grid{nx, ny, nz}, sel);
+    if (G > NOALLOC_MAX_CTAS) G = stream_ctas(Grid{nx, ny, nz}, sel |= VX_STREAM_XP);
     VX_CHECK_ARG(G <= NOALLOC_MAX_CTAS, VX_ERR_INVALID_ARGUMENT,
                  "vx_true_residual_noalloc: grid (%d, %d, %d) needs %lld partial sums but the built-in scratch "
                  "holds %lld; use vx_true_residual with a caller-provided buffer",
@@ -1379,7 +1383,7 @@ extern "C" int vx_true_residual_noalloc(int prec, int nx, int ny, int nz, const 
     st = noalloc_scratch(&scratch);
     if (st) return st;
     // every CTA overwrites its own slot before the reduction reads it: nothing needs clearing
-    st = fused_dispatch<EPI_TRUE_RES>("vx_true_residual_noalloc", prec, nx, ny, nz, blocks, E, node_mask, x, b,
+    st = fused_dispatch<EPI_TRUE_RES>("vx_true_residual_noalloc", sel, nx, ny, nz, blocks, E, node_mask, x, b,
                                       nullptr, 0.0, res, scratch, stream);
     if (st) return st;
     return vx_reduce_partials(G, 1, scratch, norm2, stream);

@@ -74,3 +74,24 @@ def test_agrees_with_the_other_streaming_kernels(dtype, tol):
     finally:
         _lib.set_stream_kernel(prev)
     assert float((y - ref).abs().max()) <= tol * float(ref.abs().max())
+
+
+def test_noalloc_residual_takes_long_thin_grids():
+    """A grid six nodes thin in y needs more FP64 march tiles than the built-in scratch holds, but fits it
+    by the xp kernel's: accepted, and equal to the residual with a caller's buffer to rounding."""
+    shape = (1, 5, 240000)
+    rng = np.random.default_rng(4)
+    op = vx.VoxelOperator(shape, CUBE, F64)
+    L = _lib.load()
+    assert op.partials_size > 16384 >= L.vx_operator_partials(_lib.VX_F64 | _lib.VX_STREAM_XP, *shape)
+    x, b = (torch.as_tensor(rng.standard_normal(op.ndof), device="cuda") for _ in range(2))
+    E = torch.as_tensor(1e-3 + rng.random(op.n_elem), device="cuda")
+    nm = torch.full((op.nodes,), 7, dtype=torch.uint8, device="cuda")
+    nm[:36] = 0
+    part = torch.empty(op.partials_size, dtype=F64, device="cuda")
+    ref, res, n2 = torch.empty_like(x), torch.empty_like(x), torch.zeros(1, dtype=F64, device="cuda")
+    op.true_residual(x, b, E, nm, ref, part)
+    _lib.call("vx_true_residual_noalloc", op.prec, *shape, op._bp, E.data_ptr(), nm.data_ptr(), x.data_ptr(),
+              b.data_ptr(), res.data_ptr(), n2.data_ptr(), torch.cuda.current_stream().cuda_stream)
+    assert float((res - ref).abs().max()) <= 1e-13 * float(ref.abs().max())
+    assert abs(float(n2) - float(ref @ ref)) <= 1e-12 * float(ref @ ref)
