@@ -24,7 +24,7 @@
 // Eight warps and two CTAs an SM (128 registers) let one CTA compute while the other waits at its barrier;
 // measured at 576x288x288 (us, matvec FP64 / FP32, Jacobi FP64 / FP32) before the changes noted below: 2 x 8
 // warps 1053 / 513 / 1193 / 606, 1 x 12 warps 1137 / 562 / 1242 / 685, 1 x 16 warps 1193 / 550 / 1250 / 610, named
-// barriers between neighbouring rows 1102 / 551 (matvecs).  As it is now: 898 / 484 / 1131 / 606 (3.1, 3.3, 4.0
+// barriers between neighbouring rows 1102 / 551 (matvecs).  As it is now: 960 / 484 / 1081 / 609 (2.9, 3.3, 4.2
 // and 4.2 TB/s); parity_stream_xp: 1405 / 638 / 1615 / 732.
 #pragma once
 
@@ -79,10 +79,7 @@ template <typename TC, bool CUBIC, int PY, int PZ, typename P, typename Args>
 __device__ __forceinline__ void march_blocks(const Args& args, P (&s)[3], P (&d)[3]) {
     if constexpr (CUBIC) {
         const auto& K = args.M;
-        auto cd = [&](P other, P self) {                     // a row of [c d; d c]
-            if constexpr (MarchK<TC>::SCALED) return cfma2(K.d, other, self);
-            else return cfma2(K.d, other, cmul2(K.c, self));
-        };
+        auto cd = [&](P other, P self) { return cfma2(K.d, other, cmul2(K.c, self)); };      // a row of [c d; d c]
         if constexpr (PY == 0 && PZ == 0) {
             const P bs = cmul2(K.b0, add2(add2(d[0], s[1]), s[2]));          // g0: x@1 y@2 z@4
             d[0] = cfma2(K.amb0, d[0], bs);
@@ -158,6 +155,10 @@ parity_march(const __grid_constant__ OpArgs2<TC, TU, TE, TY, TR> args) {
     // second step loop keep one (FP32 sweep 603 us, with it 701; FP64 apply 976, with it 1000).
     constexpr bool LEAN = N == 2 ? EPI == EPI_JACOBI || EPI == EPI_TRUE_RES : EPI == EPI_APPLY_DOT;
     constexpr bool VOTE = N == 2 && !LEAN;
+    // The x stage's E (p +- c) is E p +- E c by multiply-adds, or the sum times E: one FP64 operation more a value, yet
+    // the faster schedule in all FP64 forms but one (576x288x288, multiply-adds -> sums: matvec 1043 -> 960 us, sweep
+    // 1138 -> 1081, true residual 1027 -> 1008, apply 1029 -> 1031, residual 1000 -> 1154; FP32 matvec 483 -> 494).
+    constexpr bool SUM_FIRST = N == 1 && EPI != EPI_RESIDUAL;
     const auto& a = args.a;
     const int lane = threadIdx.x % LZ;                       // node column of the row
     const int row = threadIdx.x / LZ;
@@ -285,10 +286,7 @@ parity_march(const __grid_constant__ OpArgs2<TC, TU, TE, TY, TR> args) {
         constexpr bool FIRST = decltype(first)::value, BULK = decltype(bulk)::value;
         TC ev[N];
         #pragma unroll
-        for (int c = 0; c < N; ++c) {
-            ev[c] = TC(Storage<TE>::cvt(er[c]));
-            if constexpr (CUBIC && MarchK<TC>::SCALED) ev[c] *= args.M.scale;
-        }
+        for (int c = 0; c < N; ++c) ev[c] = TC(Storage<TE>::cvt(er[c]));
         if (BULK || e + 2 <= x1) {
             bits2 = put_u(at2);
             if (BULK || e + 3 <= x1) load_u(e + 3, BULK);
@@ -323,9 +321,15 @@ parity_march(const __grid_constant__ OpArgs2<TC, TU, TE, TY, TR> args) {
                 #pragma unroll
                 for (int k = 0; k < 3; ++k) {
                     const P c0 = pz[k] ? sub2(ya[k][py[k]], yb[k][py[k]]) : add2(ya[k][py[k]], yb[k][py[k]]);
-                    const P m = mul2(E, pp[k][py[k]][pz[k]]);
-                    s[k] = fma2(E, c0, m);
-                    d[k] = fma2(nE, c0, m);
+                    const P p0 = pp[k][py[k]][pz[k]];
+                    if constexpr (SUM_FIRST) {
+                        s[k] = mul2(E, add2(p0, c0));
+                        d[k] = mul2(E, sub2(p0, c0));
+                    } else {
+                        const P m = mul2(E, p0);
+                        s[k] = fma2(E, c0, m);
+                        d[k] = fma2(nE, c0, m);
+                    }
                     pp[k][py[k]][pz[k]] = c0;
                 }
                 march_blocks<TC, CUBIC, PY, PZ>(args, s, d);
