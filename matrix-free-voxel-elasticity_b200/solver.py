@@ -534,9 +534,8 @@ class FCGSolver:
         self.G_vec = int(_lib.load().vx_solver_partials(n))
         steps = int(_lib.load().vx_jacobi_step_partials(n))
         self.partials = torch.empty(max(self.G_op, 2 * self.G_vec, steps), **f64)
-        self._jacobi = type(precond) is JacobiPreconditioner
-        self._small = self._jacobi and n <= int(_lib.load().vx_small_cg_limit())
-        self.step_partials = torch.empty(steps, **f64) if self._small else None
+        self._few = n <= int(_lib.load().vx_small_cg_limit())
+        self.step_partials = torch.empty(steps, **f64)
         self.zprec = PREC[precond.dtype]
         self.stream = torch.cuda.Stream()
         self.use_graph = bool(graph)
@@ -549,6 +548,12 @@ class FCGSolver:
         return 6 * self.n * 8 + self.M.footprint_bytes() + self.E.numel() * 8
 
     # ------------------------------------------------------------------ kernel emission
+    @property
+    def _jacobi(self):
+        """Do the fused Jacobi kernels stand for M.emit?  They keep the previous z in this solver's z_old: M.z is
+        scratch that other solvers with the same M write too."""
+        return type(self.M) is JacobiPreconditioner
+
     def _true_residual(self, out):
         """out = b - A x and the true relative residual in S."""
         self.op.true_residual_fin(self.x, self.b, self.E, self.mask, out, self.partials, self.S, self.counter, FIN_TRUE)
@@ -562,7 +567,7 @@ class FCGSolver:
     def _small_iteration(self, check: bool):
         """One Jacobi-preconditioned iteration on a small system: three launches, five at a check."""
         S, M, pq, sp = self.S.data_ptr(), self.M, self.partials.data_ptr(), self.step_partials.data_ptr()
-        x, r, p, q, d, z = (t.data_ptr() for t in (self.x, self.r, self.p, self.q, M.invd, M.z))
+        x, r, p, q, d, z = (t.data_ptr() for t in (self.x, self.r, self.p, self.q, M.invd, self.z_old))
         self.op.apply_dot(self.p, self.E, self.mask, self.q, self.partials)      # q = A p, p.q
         if check:
             _lib.call("vx_small_step", self.n, self.G_op, pq, S, x, p, None, None, None, None, 1, 0, None, _s())
@@ -571,7 +576,8 @@ class FCGSolver:
         _lib.call("vx_small_direction", self.n, sp, S, z, p, _s())
 
     def _iteration(self, check: bool):
-        if self._small:
+        jacobi = self._jacobi
+        if jacobi and self._few:
             return self._small_iteration(check)
         op, S, pp = self.op, self.S.data_ptr(), self.partials.data_ptr()
         # Off the check iterations the updates ride on kernels that stream the same vectors anyway:
@@ -580,13 +586,13 @@ class FCGSolver:
         # At a check iteration x is updated here and r is replaced by b - A x.
         fuse = not check and getattr(self.M, "fuses_residual_update", False)
         op.apply_dot_fin(self.p, self.E, self.mask, self.q, self.partials, self.S, self.counter, FIN_PQ)   # q = A p, p.q
-        if not fuse and (check or not self._jacobi):
+        if not fuse and (check or not jacobi):
             _lib.call("vx_cg_update", _lib.VX_F64, self.n, S, self.x.data_ptr(), self.p.data_ptr(),
                       self.r.data_ptr(), self.q.data_ptr(), 0 if check else 1, _s())
         if check:                                                                # r = b - A x (replacement)
             self._true_residual(self.r)
-        if self._jacobi:                                                         # z = M r over the previous z
-            z = self.M.z
+        if jacobi:                                                               # z = M r over the previous z
+            z = self.z_old
             _lib.call("vx_jacobi_step", self.n, S, self.x.data_ptr(), self.p.data_ptr(), self.r.data_ptr(),
                       self.q.data_ptr(), self.M.invd.data_ptr(), z.data_ptr(), 0 if check else 1, pp,
                       self.counter.data_ptr(), _s())
