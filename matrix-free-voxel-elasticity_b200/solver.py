@@ -419,6 +419,9 @@ class JacobiPreconditioner:
         return self.invd.numel() * 16
 
 
+_JACOBI_EMIT = JacobiPreconditioner.emit
+
+
 @dataclass
 class SolveResult:
     x: torch.Tensor
@@ -550,9 +553,9 @@ class FCGSolver:
     # ------------------------------------------------------------------ kernel emission
     @property
     def _jacobi(self):
-        """Do the fused Jacobi kernels stand for M.emit?  They keep the previous z in this solver's z_old: M.z is
-        scratch that other solvers with the same M write too."""
-        return type(self.M) is JacobiPreconditioner
+        """Do the fused Jacobi kernels stand for M.emit?  (Not for a subclass or a replaced emit.)  They keep the
+        previous z in this solver's z_old: M.z is scratch that other solvers with the same M write too."""
+        return type(self.M) is JacobiPreconditioner and getattr(self.M.emit, "__func__", None) is _JACOBI_EMIT
 
     def _true_residual(self, out):
         """out = b - A x and the true relative residual in S."""

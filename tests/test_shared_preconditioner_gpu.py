@@ -1,4 +1,4 @@
-"""Solvers that share one JacobiPreconditioner and take turns."""
+"""Solvers that share one JacobiPreconditioner and take turns, and a preconditioner whose emit was replaced."""
 import numpy as np
 import pytest
 import torch
@@ -37,3 +37,27 @@ def test_solvers_sharing_a_preconditioner_take_turns(shape, graph):
     b.finish()
     assert (res.iterations, res.rel) == want[1:]
     assert torch.equal(res.x, want[0])
+
+
+@pytest.mark.parametrize("shape", SHAPES)
+def test_a_replaced_emit_is_called(shape):
+    """z = r instead of d r: plain conjugate gradients."""
+    op, E, nm, force, _ = problem(shape)
+    M = vs.JacobiPreconditioner(op, E, nm)
+    calls = []
+
+    def emit(r):
+        calls.append(1)
+        M.z.copy_(r)
+        return M.z
+
+    class Plain(vs.JacobiPreconditioner):
+        def emit(self, r):
+            self.z.copy_(r)
+            return self.z
+
+    want = vs.FCGSolver(op, E, nm, Plain(op, E, nm), tol=1e-12, maxiter=20, check_every=5, graph=False).solve(force)
+    M.emit = emit
+    res = vs.FCGSolver(op, E, nm, M, tol=1e-12, maxiter=20, check_every=5, graph=False).solve(force)
+    assert len(calls) == 21
+    assert torch.equal(res.x, want.x) and res.rel == want.rel
