@@ -212,8 +212,9 @@ STREAM_KERNELS = {"xp": 0, "zp": 1, "march": 2}
 
 def set_stream_kernel(kind: str) -> str:
     """Select the streaming operator kernel for FP64 / FP32 iterates ("march", "xp" or "zp"); returns
-    the previous selection.  Operators size their partial sums at each call, so a change takes
-    effect at the next launch; captured graphs keep the kernel they were captured with."""
+    the previous selection.  A change takes effect at the next launch: the solvers take scratch for the
+    selected kernel at each one, and an operator call refuses `partials` that are too short for it.  Captured
+    graphs keep the kernel they were captured with."""
     prev = int(load().vx_set_stream_kernel(STREAM_KERNELS[kind]))
     if prev < 0:
         raise ValueError(kind)

@@ -115,7 +115,8 @@ class BatchedSolver:
         self.S_host = torch.zeros(self.B, 16, dtype=torch.float64, pin_memory=True)
         self.G = int(_lib.load().vx_solver_partials(self.n_job))
         self.partials = torch.zeros(self.B * 2 * self.G, **f64)
-        self.op_partials = torch.zeros(self.op.partials_size, **f64)       # the stacked forms' sums (unused)
+        self.op_partials = self.op.scratch()               # the stacked forms' sums (unused)
+        self._scratch = [self.op_partials]                 # a captured chunk keeps the one it was captured with
         self.maxiter = int(maxiter)
         self.chunk = int(chunk)
         self.stream = torch.cuda.Stream()
@@ -146,6 +147,10 @@ class BatchedSolver:
     def _iteration(self):
         """One fcg iteration for every slot (true residual every iteration, src/voxel_mg.py:192-209)."""
         S = self.S.data_ptr()
+        t = self.op.scratch(self.op_partials)              # longer where the streaming kernel was changed since
+        if t is not self.op_partials:
+            self.op_partials = t
+            self._scratch.append(t)
         self.op.apply_dot(self.p, self.E64, self.node_mask, self.q, self.op_partials)      # q = A p (stacked)
         self._dots(self.p, self.q)
         self._fin(FIN_PQ)

@@ -112,6 +112,18 @@ class VoxelOperator:
         """doubles of scratch the fused reducing forms (apply_dot / true_residual) need"""
         return int(_lib.load().vx_operator_partials(self._sel, *self.shape))
 
+    def scratch(self, t=None):
+        """`t` where the fused reducing forms can use it as their partials now, else a new tensor that they can.  What
+        they need follows the selected streaming kernel, so a buffer made under another selection may be too short."""
+        n = self.partials_size
+        return t if t is not None and t.numel() >= n else torch.empty(n, dtype=torch.float64, device="cuda")
+
+    def _partials(self, t):
+        p, n = _ptr(t, "partials", torch.float64), self.partials_size
+        if t.numel() < n:
+            raise ValueError(f"partials: expected at least {n} elements for the selected streaming kernel, got {t.numel()}")
+        return p
+
     def _vec(self, t, what, dtype=None):
         return _ptr(t, what, dtype or self.dtype, self.ndof)
 
@@ -174,26 +186,26 @@ class VoxelOperator:
     def apply_dot(self, p, E, node_mask, q, partials):
         """q = A p; partials[cta] = sum p.q over the CTA's nodes (reduce with reduce_partials)."""
         _lib.call("vx_apply_dot", self._sel, *self.shape, self._bp, self._E(E), self._mask(node_mask),
-                  self._vec(p, "p"), self._vec(q, "q"), _ptr(partials, "partials", torch.float64), stream_ptr())
+                  self._vec(p, "p"), self._vec(q, "q"), self._partials(partials), stream_ptr())
 
     def true_residual(self, x, b, E, node_mask, res, partials):
         """res = b - A x; partials[cta] = sum res^2 over the CTA's nodes."""
         _lib.call("vx_true_residual", self._sel, *self.shape, self._bp, self._E(E), self._mask(node_mask),
                   self._vec(x, "x"), self._vec(b, "b"), self._vec(res, "res"),
-                  _ptr(partials, "partials", torch.float64), stream_ptr())
+                  self._partials(partials), stream_ptr())
 
     def apply_dot_fin(self, p, E, node_mask, q, partials, S, counter, fin):
         """apply_dot followed by the finalisation `fin` of its sum into the solver scalars S; counter: one
         zeroed int32, zero again afterwards."""
         _lib.call("vx_apply_dot_fin", fin, self._sel, *self.shape, self._bp, self._E(E), self._mask(node_mask),
-                  self._vec(p, "p"), self._vec(q, "q"), _ptr(partials, "partials", torch.float64),
+                  self._vec(p, "p"), self._vec(q, "q"), self._partials(partials),
                   _ptr(S, "S", torch.float64), _ptr(counter, "counter", torch.int32), stream_ptr())
 
     def true_residual_fin(self, x, b, E, node_mask, res, partials, S, counter, fin):
         """true_residual followed by the finalisation `fin` of its sum into S."""
         _lib.call("vx_true_residual_fin", fin, self._sel, *self.shape, self._bp, self._E(E), self._mask(node_mask),
                   self._vec(x, "x"), self._vec(b, "b"), self._vec(res, "res"),
-                  _ptr(partials, "partials", torch.float64), _ptr(S, "S", torch.float64),
+                  self._partials(partials), _ptr(S, "S", torch.float64),
                   _ptr(counter, "counter", torch.int32), stream_ptr())
 
     def energy(self, u, rho=None, emin=1e-9, emax=1.0, penal=3.0, ce=None, dc=None):

@@ -612,10 +612,7 @@ class SlabSolver:
                                p=torch.zeros(n, **f64), q=torch.zeros(n, **f64),
                                z_old=torch.zeros(n, dtype=dt, device="cuda"),
                                part=torch.zeros(2 * int(_lib.load().vx_solver_partials(L.n_own)), **f64),
-                               # fused-kernel partials, then the two shared planes' corrections (zero when absent)
-                               opp=torch.zeros(L.op64.partials_size + 2 * int(_lib.load().vx_plane_fix_partials(L.P)),
-                                               **f64),
-                               sums=torch.zeros(2, **f64))
+                               opp={}, sums=torch.zeros(2, **f64))
         self.S = torch.zeros(16, **f64)
         self.S_host = torch.zeros(16, dtype=torch.float64, pin_memory=True)
         self.stream = torch.cuda.Stream()
@@ -637,6 +634,16 @@ class SlabSolver:
     def _levels(self):
         return self.M._level(0)
 
+    def _opp(self, i, L):
+        """Slab i's fused-kernel partials under the selected streaming kernel followed by its two shared planes'
+        corrections (zero when absent), and where these begin.  One buffer for each count that a selection gives: a
+        captured loop keeps its own."""
+        n = L.op64.partials_size
+        t = self.vec[i]["opp"].get(n)
+        if t is None:
+            t = self.vec[i]["opp"][n] = torch.zeros(n + 2 * L.G_fix, dtype=torch.float64, device="cuda")
+        return t, n
+
     def _reduce(self, fin, count, fill=None, buf="part"):
         """fill(i, L, partials) writes each slab's dot partials over its owned prefix (or, with
         buf="opp", a fused operator kernel and its plane corrections already did); the slab sums
@@ -644,10 +651,11 @@ class SlabSolver:
         sums = []
         for i, L in self._levels():
             v = self.vec[i]
+            part = v["part"] if buf == "part" else self._opp(i, L)[0]
             if fill is not None:
-                fill(i, L, v[buf].data_ptr())
-            G = int(_lib.load().vx_solver_partials(L.n_own)) if buf == "part" else v["opp"].numel()
-            _lib.call("vx_reduce_partials", G, count, v[buf].data_ptr(), v["sums"].data_ptr(), _s())
+                fill(i, L, part.data_ptr())
+            G = int(_lib.load().vx_solver_partials(L.n_own)) if buf == "part" else part.numel()
+            _lib.call("vx_reduce_partials", G, count, part.data_ptr(), v["sums"].data_ptr(), _s())
             sums.append(v["sums"][:count])
         acc = self.comm.allreduce_(sums)
         _lib.call("vx_solver_finalize", fin, 1, acc.data_ptr(), self.S.data_ptr(), _s())
@@ -660,27 +668,27 @@ class SlabSolver:
     def _apply_dot(self):
         """q = A p and p.q: the fused apply-dot on each slab, its shared planes rewritten with their
         dot terms corrected, the partials summed over slabs (FIN_PQ)."""
-        v = self.vec
+        v, opp = self.vec, {i: self._opp(i, L) for i, L in self._levels()}
         self.M._op(0, lambda i, L: L.partials(_lib.VX_F64, v[i]["p"], L.halo64, L.E64),
                    {i: L.halo64 for i, L in self._levels()},
                    lambda i, L: _lib.call("vx_apply_dot_planes", _lib.VX_F64, *L.shape, L.op64._bp, L.E64.data_ptr(),
                                           L.mask.data_ptr(), v[i]["p"].data_ptr(), v[i]["q"].data_ptr(),
-                                          v[i]["opp"].data_ptr(), *L.interior, _s()),
-                   lambda i, L: L.fix(_lib.VX_F64, PLANE_APPLY, L.halo64, v[i]["p"], v[i]["q"], dot=v[i]["opp"],
-                                      dot_at=L.op64.partials_size))
+                                          opp[i][0].data_ptr(), *L.interior, _s()),
+                   lambda i, L: L.fix(_lib.VX_F64, PLANE_APPLY, L.halo64, v[i]["p"], v[i]["q"], dot=opp[i][0],
+                                      dot_at=opp[i][1]))
         self._reduce(FIN_PQ, 1, buf="opp")
 
     def _true_residual(self, out="r"):
         """out = b - A x and |b - A x|^2 (FIN_TRUE), fused the same way."""
-        v = self.vec
+        v, opp = self.vec, {i: self._opp(i, L) for i, L in self._levels()}
         self.M._op(0, lambda i, L: L.partials(_lib.VX_F64, v[i]["x"], L.halo64, L.E64),
                    {i: L.halo64 for i, L in self._levels()},
                    lambda i, L: _lib.call("vx_true_residual_planes", _lib.VX_F64, *L.shape, L.op64._bp,
                                           L.E64.data_ptr(), L.mask.data_ptr(), v[i]["x"].data_ptr(),
-                                          v[i]["b"].data_ptr(), v[i][out].data_ptr(), v[i]["opp"].data_ptr(),
+                                          v[i]["b"].data_ptr(), v[i][out].data_ptr(), opp[i][0].data_ptr(),
                                           *L.interior, _s()),
                    lambda i, L: L.fix(_lib.VX_F64, PLANE_TRUE_RES, L.halo64, v[i]["x"], v[i][out], v[i]["b"],
-                                      dot=v[i]["opp"], dot_at=L.op64.partials_size))
+                                      dot=opp[i][0], dot_at=opp[i][1]))
         self._reduce(FIN_TRUE, 1, buf="opp")
 
     def _precondition(self):

@@ -533,10 +533,10 @@ class FCGSolver:
         self.dot_host = torch.zeros(1, dtype=torch.float64, pin_memory=True)
         self._dot_with = None
         self.last_dot = None
-        self.G_op = op64.partials_size
         self.G_vec = int(_lib.load().vx_solver_partials(n))
         steps = int(_lib.load().vx_jacobi_step_partials(n))
-        self.partials = torch.empty(max(self.G_op, 2 * self.G_vec, steps), **f64)
+        self.partials = torch.empty(max(op64.partials_size, 2 * self.G_vec, steps), **f64)
+        self._scratch = [self.partials]                      # a captured loop keeps the one it was captured with
         self._few = n <= int(_lib.load().vx_small_cg_limit())
         self.step_partials = torch.empty(steps, **f64)
         self.zprec = PREC[precond.dtype]
@@ -557,8 +557,17 @@ class FCGSolver:
         previous z in this solver's z_old: M.z is scratch that other solvers with the same M write too."""
         return type(self.M) is JacobiPreconditioner and getattr(self.M.emit, "__func__", None) is _JACOBI_EMIT
 
+    def _op_partials(self):
+        """The partials of an operator launch; longer ones where the streaming kernel was changed to one that needs them."""
+        t = self.op.scratch(self.partials)
+        if t is not self.partials:
+            self.partials = t
+            self._scratch.append(t)
+        return t
+
     def _true_residual(self, out):
         """out = b - A x and the true relative residual in S."""
+        self._op_partials()
         self.op.true_residual_fin(self.x, self.b, self.E, self.mask, out, self.partials, self.S, self.counter, FIN_TRUE)
 
     def _dots(self, fin, prec, a, b, c=None):
@@ -569,20 +578,21 @@ class FCGSolver:
 
     def _small_iteration(self, check: bool):
         """One Jacobi-preconditioned iteration on a small system: three launches, five at a check."""
-        S, M, pq, sp = self.S.data_ptr(), self.M, self.partials.data_ptr(), self.step_partials.data_ptr()
+        S, M, pq, sp = self.S.data_ptr(), self.M, self._op_partials().data_ptr(), self.step_partials.data_ptr()
+        G = self.op.partials_size
         x, r, p, q, d, z = (t.data_ptr() for t in (self.x, self.r, self.p, self.q, M.invd, self.z_old))
         self.op.apply_dot(self.p, self.E, self.mask, self.q, self.partials)      # q = A p, p.q
         if check:
-            _lib.call("vx_small_step", self.n, self.G_op, pq, S, x, p, None, None, None, None, 1, 0, None, _s())
+            _lib.call("vx_small_step", self.n, G, pq, S, x, p, None, None, None, None, 1, 0, None, _s())
             self._true_residual(self.r)
-        _lib.call("vx_small_step", self.n, self.G_op, pq, S, x, p, r, q, d, z, 0 if check else 1, 1, sp, _s())
+        _lib.call("vx_small_step", self.n, G, pq, S, x, p, r, q, d, z, 0 if check else 1, 1, sp, _s())
         _lib.call("vx_small_direction", self.n, sp, S, z, p, _s())
 
     def _iteration(self, check: bool):
         jacobi = self._jacobi
         if jacobi and self._few:
             return self._small_iteration(check)
-        op, S, pp = self.op, self.S.data_ptr(), self.partials.data_ptr()
+        op, S, pp = self.op, self.S.data_ptr(), self._op_partials().data_ptr()
         # Off the check iterations the updates ride on kernels that stream the same vectors anyway:
         # r -= alpha q in the preconditioner's first kernel, x += alpha p in the direction update (both in
         # the one step kernel of a Jacobi preconditioner).
@@ -754,9 +764,9 @@ class JacobiPCG:
         self.q = torch.zeros(n, **t)
         self.S = torch.zeros(16, dtype=torch.float64, device="cuda")
         self.S_host = torch.zeros(16, dtype=torch.float64, pin_memory=True)
-        self.G_op = op.partials_size
         self.G_vec = int(_lib.load().vx_solver_partials(n))
-        self.partials = torch.zeros(max(self.G_op, 2 * self.G_vec), dtype=torch.float64, device="cuda")
+        self.partials = torch.zeros(max(op.partials_size, 2 * self.G_vec), dtype=torch.float64, device="cuda")
+        self._scratch = [self.partials]                      # as FCGSolver's
         self.stream = torch.cuda.Stream()
         self.use_graph = bool(graph)
         self._graph = None
@@ -764,15 +774,20 @@ class JacobiPCG:
     def _fin(self, op, G):
         _lib.call("vx_solver_finalize", op, G, self.partials.data_ptr(), self.S.data_ptr(), _s())
 
+    _op_partials = FCGSolver._op_partials
+
+    def _true_residual(self, out, fin):
+        self.op.true_residual(self.x, self.b, self.E, self.mask, out, self._op_partials())
+        self._fin(fin, self.op.partials_size)
+
     def _iteration(self, check):
         op, S = self.op, self.S.data_ptr()
-        op.apply_dot(self.p, self.E, self.mask, self.q, self.partials)
-        self._fin(FIN_PQ, self.G_op)
+        op.apply_dot(self.p, self.E, self.mask, self.q, self._op_partials())
+        self._fin(FIN_PQ, op.partials_size)
         _lib.call("vx_cg_update", self.prec, self.n, S, self.x.data_ptr(), self.p.data_ptr(), self.r.data_ptr(),
                   self.q.data_ptr(), 0 if check else 1, _s())
         if check:
-            op.true_residual(self.x, self.b, self.E, self.mask, self.r, self.partials)
-            self._fin(FIN_TRUE, self.G_op)
+            self._true_residual(self.r, FIN_TRUE)
         _lib.call("vx_jacobi_precond_dot", self.prec, self.n, self.invd.data_ptr(), self.r.data_ptr(),
                   self.z.data_ptr(), self.partials.data_ptr(), _s())
         self._fin(FIN_BETA_FR, self.G_vec)
@@ -807,8 +822,7 @@ class JacobiPCG:
             _lib.call("vx_dots_pr", self.prec, self.prec, self.n, self.b.data_ptr(), self.b.data_ptr(), None,
                       self.partials.data_ptr(), _s())
             self._fin(FIN_NB, self.G_vec)
-            self.op.true_residual(self.x, self.b, self.E, self.mask, self.r, self.partials)   # r = b - A x
-            self._fin(FIN_RR_ONLY, self.G_op)
+            self._true_residual(self.r, FIN_RR_ONLY)                                          # r = b - A x
             _lib.call("vx_jacobi_precond_dot", self.prec, self.n, self.invd.data_ptr(), self.r.data_ptr(),
                       self.z.data_ptr(), self.partials.data_ptr(), _s())
             self._fin(FIN_RZ, self.G_vec)
@@ -841,8 +855,7 @@ class JacobiPCG:
                 s = self._read()
                 it = int(s[S_IT])
             if not s[S_DONE]:
-                self.op.true_residual(self.x, self.b, self.E, self.mask, self.q, self.partials)
-                self._fin(FIN_RR_ONLY, self.G_op)
+                self._true_residual(self.q, FIN_RR_ONLY)
                 s = self._read()
         caller.wait_stream(self.stream)
         return PCGResult(self.x, int(s[S_IT]), bool(s[S_DONE]), float(s[S_REL]))
@@ -897,8 +910,9 @@ class PCGIR:
         self.norm = torch.zeros(1, **f64)
 
     def _residual_norm(self, b):
+        self.partials = self.op64.scratch(self.partials)
         self.op64.true_residual(self.x, b, self.E64, self.mask, self.r, self.partials)
-        _lib.call("vx_reduce_partials", self.partials.numel(), 1, self.partials.data_ptr(), self.norm.data_ptr(), _s())
+        _lib.call("vx_reduce_partials", self.op64.partials_size, 1, self.partials.data_ptr(), self.norm.data_ptr(), _s())
         return float(self.norm) ** 0.5
 
     def solve(self, b: torch.Tensor, x0: torch.Tensor | None = None) -> IRResult:
