@@ -272,7 +272,8 @@ int vx_device_status(int* status, int clear);
 /* Streaming operator kernel for FP64 / FP32 iterates (VX_F64, VX_F32), process-wide; the bf16
  * iterate form always uses the default.  All compute the same arithmetic; they differ in how work is
  * laid out and in the order of the three separable stages:
- *   VX_KERNEL_MARCH  stages y, z, x: the x stage's twelve values stay in registers (default)
+ *   VX_KERNEL_MARCH  stages y, z, x: the x stage's twelve values stay in registers (default; on a grid
+ *                    few nodes thin in y, where its tiles stay mostly empty, the default runs XP)
  *   VX_KERNEL_XP     stages x, y, z: a pair of element planes per thread, CTA barriers between rows
  *   VX_KERNEL_ZP     stages x, y, z: a pair of z node columns per thread, coalesced row spans staged by
  *                    cp.async, warps in a wavefront handing partial sums over mbarriers
@@ -282,10 +283,13 @@ int vx_device_status(int* status, int clear);
  * after it.  Returns the previous selection, or -1 for an unknown kind.  No counterpart in the
  * reference. */
 enum { VX_KERNEL_XP = 0, VX_KERNEL_ZP = 1, VX_KERNEL_MARCH = 2 };
-/* Or'ed into the `prec` of vx_matvec, vx_jacobi_sweep, vx_residual, vx_apply_dot, vx_true_residual and
- * vx_operator_partials: this call runs VX_KERNEL_XP where it would run VX_KERNEL_MARCH. */
-enum { VX_STREAM_XP = 0x100 };
+/* Or'ed into the `prec` of vx_matvec, vx_jacobi_sweep, vx_residual, vx_apply_dot, vx_true_residual (their
+ * _planes and _fin forms too) and vx_operator_partials: this call runs the named kernel where it would run
+ * the default. */
+enum { VX_STREAM_XP = 0x100, VX_STREAM_MARCH = 0x200 };
 int vx_set_stream_kernel(int kind);
+/* The kernel (VX_KERNEL_*) that a call with this `prec` runs on the grid; -1 for an unknown one. */
+int vx_stream_kernel(int prec, int nx, int ny, int nz);
 
 /* Tensor-core element-block operator, an experiment measured against the streaming kernels and not
  * used by the solvers: the dense 24 x 24 element matrix applied to 128 elements at a time by

@@ -16,7 +16,7 @@ LIB_PATH = Path(__file__).resolve().parent / "libvoxel_b200.so"
 VX_OK, VX_ERR_INVALID_ARGUMENT, VX_ERR_NULL_POINTER, VX_ERR_ALIGNMENT = 0, 1, 2, 3
 VX_ERR_LAUNCH, VX_ERR_UNSUPPORTED, VX_ERR_TIMEOUT, VX_ERR_CUDA = 4, 5, 6, 7
 VX_F64, VX_F32, VX_BF16_F32, VX_F32_BF16AUX = 0, 1, 2, 3
-VX_STREAM_XP = 0x100
+VX_STREAM_XP, VX_STREAM_MARCH = 0x100, 0x200
 
 _P = c_void_p          # device or host pointer
 _D = POINTER(c_double)  # host double array
@@ -64,6 +64,7 @@ SIGNATURES = {
     "vx_true_residual_noalloc": (c_int, [c_int, c_int, c_int, c_int, _D, _P, _P, _P, _P, _P, _P, _P]),
     "vx_device_status": (c_int, [POINTER(c_int), c_int]),
     "vx_set_stream_kernel": (c_int, [c_int]),
+    "vx_stream_kernel": (c_int, [c_int, c_int, c_int, c_int]),
     "vx_tc_element_product": (c_int, [c_int, c_int, c_int, _D, c_void_p, c_void_p, c_void_p, c_void_p, c_int,
                                       c_void_p]),
     "vx_tc_status": (c_int, [POINTER(c_int), c_int]),
@@ -166,7 +167,7 @@ HOST_ONLY = {"vx_last_error", "vx_version", "vx_element_matrix", "vx_element", "
              "vx_operator_partials", "vx_partials_size", "vx_jacobi_step_partials", "vx_small_cg_limit", "vx_solver_slots", "vx_solver_partials",
              "vx_graph_while_begin", "vx_graph_destroy", "vx_capture_status", "vx_graph_launch",
              "vx_oc_partials", "vx_graph_body_nodes", "vx_plane_fix_partials", "vx_device_status",
-             "vx_coarse_factor_workspace", "vx_split_factor_size", "vx_split_workspace", "vx_set_stream_kernel",
+             "vx_coarse_factor_workspace", "vx_split_factor_size", "vx_split_workspace", "vx_set_stream_kernel", "vx_stream_kernel",
              "vx_tc_status"}
 launches = 0          # kernels launched directly (graph launches are counted by the solvers)
 

@@ -58,7 +58,7 @@ struct OpArgs {
     int cx;                   // owned node planes per CTA (x chunk)
     bool cubic;               // host side: the blocks have the cube pattern (CubeK)
     const double* blocks;     // host side: the 72 parity coefficients
-    bool xp;                  // host side: parity_stream_xp instead of parity_march (VX_STREAM_XP)
+    int sel;                  // host side: the call's selector (VX_STREAM_XP, VX_STREAM_MARCH)
     BlocksT<TC> C;
 };
 
@@ -809,20 +809,36 @@ dim3 march_grid(const Grid& g, int* cx) {
     return dim3(tz, ty, (g.nx + 1 + *cx - 1) / *cx);
 }
 
-// Streaming kernel for FP64 / FP32 iterates (process-wide; the other storage forms run parity_march):
+// Streaming kernel for FP64 / FP32 iterates (process-wide; the other storage forms always run the default):
 // VX_KERNEL_MARCH (the default), VX_KERNEL_XP (element-plane pairs) or VX_KERNEL_ZP (node-column pairs).
-// A call whose selector carries VX_STREAM_XP runs parity_stream_xp instead of parity_march.
 static std::atomic<int> g_stream_kernel{VX_KERNEL_MARCH};
+constexpr int STREAM_BITS = VX_STREAM_XP | VX_STREAM_MARCH;
 
-inline int stream_kind(bool selectable, bool xp) {
+// Grids few nodes thin in y, where the default runs parity_stream_xp: its tiles of 6 node rows are fuller there than
+// parity_march's of 14.  Two of them take about as long as one of march's in FP32, so xp is ahead where a march tile
+// is covered by one: up to 6 rows always, 15 to 18 and 29 or 30 on grids with many waves of CTAs, whose last one no
+// longer decides; in FP64 up to 6 rows on such grids.  Measured (us, matvec, march / xp): FP32 512x5x1500 117 / 74,
+// 300x3x300 22.6 / 18.4, 512x15x1500 217 / 188, 300x15x300 37 / 35, 600x15x45 18.5 / 20.5, 512x6x1500 117 / 131;
+// FP64 512x5x1500 191 / 141, 24x5x5000 43 / 35, 300x5x300 31 / 35, 1x5x240000 193 / 191, 512x6x1500 191 / 262.
+inline bool thin_in_y(const Grid& g, bool f64) {
+    const int rows = g.ny + 1, xp = (rows + 5) / 6, march = (rows + 13) / 14;
+    if (xp >= 2 * march || (f64 && rows > 6)) return false;
+    return (!f64 && rows <= 6) || (g.nx >= 3 && int64_t(g.nx + 1) * (g.nz + 1) >= 125000);
+}
+
+// The kernel of a call: `selectable` for FP64 / FP32 iterates; sel's VX_STREAM_ bits pick for this call alone, in
+// place of the default.
+inline int stream_kind(bool selectable, int sel, const Grid& g, bool f64) {
     const int kind = selectable ? g_stream_kernel.load(std::memory_order_relaxed) : VX_KERNEL_MARCH;
-    return xp && kind == VX_KERNEL_MARCH ? VX_KERNEL_XP : kind;
+    if (kind != VX_KERNEL_MARCH) return kind;
+    if (sel & VX_STREAM_XP) return VX_KERNEL_XP;
+    return !(sel & VX_STREAM_MARCH) && thin_in_y(g, f64) ? VX_KERNEL_XP : VX_KERNEL_MARCH;
 }
 
 // CTAs (= partial sums) of a fused reducing launch of precision `prec` on grid g
 int64_t stream_ctas(const Grid& g, int sel) {
-    const int prec = sel & ~VX_STREAM_XP;
-    const int kind = stream_kind(true, sel & VX_STREAM_XP);
+    const int prec = sel & ~STREAM_BITS;
+    const int kind = stream_kind(true, sel, g, prec == VX_F64);
     if (prec == VX_F32 || prec == VX_F64) {
         if (kind == VX_KERNEL_ZP) {
             const ZpGrid z = prec == VX_F32 ? zp_grid_for<float>(g) : zp_grid_for<double>(g);
@@ -864,7 +880,7 @@ int launch_stream(const OpArgs<TC, TU, TE, TY, TR>& a_in, cudaStream_t s, const 
     static std::atomic<uint64_t> configured[2];            // per kernel of this instantiation: devices opted in
     if constexpr (v2) {
         const bool cubic = a.cubic;
-        const int kind = stream_kind(selectable, a.xp);
+        const int kind = stream_kind(selectable, a.sel, a.g, std::is_same<TC, double>::value);
         using Args = OpArgs2<TC, TU, TE, TY, TR>;
         auto go = [&](void (*k)(const Args), std::atomic<uint64_t>& done, dim3 grid, unsigned threads, size_t smem) -> int {
             const Args a2 = packed_args<TC, TU, TE, TY, TR, EPI, MASK>(a);
@@ -1037,7 +1053,7 @@ using namespace vx;
 // =========================================================================== C ABI
 extern "C" int vx_matvec(int sel, int nx, int ny, int nz, const double* blocks, const void* E,
                          const void* u, void* y, const uint8_t* node_mask, cudaStream_t stream) {
-    const int prec = sel & ~VX_STREAM_XP;
+    const int prec = sel & ~STREAM_BITS;
     int st = check_grid(nx, ny, nz);
     if (st) return st;
     VX_CHECK_ARG(blocks && E && u && y, VX_ERR_NULL_POINTER, "vx_matvec: NULL pointer");
@@ -1050,8 +1066,8 @@ extern "C" int vx_matvec(int sel, int nx, int ny, int nz, const double* blocks, 
         a.g = Grid{nx, ny, nz}; a.u = (const X*)u; a.E = (const M*)E; a.y = (TC*)y; a.node_mask = node_mask;
         a.C = convert_blocks<TC>(blocks);
         a.cubic = cube_pattern(blocks);
-            a.blocks = blocks;
-        a.xp = sel & VX_STREAM_XP;
+        a.blocks = blocks;
+        a.sel = sel;
         rc = node_mask ? launch_stream<TC, X, M, TC, EPI_RAW, MASK_NODE, false, false>(a, stream, "vx_matvec")
                        : launch_stream<TC, X, M, TC, EPI_RAW, MASK_NONE, false, false>(a, stream, "vx_matvec");
     });
@@ -1193,7 +1209,7 @@ int fused_dispatch(const char* what, int sel, int nx, int ny, int nz, const doub
                    const uint8_t* node_mask, const void* x, const void* r, const void* invd, double omega,
                    void* out, double* partials, cudaStream_t stream, int dot_x0 = 0, int dot_x1 = INT_MAX, int fin = 0,
                    double* S = nullptr, unsigned* counter = nullptr) {
-    const int prec = sel & ~VX_STREAM_XP;
+    const int prec = sel & ~STREAM_BITS;
     int st = check_grid(nx, ny, nz);
     if (st) return st;
     VX_CHECK_ARG(blocks && E && x && out, VX_ERR_NULL_POINTER, "%s: NULL pointer", what);
@@ -1222,7 +1238,7 @@ int fused_dispatch(const char* what, int sel, int nx, int ny, int nz, const doub
             a.C = convert_blocks<TC>(blocks);
             a.cubic = cube_pattern(blocks);
             a.blocks = blocks;
-            a.xp = sel & VX_STREAM_XP;
+            a.sel = sel;
             rc = node_mask ? launch_stream<TC, X, M, TY, EPI, MASK_NODE, false, false, R>(a, stream, what)
                            : launch_stream<TC, X, M, TY, EPI, MASK_NONE, false, false, R>(a, stream, what);
         }
@@ -1249,7 +1265,7 @@ extern "C" int vx_residual(int prec, int nx, int ny, int nz, const double* block
 }
 
 extern "C" int64_t vx_operator_partials(int sel, int nx, int ny, int nz) {
-    const int prec = sel & ~VX_STREAM_XP;
+    const int prec = sel & ~STREAM_BITS;
     if (check_grid(nx, ny, nz) || (prec != VX_F64 && prec != VX_F32)) return -1;
     return stream_ctas(Grid{nx, ny, nz}, sel);
 }
@@ -1279,7 +1295,7 @@ int fused_fin(const char* what, int op, int sel, int nx, int ny, int nz, const d
               unsigned* counter, cudaStream_t stream) {
     VX_CHECK_ARG(partials && S && counter, VX_ERR_NULL_POINTER, "%s: NULL pointer", what);
     VX_CHECK_ARG(op >= 0 && op <= FIN_RR_ONLY && op != FIN_BETA_PR, VX_ERR_INVALID_ARGUMENT, "%s: bad op %d", what, op);
-    const bool march = stream_kind(true, sel & VX_STREAM_XP) == VX_KERNEL_MARCH;
+    const bool march = stream_kind(true, sel, Grid{nx, ny, nz}, (sel & ~STREAM_BITS) == VX_F64) == VX_KERNEL_MARCH;
     int st = fused_dispatch<EPI>(what, sel, nx, ny, nz, blocks, E, node_mask, x, r, nullptr, 0.0, out, partials, stream, 0,
                                  INT_MAX, op, S, march ? counter : nullptr);
     if (st || march) return st;
@@ -1394,6 +1410,12 @@ extern "C" int vx_true_residual_noalloc(int prec, int nx, int ny, int nz, const 
                                       nullptr, 0.0, res, scratch, stream);
     if (st) return st;
     return vx_reduce_partials(G, 1, scratch, norm2, stream);
+}
+
+extern "C" int vx_stream_kernel(int sel, int nx, int ny, int nz) {
+    const int prec = sel & ~STREAM_BITS;
+    if (check_grid(nx, ny, nz) || prec < VX_F64 || prec > VX_F32_BF16AUX) return -1;
+    return stream_kind(prec != VX_BF16_F32, sel, Grid{nx, ny, nz}, prec == VX_F64);
 }
 
 extern "C" int vx_set_stream_kernel(int kind) {

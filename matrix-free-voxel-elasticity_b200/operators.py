@@ -78,12 +78,15 @@ def dofs_from_node_mask(node_mask: torch.Tensor, dtype=torch.float64) -> torch.T
     return torch.stack([(bits >> c) & 1 for c in range(3)], dim=1).reshape(-1).to(dtype)
 
 
+STREAM_BITS = {None: 0, "xp": _lib.VX_STREAM_XP, "march": _lib.VX_STREAM_MARCH}
+
+
 class VoxelOperator:
     """K(E) on a (nx, ny, nz) voxel grid in `dtype` storage (float64, float32, or bfloat16 with
     FP32 arithmetic).  `aux_dtype` (default `dtype`) is the storage of the modulus and of the
     auxiliary vectors (right-hand side, inverse diagonal, residual output); float32 iterates with
-    bfloat16 auxiliaries is the VX_F32_BF16AUX mode.  `stream="xp"` has the matvec, sweep, residual and
-    reducing forms run the element-plane-pair kernel where the default would run (VX_STREAM_XP)."""
+    bfloat16 auxiliaries is the VX_F32_BF16AUX mode.  `stream="xp"` ("march") has the matvec, sweep, residual
+    and reducing forms run that kernel where they would run the default."""
 
     def __init__(self, shape, ke, dtype=torch.float64, aux_dtype=None, stream=None):
         self.shape = tuple(int(s) for s in shape)
@@ -96,9 +99,9 @@ class VoxelOperator:
             raise ValueError(f"unsupported storage: iterate {dtype}, auxiliary {aux_dtype}")
         self.dtype, self.aux_dtype = dtype, aux_dtype
         self.prec = STORAGE[(dtype, aux_dtype)]
-        if stream not in (None, "xp"):
+        if stream not in STREAM_BITS:
             raise ValueError(f"unknown stream kernel {stream!r}")
-        self._sel = self.prec | (_lib.VX_STREAM_XP if stream == "xp" else 0)
+        self._sel = self.prec | STREAM_BITS[stream]
         self.nodes = n_nodes(self.shape)
         self.ndof = 3 * self.nodes
         self.n_elem = n_elems(self.shape)
