@@ -288,8 +288,10 @@ enum { VX_KERNEL_XP = 0, VX_KERNEL_ZP = 1, VX_KERNEL_MARCH = 2 };
  * the default. */
 enum { VX_STREAM_XP = 0x100, VX_STREAM_MARCH = 0x200 };
 int vx_set_stream_kernel(int kind);
-/* The kernel (VX_KERNEL_*) that a call with this `prec` runs on the grid; -1 for an unknown one. */
+/* The kernel (VX_KERNEL_*) that a call with this `prec` runs on the grid, and what the default is there whatever
+ * kernel is selected; -1 for an unknown `prec`. */
 int vx_stream_kernel(int prec, int nx, int ny, int nz);
+int vx_default_kernel(int prec, int nx, int ny, int nz);
 
 /* Tensor-core element-block operator, an experiment measured against the streaming kernels and not
  * used by the solvers: the dense 24 x 24 element matrix applied to 128 elements at a time by

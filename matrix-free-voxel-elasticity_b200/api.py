@@ -13,7 +13,7 @@ import torch
 
 from .element import quadrature
 from .operators import VoxelOperator, node_mask_from_dofs
-from .solver import FCGSolver, JacobiPreconditioner, MGHierarchy, hierarchy_shapes, small_grid_stream
+from .solver import FCGSolver, JacobiPreconditioner, MGHierarchy, hierarchy_shapes
 
 PRECISIONS = ("fp64", "mixed", "bf16", "bf16-all", "jacobi")
 # V-cycle storage: (iterate dtype, auxiliary-vector and modulus dtype)
@@ -47,8 +47,7 @@ class ElasticitySolver:
         self.E = _dev(E).clone()          # owned: update_modulus rewrites it in place
         m = mask.to("cuda", non_blocking=True) if isinstance(mask, torch.Tensor) else _dev(mask)
         self.node_mask = m.contiguous() if m.dtype == torch.uint8 else node_mask_from_dofs(m.to(torch.float64))
-        self.op64 = VoxelOperator(self.shape, self.ke, torch.float64,
-                                  stream=None if precision == "jacobi" else small_grid_stream(self.shape))
+        self.op64 = VoxelOperator(self.shape, self.ke, torch.float64)
         self.precision = precision
         if precision == "jacobi":
             self.M = JacobiPreconditioner(self.op64, self.E, self.node_mask)

@@ -104,7 +104,7 @@ class BatchedSolver:
         self.M = MGHierarchy(geo.grid, self.ke, E64, self.node_mask, dt, pre, post, omega, shapes=list(geo.shapes),
                              aux_dtype=aux, coarse_blocks=self.B)
         self.E64 = self.M.levels[0].E64                    # the hierarchy's own finest moduli
-        self.op = VoxelOperator(geo.grid, self.ke, torch.float64)
+        self.op = VoxelOperator(geo.grid, self.ke, torch.float64, stream=self.M.levels[0].op64.stream)
         n = self.op.ndof
         f64 = dict(dtype=torch.float64, device="cuda")
         self.b, self.x, self.r, self.p, self.q = (torch.zeros(n, **f64) for _ in range(5))

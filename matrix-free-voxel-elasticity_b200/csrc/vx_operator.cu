@@ -1418,6 +1418,11 @@ extern "C" int vx_stream_kernel(int sel, int nx, int ny, int nz) {
     return stream_kind(prec != VX_BF16_F32, sel, Grid{nx, ny, nz}, prec == VX_F64);
 }
 
+extern "C" int vx_default_kernel(int prec, int nx, int ny, int nz) {
+    if (check_grid(nx, ny, nz) || prec < VX_F64 || prec > VX_F32_BF16AUX) return -1;
+    return stream_kind(false, 0, Grid{nx, ny, nz}, prec == VX_F64);
+}
+
 extern "C" int vx_set_stream_kernel(int kind) {
     if (kind != VX_KERNEL_MARCH && kind != VX_KERNEL_ZP && kind != VX_KERNEL_XP) {
         set_error("vx_set_stream_kernel: unknown kernel %d", kind);

@@ -10,6 +10,7 @@ All tensors are CUDA, contiguous, author layout.  Nothing here falls back to the
 """
 from __future__ import annotations
 
+import copy
 import ctypes
 
 import numpy as np
@@ -101,6 +102,7 @@ class VoxelOperator:
         self.prec = STORAGE[(dtype, aux_dtype)]
         if stream not in STREAM_BITS:
             raise ValueError(f"unknown stream kernel {stream!r}")
+        self.stream = stream
         self._sel = self.prec | STREAM_BITS[stream]
         self.nodes = n_nodes(self.shape)
         self.ndof = 3 * self.nodes
@@ -108,6 +110,12 @@ class VoxelOperator:
         self._ydtype = torch.float32 if dtype == torch.bfloat16 else dtype     # of vx_matvec's result
         self._bp = _lib.dptr(self.blocks)
         self._kp = _lib.dptr(self.ke)
+
+    def on(self, stream):
+        """This operator with another `stream`."""
+        op = copy.copy(self)
+        op.stream, op._sel = stream, self.prec | STREAM_BITS[stream]
+        return op
 
     # --------------------------------------------------------------- helpers
     @property

@@ -32,7 +32,8 @@ from . import _lib
 from .element import quadrature
 from .operators import PREC, STORAGE, VoxelOperator, node_mask_from_dofs, stream_ptr
 from .solver import (FIN_BETA_PR, FIN_NB, FIN_PQ, FIN_RZ, FIN_TRUE, S_BREAK, S_CHECK, S_DONE, S_IT, S_MAXIT,
-                     S_MV, S_REL, S_TOL, SolveResult, _GraphLoop, hierarchy_shapes, small_grid_stream)
+                     S_MV, S_REL, S_TOL, SolveResult, _GraphLoop, hierarchy_shapes, level_stream,
+                     small_grid_stream)
 
 PLANE_APPLY, PLANE_JACOBI, PLANE_RESIDUAL, PLANE_TRUE_RES = range(4)
 _ARITH = {torch.float64: torch.float64, torch.float32: torch.float32, torch.bfloat16: torch.float32}
@@ -182,7 +183,8 @@ class _Halo:
 class _SlabLevel:
     """One level of one slab: the slab-local grid and its buffers."""
 
-    def __init__(self, index, nparts, shape, a, ke, dtype, aux):
+    def __init__(self, index, nparts, shape, a, ke, dtype, aux, streams):
+        """streams: of the operator in (dtype, aux) and of the FP64 one (solver.level_stream of the global grids)."""
         self.index, self.shape, self.a = index, tuple(shape), int(a)
         nlx, ny, nz = self.shape
         self.P = (ny + 1) * (nz + 1)
@@ -195,8 +197,8 @@ class _SlabLevel:
         self.G_fix = int(_lib.load().vx_plane_fix_partials(self.P))
         self.ke = np.ascontiguousarray(ke)
         self.kp = _lib.dptr(self.ke)
-        self.op = VoxelOperator(self.shape, self.ke, dtype, aux)
-        self.op64 = self.op if dtype == torch.float64 else VoxelOperator(self.shape, self.ke, torch.float64)
+        self.op = VoxelOperator(self.shape, self.ke, dtype, aux, stream=streams[0])
+        self.op64 = self.op if dtype == torch.float64 else VoxelOperator(self.shape, self.ke, torch.float64, stream=streams[1])
         self.halo = _Halo(3 * self.P, _ARITH[dtype], self.has_lo, self.has_hi)
         self.halo64 = self.halo if _ARITH[dtype] == torch.float64 else _Halo(3 * self.P, torch.float64,
                                                                            self.has_lo, self.has_hi)
@@ -265,7 +267,8 @@ class SlabHierarchy:
             levels = []
             for l, s in enumerate(self.shapes):
                 f = 1 << l
-                L = _SlabLevel(i, self.nparts, (b // f - a // f, s[1], s[2]), a // f, self.ke * f, dtype, aux_dtype)
+                L = _SlabLevel(i, self.nparts, (b // f - a // f, s[1], s[2]), a // f, self.ke * f, dtype, aux_dtype,
+                               [level_stream(self.shapes[0], s, prec) for prec in (self.prec, _lib.VX_F64)])
                 if l == 0:
                     # owned copies: a caller rewriting its global arrays does not change the solver
                     L.E64 = E[a * ny * nz:b * ny * nz].to(torch.float64).clone()
@@ -671,7 +674,7 @@ class SlabSolver:
         v, opp = self.vec, {i: self._opp(i, L) for i, L in self._levels()}
         self.M._op(0, lambda i, L: L.partials(_lib.VX_F64, v[i]["p"], L.halo64, L.E64),
                    {i: L.halo64 for i, L in self._levels()},
-                   lambda i, L: _lib.call("vx_apply_dot_planes", _lib.VX_F64, *L.shape, L.op64._bp, L.E64.data_ptr(),
+                   lambda i, L: _lib.call("vx_apply_dot_planes", L.op64._sel, *L.shape, L.op64._bp, L.E64.data_ptr(),
                                           L.mask.data_ptr(), v[i]["p"].data_ptr(), v[i]["q"].data_ptr(),
                                           opp[i][0].data_ptr(), *L.interior, _s()),
                    lambda i, L: L.fix(_lib.VX_F64, PLANE_APPLY, L.halo64, v[i]["p"], v[i]["q"], dot=opp[i][0],
@@ -683,7 +686,7 @@ class SlabSolver:
         v, opp = self.vec, {i: self._opp(i, L) for i, L in self._levels()}
         self.M._op(0, lambda i, L: L.partials(_lib.VX_F64, v[i]["x"], L.halo64, L.E64),
                    {i: L.halo64 for i, L in self._levels()},
-                   lambda i, L: _lib.call("vx_true_residual_planes", _lib.VX_F64, *L.shape, L.op64._bp,
+                   lambda i, L: _lib.call("vx_true_residual_planes", L.op64._sel, *L.shape, L.op64._bp,
                                           L.E64.data_ptr(), L.mask.data_ptr(), v[i]["x"].data_ptr(),
                                           v[i]["b"].data_ptr(), v[i][out].data_ptr(), opp[i][0].data_ptr(),
                                           *L.interior, _s()),

@@ -36,16 +36,27 @@ def hierarchy_shapes(shape, max_coarse_x=16):
     return shapes
 
 
-# Grids whose multigrid solves keep the element-plane-pair kernel on every level.  Below about 20,000
-# elements such a solve is bound by its launches, and on rough moduli its two- or three-level cycle often
-# does not converge: the iterate at maxiter then depends on every rounding, so these solves keep the
-# operations in the order they always had.
+# Multigrid solves on finest grids below this many elements keep the order of operations that they have always had:
+# the element-plane-pair kernel on every level and one band for the coarsest system.  That is not the faster form
+# (V-cycle FP32 / FP64, us, with these -> with parity_march and the split factor: 20x10x10 27 / 35 -> 23 / 23, 32x16x16
+# 56 / 66 -> 39 / 41, 40x24x24 50 / 64 -> 41 / 43).  The reason is their results.  Uncorrelated random moduli are the
+# usual field of small problems, and on them the cycle does not converge: at maxiter 200 all eight grids tried from
+# 20x10x10 to 32x18x18 stand 1e-4 to 9e-3 from the solution, in every precision, and another order of operations
+# returns an iterate 2e-5 (FP64 cycle) to 7e-3 (bf16) from this one, though no better or worse one.  (Correlated moduli
+# converge in 15 iterations, to the same x within 1e-13, either way.)
 SMALL_GRID = 20000
 
 
 def small_grid_stream(shape):
-    """`stream` of the VoxelOperators of a multigrid solve on the finest grid `shape`."""
+    """`stream` of the VoxelOperators of a multigrid solve on the finest grid `shape` of one job."""
     return "xp" if shape[0] * shape[1] * shape[2] < SMALL_GRID else None
+
+
+def level_stream(finest, shape, prec):
+    """`stream` of the operator on a level of `shape` under the finest grid `finest`, both a job's own: how the grid is
+    stacked or cut into slabs must not change a job's arithmetic."""
+    kind = _lib.load().vx_default_kernel(prec, *shape)
+    return small_grid_stream(finest) or ("xp" if kind == _lib.STREAM_KERNELS["xp"] else "march")
 
 
 def _s():
@@ -106,6 +117,8 @@ class MGHierarchy:
         E64 = E.to(torch.float64).contiguous()
         mask = node_mask if node_mask is not None else all_free_mask(self.shapes[0])
         self.levels = []
+        job = self._job_shape(coarse_blocks)
+        self.operator_stream = small_grid_stream(job)               # of an outer operator that names none
         for i, s in enumerate(self.shapes):
             if i:
                 prev = self.shapes[i - 1]
@@ -116,9 +129,10 @@ class MGHierarchy:
                 E64, mask = Ec, mc
             L = _Level()
             L.shape = s
-            st = small_grid_stream(self.shapes[0])
-            L.op = VoxelOperator(s, self.ke * 2 ** i, dtype, aux_dtype, stream=st)
-            L.op64 = L.op if dtype == torch.float64 else VoxelOperator(s, self.ke * 2 ** i, torch.float64, stream=st)
+            mk = lambda dt, aux: VoxelOperator(s, self.ke * 2 ** i, dt, aux,                         # noqa: E731
+                                               stream=level_stream(job, (job[0] >> i, *s[1:]), STORAGE[(dt, aux)]))
+            L.op = mk(dtype, aux_dtype)
+            L.op64 = L.op if dtype == torch.float64 else mk(torch.float64, torch.float64)
             L.E64, L.mask = E64, mask
             L.E = E64 if aux_dtype == torch.float64 else E64.to(aux_dtype)
             inv64 = L.op64.diagonal(E64, mask, inverse=True)
@@ -135,8 +149,6 @@ class MGHierarchy:
         self._split = None
         if self.blocks:
             nxc, nyc, nzc = c.shape
-            if (nxc + 1) % self.blocks:
-                raise ValueError(f"coarsest grid {c.shape} does not split into {self.blocks} jobs")
             pc = (nxc + 1) // self.blocks                       # job pitch: nx_job + 1 separator element
             self.job_coarse = (pc - 1, nyc, nzc)
             nb_ = 3 * pc * (nyc + 1) * (nzc + 1)
@@ -152,8 +164,8 @@ class MGHierarchy:
                       _ptr(c.E64, "E"), _ptr(c.mask, "mask"), A.data_ptr(), _s())
             self.A_coarse = A
             # The coarsest planes split at the middle one where that is possible (half the factor's chain, 0.56
-            # of the bytes of a solve); small grids keep the one band (small_grid_stream)
-            size = 0 if small_grid_stream(self.shapes[0]) else int(_lib.load().vx_split_factor_size(*c.shape))
+            # of the bytes of a solve); small grids keep the one band (SMALL_GRID)
+            size = 0 if self.operator_stream else int(_lib.load().vx_split_factor_size(*c.shape))
             f64 = dict(dtype=torch.float64, device="cuda")
             if size:
                 self._split = torch.empty(size, **f64)
@@ -305,6 +317,15 @@ class MGHierarchy:
         work = getattr(self, "_factor_work", None)
         factor = self.coarse_packed if self._split is None else self._split
         return b + (self.A_coarse.numel() + factor.numel() + (0 if work is None else work.numel())) * 8
+
+    def _job_shape(self, blocks):
+        """The finest grid of one job: the whole one, or one of `blocks` stacked along x."""
+        if not blocks:
+            return self.shapes[0]
+        l, (nxc, nyc, nzc) = len(self.shapes) - 1, self.shapes[-1]
+        if (nxc + 1) % blocks:
+            raise ValueError(f"coarsest grid {self.shapes[-1]} does not split into {blocks} jobs")
+        return (((nxc + 1) // blocks - 1) << l, *self.shapes[0][1:])
 
     def spectral_omegas(self, iterations=30, seed=20260923):
         """omega_l = 4 / (3 lambda_l), lambda_l from a seeded FP64 power iteration on D^-1 A over the
@@ -511,6 +532,8 @@ class FCGSolver:
                  fixed_iterations=None, graph=True):
         if op64.dtype != torch.float64:
             raise ValueError("the outer operator must be float64")
+        if op64.stream is None and getattr(precond, "operator_stream", None):
+            op64 = op64.on(precond.operator_stream)                 # one kernel for a small grid's whole solve
         self.op, self.E, self.mask, self.M = op64, E64.contiguous(), node_mask, precond
         self.tol, self.maxiter, self.fixed = float(tol), int(maxiter), fixed_iterations
         self.check_every = max(1, int(check_every))
