@@ -1393,11 +1393,13 @@ extern "C" int vx_true_residual_noalloc(int prec, int nx, int ny, int nz, const 
                  "vx_true_residual_noalloc: NULL pointer");
     VX_CHECK_ARG(prec == VX_F64 || prec == VX_F32, VX_ERR_INVALID_ARGUMENT,
                  "vx_true_residual_noalloc: unsupported precision %d", prec);
-    // parity_march's 14 x 14 FP64 tiles are more than parity_stream_xp's 6 x 30 on a grid a few nodes thin
-    // in y and very long in z (28572 against 13334 on 1x5x400000): such a grid still fits by the latter
+    // On a grid a few nodes thin in y and very long in z the default kernel's tiles may be too many where the other's
+    // still fit: parity_march's 14 x 14 in FP64 (28572 against 13334 on 1x5x400000), parity_stream_xp's 6 x 30 against
+    // 14 x 30 in FP32 (17001 against 11334 on 4x16x170000)
     int sel = prec;
     int64_t G = stream_ctas(Grid{nx, ny, nz}, sel);
-    if (G > NOALLOC_MAX_CTAS) G = stream_ctas(Grid{nx, ny, nz}, sel |= VX_STREAM_XP);
+    for (int bit : {VX_STREAM_XP, VX_STREAM_MARCH})
+        if (G > NOALLOC_MAX_CTAS) G = stream_ctas(Grid{nx, ny, nz}, sel = prec | bit);
     VX_CHECK_ARG(G <= NOALLOC_MAX_CTAS, VX_ERR_INVALID_ARGUMENT,
                  "vx_true_residual_noalloc: grid (%d, %d, %d) needs %lld partial sums but the built-in scratch "
                  "holds %lld; use vx_true_residual with a caller-provided buffer",

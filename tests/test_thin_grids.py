@@ -61,3 +61,23 @@ def test_every_form(shape, dtype):
         y, x, m = (form(ops[s]) for s in (None, "xp", "march"))
         assert torch.equal(y, x if thin else m), name
         assert float((x.double() - m.double()).abs().max()) <= tol * float(x.double().abs().max()), name
+
+
+@pytest.mark.gpu
+def test_noalloc_residual_where_only_march_fits():
+    """A grid on which the default kernel's FP32 partial sums are more than the built-in scratch holds."""
+    shape = (4, 16, 170000)
+    lib, op = _lib.load(), vx.VoxelOperator(shape, vo.quadrature([1, 1, 1], 0.3), torch.float32)
+    assert lib.vx_operator_partials(F32 | _lib.VX_STREAM_MARCH, *shape) <= 16384 < op.partials_size
+    g = torch.Generator("cuda").manual_seed(1)
+    x, b = (torch.randn(op.ndof, dtype=torch.float32, device="cuda", generator=g) for _ in range(2))
+    E = torch.rand(op.n_elem, dtype=torch.float32, device="cuda", generator=g) + 0.01
+    nm = torch.full((op.nodes,), 7, dtype=torch.uint8, device="cuda")
+    nm[:17] = 0
+    part = torch.empty(op.partials_size, dtype=torch.float64, device="cuda")
+    ref, res, n2 = torch.empty_like(x), torch.empty_like(x), torch.zeros(1, dtype=torch.float64, device="cuda")
+    op.true_residual(x, b, E, nm, ref, part)
+    _lib.call("vx_true_residual_noalloc", op.prec, *shape, op._bp, E.data_ptr(), nm.data_ptr(), x.data_ptr(),
+              b.data_ptr(), res.data_ptr(), n2.data_ptr(), torch.cuda.current_stream().cuda_stream)
+    assert float((res - ref).abs().max()) <= 1e-5 * float(ref.abs().max())
+    assert abs(float(n2) - float(ref.double() @ ref.double())) <= 1e-6 * float(n2)
