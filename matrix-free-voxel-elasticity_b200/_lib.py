@@ -177,9 +177,19 @@ launches = 0          # kernels launched directly (graph launches are counted by
 _FNS = {}             # name -> (bound entry point, its kernels per call; None: counted from its arguments)
 
 
+def _kernels(name: str, args) -> int:
+    """Kernels that a call launches, of the entry points for which this follows from the arguments."""
+    if name in ("vx_apply_dot_fin", "vx_true_residual_fin"):     # parity_march finishes its sum itself
+        return 1 if _lib.vx_stream_kernel(*args[1:5]) == STREAM_KERNELS["march"] else 2
+    if name == "vx_split_factor":                                # two chains as below, four products
+        planes, p = int(args[0]) + 1, 3 * (int(args[1]) + 1) * (int(args[2]) + 1)
+        return 2 * ((planes // 2 * p + 63) // 64) + 2 * ((p + 63) // 64) + 6
+    return 2 * ((int(args[0]) + 63) // 64) + 1                   # load, a factor and an update per block, inverse
+
+
 def _bind(name: str):
     count = KERNELS_PER_CALL.get(name, 0 if name in HOST_ONLY else 1)
-    if name in ("vx_coarse_factor", "vx_batch_coarse_factor", "vx_split_factor"):
+    if name in ("vx_coarse_factor", "vx_batch_coarse_factor", "vx_split_factor", "vx_apply_dot_fin", "vx_true_residual_fin"):
         count = None
     entry = _FNS[name] = (getattr(load(), name), count)
     return entry
@@ -193,12 +203,7 @@ def call(name: str, *args) -> None:
     status = fn(*args)
     if status:
         check(status, name)
-    if count is None and name == "vx_split_factor":    # two chains as below, four products
-        planes, p = int(args[0]) + 1, 3 * (int(args[1]) + 1) * (int(args[2]) + 1)
-        count = 2 * ((planes // 2 * p + 63) // 64) + 2 * ((p + 63) // 64) + 6
-    elif count is None:                   # load, a factor and an update per block, inverse
-        count = 2 * ((int(args[0]) + 63) // 64) + 1
-    launches += count
+    launches += _kernels(name, args) if count is None else count
     if CAPTURE_STREAM is not None and _lib.vx_capture_status(CAPTURE_STREAM) == 2:
         raise RuntimeError(f"{name} invalidated the stream capture")
 
