@@ -892,7 +892,7 @@ def run_serving(args):
 
 def main():
     args = parse()
-    if args.impl == "b200" and args.stream_kernel != "xp":
+    if args.impl == "b200":
         from voxel_b200 import _lib
         _lib.set_stream_kernel(args.stream_kernel)
     if args.kernels:
