@@ -12,6 +12,7 @@ from __future__ import annotations
 
 import copy
 import ctypes
+import os
 
 import numpy as np
 import torch
@@ -28,7 +29,15 @@ STORAGE = {(torch.float64, torch.float64): _lib.VX_F64, (torch.float32, torch.fl
 
 _RAW_STREAM = getattr(torch._C, "_cuda_getCurrentRawStream", None)
 _CUR_DEVICE = getattr(torch._C, "_cuda_getDevice", None)
-_initialized = False          # CUDA's initialisation is for the life of the process
+_initialized = False          # CUDA's initialisation is for the life of the process, but not of one forked from it
+
+
+def _forked():
+    global _initialized
+    _initialized = False
+
+
+os.register_at_fork(after_in_child=_forked)
 
 
 def stream_ptr(device=None) -> int:
