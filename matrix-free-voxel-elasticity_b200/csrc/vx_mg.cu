@@ -113,14 +113,17 @@ inline RestrictShape restrict_shape(const Grid& c) {
 // access is a run of consecutive words.  3-D launch, so no thread divides by a grid extent.
 // Bound by HBM (4.1 TB/s in FP32); measured (us, L2 flushed, FP32 / bf16 / FP64, one fine node per thread
 // -> now): 576x288x288 463 / 557 / 580 -> 309 / 330 / 549, 256x128x128 49 / 59 / 57 -> 41 / 41 / 52.
+// SHORT: rows of at most half a CTA; it takes several coarse rows, each on the least power of two of threads that
+// holds one (us, FP32, one row a CTA -> now: 74x156x4 4.1 -> 2.6, 102x352x20 10.7 -> 6.2, 576x288x16 44.6 -> 23.1).
 constexpr int PT = 128;
-template <typename T>
+template <typename T, bool SHORT>
 __global__ void __launch_bounds__(PT) prolong_add_kernel(Grid f, Grid c, const T* __restrict__ coarse,
                                                          const uint8_t* __restrict__ fmask, T* __restrict__ x) {
     vx::pdl_begin();
     using A = arith_t<T>;
-    const int w = blockIdx.x * PT + threadIdx.x, J = blockIdx.y, I = blockIdx.z;
-    if (w >= 3 * (f.nz + 1)) return;
+    const int w = SHORT ? threadIdx.x : blockIdx.x * PT + threadIdx.x, I = blockIdx.z;
+    const int J = SHORT ? blockIdx.y * blockDim.y + threadIdx.y : blockIdx.y;
+    if (w >= 3 * (f.nz + 1) || (SHORT && J > c.ny)) return;
     const int k = w / 3, comp = w - 3 * k;
     const bool oz = k & 1, ox = 2 * I + 1 <= f.nx, oy = 2 * J + 1 <= f.ny;
     const int crow = 3 * (c.nz + 1), cplane = crow * (c.ny + 1);
@@ -380,8 +383,11 @@ extern "C" int vx_prolong_add(int prec, int nx, int ny, int nz, const void* coar
     Grid f{nx, ny, nz}, c{nx / 2, ny / 2, nz / 2};
     const bool ok = dispatch_prec(prec, [&](auto t) {             // iterates on both sides
         using X = typename decltype(t)::X;
-        const dim3 grid(blocks_for(3 * (int64_t(nz) + 1), PT), unsigned(c.ny + 1), unsigned(c.nx + 1));
-        vx::launch(prolong_add_kernel<X>, grid, PT, 0, stream, f, c, (const X*)coarse, fine_mask, (X*)x);
+        unsigned tx = PT;
+        while (tx > 16 && tx / 2 >= 3 * (unsigned(nz) + 1)) tx /= 2;
+        const dim3 grid(blocks_for(3 * (int64_t(nz) + 1), tx), blocks_for(c.ny + 1, PT / tx), unsigned(c.nx + 1));
+        vx::launch(tx < PT ? prolong_add_kernel<X, true> : prolong_add_kernel<X, false>, grid, dim3(tx, PT / tx), 0, stream, f, c,
+                   (const X*)coarse, fine_mask, (X*)x);
     });
     VX_CHECK_ARG(ok, VX_ERR_INVALID_ARGUMENT, "vx_prolong_add: unsupported precision %d", prec);
     VX_CHECK_LAUNCH("vx_prolong_add");

@@ -115,3 +115,22 @@ def test_restriction_with_the_first_coarse_sweep(shape, dtype, aux):
     _lib.call("vx_restrict_sweep", prec, *shape, rf.data_ptr(), cm.data_ptr(), rs.data_ptr(), d.data_ptr(), 0.6,
               xs.data_ptr(), _s())
     assert torch.equal(rs, rc) and torch.equal(xs, xc)
+
+
+@pytest.mark.parametrize("nz", [2, 4, 6, 10, 18, 20, 42, 44])
+def test_prolongation_of_short_rows(nz):
+    """Rows of 9 to 135 words, at and across the powers of two at which a CTA takes 8, 4, 2 or 1 coarse rows, with a
+    last CTA of fewer: the oracle's bits, inside guard bands."""
+    for ny in (2, 30, 36):
+        shape = (6, ny, nz)
+        coarse = tuple(s // 2 for s in shape)
+        rng = np.random.default_rng(sum(shape))
+        nf, nc = 3 * vo.n_nodes(shape), 3 * vo.n_nodes(coarse)
+        x0, uc, fm = rng.standard_normal(nf), rng.standard_normal(nc), _masks(shape, rng)
+        whole = torch.full((nf + 512,), float("nan"), dtype=torch.float64, device="cuda")
+        x = whole[256:256 + nf]
+        x.copy_(torch.as_tensor(x0))
+        u_d, m_d = torch.as_tensor(uc, device="cuda"), torch.as_tensor(fm, device="cuda")
+        _lib.call("vx_prolong_add", _lib.VX_F64, *shape, u_d.data_ptr(), m_d.data_ptr(), x.data_ptr(), _s())
+        assert np.array_equal(x.cpu().numpy(), np.where(_dof(fm) > 0, x0 + vo.prolong(uc, coarse), x0))
+        assert bool(whole[:256].isnan().all()) and bool(whole[256 + nf:].isnan().all())
