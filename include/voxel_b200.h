@@ -288,6 +288,7 @@ enum { VX_KERNEL_XP = 0, VX_KERNEL_ZP = 1, VX_KERNEL_MARCH = 2 };
  * the default. */
 enum { VX_STREAM_XP = 0x100, VX_STREAM_MARCH = 0x200 };
 int vx_set_stream_kernel(int kind);
+int vx_selected_kernel(void);    /* the present selection */
 /* The kernel (VX_KERNEL_*) that a call with this `prec` runs on the grid, and what the default is there whatever
  * kernel is selected; -1 for an unknown `prec`. */
 int vx_stream_kernel(int prec, int nx, int ny, int nz);

@@ -64,6 +64,7 @@ SIGNATURES = {
     "vx_true_residual_noalloc": (c_int, [c_int, c_int, c_int, c_int, _D, _P, _P, _P, _P, _P, _P, _P]),
     "vx_device_status": (c_int, [POINTER(c_int), c_int]),
     "vx_set_stream_kernel": (c_int, [c_int]),
+    "vx_selected_kernel": (c_int, []),
     "vx_stream_kernel": (c_int, [c_int, c_int, c_int, c_int]),
     "vx_default_kernel": (c_int, [c_int, c_int, c_int, c_int]),
     "vx_tc_element_product": (c_int, [c_int, c_int, c_int, _D, c_void_p, c_void_p, c_void_p, c_void_p, c_int,
@@ -169,7 +170,7 @@ HOST_ONLY = {"vx_last_error", "vx_version", "vx_element_matrix", "vx_element", "
              "vx_graph_while_begin", "vx_graph_destroy", "vx_capture_status", "vx_graph_launch",
              "vx_oc_partials", "vx_graph_body_nodes", "vx_plane_fix_partials", "vx_device_status",
              "vx_coarse_factor_workspace", "vx_split_factor_size", "vx_split_workspace", "vx_set_stream_kernel", "vx_stream_kernel",
-             "vx_default_kernel",
+             "vx_default_kernel", "vx_selected_kernel",
              "vx_tc_status"}
 launches = 0          # kernels launched directly (graph launches are counted by the solvers)
 

@@ -1420,6 +1420,8 @@ extern "C" int vx_stream_kernel(int sel, int nx, int ny, int nz) {
     return stream_kind(prec != VX_BF16_F32, sel, Grid{nx, ny, nz}, prec == VX_F64);
 }
 
+extern "C" int vx_selected_kernel(void) { return g_stream_kernel.load(std::memory_order_relaxed); }
+
 extern "C" int vx_default_kernel(int prec, int nx, int ny, int nz) {
     if (check_grid(nx, ny, nz) || prec < VX_F64 || prec > VX_F32_BF16AUX) return -1;
     return stream_kind(false, 0, Grid{nx, ny, nz}, prec == VX_F64);

@@ -113,6 +113,7 @@ class VoxelOperator:
             raise ValueError(f"unknown stream kernel {stream!r}")
         self.stream = stream
         self._sel = self.prec | STREAM_BITS[stream]
+        self._sizes = {}                       # partials_size under each selected kernel
         self.nodes = n_nodes(self.shape)
         self.ndof = 3 * self.nodes
         self.n_elem = n_elems(self.shape)
@@ -123,19 +124,23 @@ class VoxelOperator:
     def on(self, stream):
         """This operator with another `stream`."""
         op = copy.copy(self)
-        op.stream, op._sel = stream, self.prec | STREAM_BITS[stream]
+        op.stream, op._sel, op._sizes = stream, self.prec | STREAM_BITS[stream], {}
         return op
 
     # --------------------------------------------------------------- helpers
     @property
     def partials_size(self) -> int:
         """doubles of scratch the fused reducing forms (apply_dot / true_residual) need"""
-        return int(_lib.load().vx_operator_partials(self._sel, *self.shape))
+        kind = (_lib._FNS.get("vx_selected_kernel") or _lib._bind("vx_selected_kernel"))[0]()
+        n = self._sizes.get(kind)
+        if n is None:
+            n = self._sizes[kind] = int(_lib.load().vx_operator_partials(self._sel, *self.shape))
+        return n
 
-    def scratch(self, t=None):
+    def scratch(self, t=None, n=None):
         """`t` where the fused reducing forms can use it as their partials now, else a new tensor that they can.  What
         they need follows the selected streaming kernel, so a buffer made under another selection may be too short."""
-        n = self.partials_size
+        n = self.partials_size if n is None else n
         return t if t is not None and t.numel() >= n else torch.empty(n, dtype=torch.float64, device="cuda")
 
     def _partials(self, t):

@@ -580,9 +580,10 @@ class FCGSolver:
         previous z in this solver's z_old: M.z is scratch that other solvers with the same M write too."""
         return type(self.M) is JacobiPreconditioner and getattr(self.M.emit, "__func__", None) is _JACOBI_EMIT
 
-    def _op_partials(self):
-        """The partials of an operator launch; longer ones where the streaming kernel was changed to one that needs them."""
-        t = self.op.scratch(self.partials)
+    def _op_partials(self, n=None):
+        """The partials of an operator launch (n of them); longer ones where the streaming kernel was changed to one that
+        needs them."""
+        t = self.op.scratch(self.partials, n)
         if t is not self.partials:
             self.partials = t
             self._scratch.append(t)
@@ -601,8 +602,8 @@ class FCGSolver:
 
     def _small_iteration(self, check: bool):
         """One Jacobi-preconditioned iteration on a small system: three launches, five at a check."""
-        S, M, pq, sp = self.S.data_ptr(), self.M, self._op_partials().data_ptr(), self.step_partials.data_ptr()
         G = self.op.partials_size
+        S, M, pq, sp = self.S.data_ptr(), self.M, self._op_partials(G).data_ptr(), self.step_partials.data_ptr()
         x, r, p, q, d, z = (t.data_ptr() for t in (self.x, self.r, self.p, self.q, M.invd, self.z_old))
         self.op.apply_dot(self.p, self.E, self.mask, self.q, self.partials)      # q = A p, p.q
         if check:

@@ -78,3 +78,19 @@ def test_a_small_job_alone_and_among_eight_is_bitwise_equal(precision):
     for k in (0, 7):
         alone = BatchedSolver(shape, 1, precision=precision, maxiter=40).solve([jobs[k]])[0]
         assert torch.equal(alone[0], all_[k][0]) and alone[1:4] == all_[k][1:4]
+
+
+def test_the_partials_size_follows_the_selection():
+    op = vx.VoxelOperator((32, 16, 16), KE)
+    lib, seen = _lib.load(), {}
+    prev = _lib.set_stream_kernel("march")
+    try:
+        for kind in ("march", "xp", "zp", "march", "xp"):
+            _lib.set_stream_kernel(kind)
+            assert lib.vx_selected_kernel() == _lib.STREAM_KERNELS[kind]
+            seen[kind] = op.partials_size
+            assert seen[kind] == lib.vx_operator_partials(op._sel, *op.shape)
+        _lib.set_stream_kernel("march")
+        assert op.on("xp").partials_size == seen["xp"] != seen["march"] == op.partials_size
+    finally:
+        _lib.set_stream_kernel(prev)
