@@ -19,7 +19,7 @@
 // plane e are written before it; their readers (rows above and below) come after it.  The operand ring
 // has three planes (own read of plane e, neighbour read of e + 1, write of e + 2), the contributions two.
 //
-// What bounds it: the FP64 forms the double-precision pipe (133 of about 270 issued instructions an element
+// What bounds it: the FP64 forms the double-precision pipe (150 of about 296 issued instructions an element
 // row, half busy) together with the latency between its barriers, the FP32 sweep HBM, issue and registers.
 // Eight warps and two CTAs an SM (128 registers) let one CTA compute while the other waits at its barrier;
 // measured at 576x288x288 (us, matvec FP64 / FP32, Jacobi FP64 / FP32) before the changes noted below: 2 x 8
@@ -185,7 +185,6 @@ parity_march(const __grid_constant__ OpArgs2<TC, TU, TE, TY, TR> args) {
         n_out[c] = (x0 - 1) * plane_nodes + cn;              // plane x0 - 1 is never stored
         e_in[c] = (x0 - 1) * plane_elems + min(max(iy, 0), g.ny - 1) * g.nz + min(max(iz, 0), g.nz - 1);
     }
-    const bool compute = N == 2 || LZ < 32 || row < ROWS - 1;    // warp-uniform
 
     extern __shared__ __align__(16) unsigned char smem_raw[];
     P* const us = reinterpret_cast<P*>(smem_raw);            // operand ring: 3 planes x ROWS x 3 x LZ
@@ -263,7 +262,7 @@ parity_march(const __grid_constant__ OpArgs2<TC, TU, TE, TY, TR> args) {
     bits1 = put_u(RING);
     load_u(x0 + 1);
     __syncthreads();
-    if (compute) {
+    {
         P ya[3][2];
         y_stage(0, ya);
         #pragma unroll
@@ -303,7 +302,7 @@ parity_march(const __grid_constant__ OpArgs2<TC, TU, TE, TY, TR> args) {
                 }
         }
         P hown[3];
-        if (compute) {
+        {
             const P E = C::make(ev);
             const TC nv[2] = {-ev[0], -ev[N - 1]};
             const P nE = C::make(nv);
@@ -365,7 +364,7 @@ parity_march(const __grid_constant__ OpArgs2<TC, TU, TE, TY, TR> args) {
             }
         }
         __syncthreads();
-        if (compute && !FIRST) {
+        if (!FIRST) {
             P yv[3];
             #pragma unroll
             for (int k = 0; k < 3; ++k) {

@@ -219,10 +219,11 @@ __global__ void __launch_bounds__(FT) jacobi_step_kernel(int64_t n, double* S, d
 // The same iteration for small grids (at most SMALL_CTAS CTAs of one entry per thread), where the hand-over of
 // a sum through the last CTA (a fence, an atomic, the partials' and scalars' round trips: 2 to 3 us) costs
 // more than the work: every CTA of the kernel that needs a sum adds up the partials itself, in the same
-// order, and CTA 0 alone writes the scalars.  No kernel reads a slot that it writes: the step takes rz from
-// S_RZN and leaves it in S_RZ, the direction takes S_RZ and leaves the new one in S_RZN.
+// order, and CTA 0 alone writes the scalars.  No CTA depends on a slot that CTA 0 may have written already: the step
+// takes rz from S_RZN and leaves it in S_RZ, the direction takes S_RZ and leaves the new one in S_RZN.  S_BREAK
+// is read and may be set in the step, but only where every CTA finds `stop` from the same sum and takes no step anyway.
 // 32x16x16, 700 iterations: 12.8 -> 9.0 us an iteration (separate update, product, dots and
-// finalize kernels: 15.2).
+// finalize kernels: 16.8).
 constexpr int64_t SMALL_CTAS = 1184;
 __device__ __forceinline__ double sum_partials(int64_t G, const double* __restrict__ partials) {
     __shared__ double total;

@@ -40,9 +40,9 @@ def hierarchy_shapes(shape, max_coarse_x=16):
 # the element-plane-pair kernel on every level and one band for the coarsest system.  That is not the faster form
 # (V-cycle FP32 / FP64, us, with these -> with parity_march and the split factor: 20x10x10 27 / 35 -> 23 / 23, 32x16x16
 # 56 / 66 -> 39 / 41, 40x24x24 50 / 64 -> 41 / 43).  The reason is their results.  Uncorrelated random moduli are the
-# usual field of small problems, and on them the cycle does not converge: at maxiter 200 all eight grids tried from
-# 20x10x10 to 32x18x18 stand 1e-4 to 9e-3 from the solution, in every precision, and another order of operations
-# returns an iterate 2e-5 (FP64 cycle) to 7e-3 (bf16) from this one, though no better or worse one.  (Correlated moduli
+# usual field of small problems, and on them (densities 0.01 to 1, cubed) the cycle does not converge: at maxiter 200
+# all eight grids tried from 20x10x10 to 32x18x18 stand 7e-5 to 9e-3 from the solution, in every precision, and another
+# order of operations returns an iterate 2e-5 (FP64 cycle) to 7e-3 (bf16) from this one, though no better or worse one.  (Correlated moduli
 # converge in 15 iterations, to the same x within 1e-13, either way.)
 SMALL_GRID = 20000
 
