@@ -152,7 +152,7 @@ def build_inputs(name, device="cuda"):
 # 256x128x128 grid (4,276,737 nodes): dram__bytes_read.sum + dram__bytes_write.sum / nodes.  Scaled by
 # the node count of the measured launch (the traffic of these streaming kernels grows with the nodes).
 NCU_TRAFFIC_PER_NODE = {"jacobi_sweep_f32": (177.938944e6 + 35.143424e6) / 4276737,
-                        "apply_dot_f64": (140.538112e6 + 67.077376e6) / 4276737}
+                        "apply_dot_f64": (140.556800e6 + 67.267584e6) / 4276737}
 NCU_TRAFFIC_SOURCE = "ncu dram bytes of the same kernel on 256x128x128, per node, scaled by nodes"
 
 
